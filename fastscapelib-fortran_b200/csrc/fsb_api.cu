@@ -167,23 +167,20 @@ size_t layout(fsb::Ctx& c, char* base) {
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaGetLastError();
-    c.ntplans = fsb::plan_tiles(c.nx, c.ny, sms, c.tplans, fsb::Ctx::kMaxPlans);
-    for (auto& t : c.tplan_of) t = fsb::TileMap{};
-    for (auto& f : c.tform_of) f = 0;
-    size_t P = 0;
-    int T = 0;
-    c.rl_icap = 0;
-    for (int i = 0; i < c.ntplans; ++i) {  // buffers for the largest of the candidate plans
-      P = std::max(P, (size_t)c.tplans[i].padded());
-      T = std::max(T, c.tplans[i].tiles());
-      c.rl_icap = std::max(c.rl_icap, 2 * ((1 << c.tplans[i].ltx) + (1 << c.tplans[i].lty)) + 16);
+    for (auto& r : c.region_ok) r = 0;
+    size_t words = 0, cells = 0, entries = 0;  // of the larger plan
+    for (int p = 0; p < fsb::kTilePlans; ++p) {
+      const int lt = fsb::kLogTileMin + p;
+      const fsb::TileMap& t = c.tplan[p] = fsb::plan_tiles(c.nx, c.ny, lt, sms);
+      if (t.ntx == 0) continue;
+      words = std::max(words, (size_t)t.tiles() * fsb::rim_words(lt));
+      cells = std::max(cells, (size_t)t.tiles() * fsb::rim_cells(lt));
+      entries = std::max(entries, t.queue_entries());
     }
-    c.rl_line = L.take<double>(16 * P);
-    c.rl_val = L.take<double>(2 * P);
-    c.rl_cnt0 = L.take<unsigned char>(P);
-    c.rl_xcnt = L.take<int>(P);
-    c.rl_inbox = L.take<int>((size_t)T * c.rl_icap);
-    c.rl_itail = L.take<unsigned>((size_t)T);
+    c.rl_wmeta = L.take<unsigned short>(N);
+    c.rl_flags = L.take<unsigned>(words);
+    c.rl_mbox = L.take<double>(2 * cells);
+    c.rl_queue = L.take<long long>(entries);
   }
   c.s_scan2 = L.take<int>(N + 1);
   c.done = L.take<unsigned>(N); c.ticket = L.take<unsigned>(4);

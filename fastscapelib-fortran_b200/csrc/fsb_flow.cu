@@ -584,11 +584,14 @@ __device__ inline void put8(T (&a)[8], int n, T v) {
 template <bool MIXED>
 __global__ void k_mfd_receivers(Bounds bd, double p, const double* __restrict__ h0, const double* __restrict__ ltab,
                                 int* __restrict__ mrec, int* __restrict__ mnrec, double* __restrict__ mwrec,
-                                double* __restrict__ mlrec) {
+                                double* __restrict__ mlrec, int* __restrict__ mmask) {
   const int nx = bd.nx, ny = bd.ny, nn = nx * ny;
   for (int ij = blockIdx.x * blockDim.x + threadIdx.x; ij < nn; ij += gridDim.x * blockDim.x) {
     const int i = ij % nx, j = ij / nx;
     int nr = 0;
+    // directions t = 0..7 in loop order: bit t a receiver slot, bit 8 + t a
+    // distinct receiver (a clamped neighbour lies in another direction)
+    int mask = 0;
     int rr[8];
     double w[8], ll[8];
 #pragma unroll
@@ -613,6 +616,9 @@ __global__ void k_mfd_receivers(Bounds bd, double p, const double* __restrict__ 
             put8(ll, nr, l);
             put8(w, nr, (hij - hk) / l);
             ++nr;
+            const int di = bd.xcyc ? ii : iii - i, dj = bd.ycyc ? jj : jjj - j;
+            const int cl = 3 * (jj + 1) + ii + 1, ca = 3 * (dj + 1) + di + 1;
+            mask |= 1 << (cl - (cl > 4)) | 256 << (ca - (ca > 4));
           }
         }
       }
@@ -661,6 +667,7 @@ __global__ void k_mfd_receivers(Bounds bd, double p, const double* __restrict__ 
       l2[t] = make_double2(ll[2 * t], ll[2 * t + 1]);
     }
     mnrec[ij] = nr;
+    mmask[ij] = mask;
   }
 }
 
@@ -1245,10 +1252,10 @@ void mfd_receivers(Ctx& c) {
   const int nn = c.nn;
   if (c.mixed)
     k_mfd_receivers<true><<<grid1d(nn), kBlock, 0, c.stream>>>(c.bd, c.p, c.hwater, c.ltab, c.mrec, c.mnrec, c.mwrec,
-                                                               c.mlrec);
+                                                               c.mlrec, c.mdmask);
   else
     k_mfd_receivers<false><<<grid1d(nn), kBlock, 0, c.stream>>>(c.bd, c.p, c.hwater, c.ltab, c.mrec, c.mnrec,
-                                                                c.mwrec, c.mlrec);
+                                                                c.mwrec, c.mlrec, c.mdmask);
   c.count_launch();
   if (c.capture) {  // a topological order of mrec (the reference's mstack is a LIFO Kahn order)
     k_order_keys<<<grid1d(nn), kBlock, 0, c.stream>>>(nn, c.stack, c.hwater, c.o_keys, c.o_vals);

@@ -23,21 +23,18 @@ inline unsigned grid1d(size_t n, int block = kBlock) {
   return (unsigned)g;
 }
 
-// Tile-major numbering of the grid for the region-owned sweeps (fsb_region.cu):
-// tiles of 2^ltx x 2^lty nodes, tile t = ty*ntx + tx, node (i, j) at
-// g = t*2^(ltx+lty) + (j mod 2^lty)*2^ltx + (i mod 2^ltx).  Slots of partial
-// tiles beyond the grid are padding.
+// Tiles of the region-owned sweeps (fsb_region.cu): squares of 2^lt nodes a
+// side, tile ty*ntx + tx, dealt out over nctas CTAs (tile t to CTA t % nctas).
+constexpr int kLogTileMin = 5, kTilePlans = 2;  // sides 32 and 64
+// per tile: mailbox cells, one for each node around it, and flag words, one bit per cell
+__host__ __device__ constexpr int rim_cells(int lt) { return ((4 << lt) + 4 + 15) & ~15; }
+__host__ __device__ constexpr int rim_words(int lt) { return (rim_cells(lt) + 127) / 128 * 4; }
 struct TileMap {
-  int nx = 0, ny = 0;
-  int ltx = 0, lty = 0;
+  int nx = 0, ny = 0, lt = 0;
   int ntx = 0, nty = 0;  // ntx == 0: no plan
-  __host__ __device__ int lr() const { return ltx + lty; }
+  int nctas = 0, ns = 0;  // CTAs, tiles per CTA at most
   __host__ __device__ int tiles() const { return ntx * nty; }
-  __host__ __device__ long long padded() const { return (long long)tiles() << lr(); }
-  __host__ __device__ int g(int i, int j) const {
-    const int t = (j >> lty) * ntx + (i >> ltx);
-    return (t << lr()) | ((j & ((1 << lty) - 1)) << ltx) | (i & ((1 << ltx) - 1));
-  }
+  size_t queue_entries() const { return ((size_t)nctas * ns) << (2 * lt); }
 };
 
 struct Ctx {
@@ -137,21 +134,14 @@ struct Ctx {
   void* mfd_line = nullptr;  // one 128-byte record per node (area, then stream power)
   double* hw = nullptr;      // (elevation, water surface) pairs of the stream-power sweep
   double* slots = nullptr;   // kSlotStride input slots per node of the multiple-flow sweeps
-  // region-owned sweeps (fsb_region.cu): tile plan and tile-major buffers
-  static constexpr int kMaxPlans = 3;
-  TileMap tplans[kMaxPlans] = {};  // candidate plans (smallest tiles first)
-  int ntplans = 0;
-  TileMap tplan_of[8] = {};        // per sweep op: the tuned plan (ntx == 0: not yet)
-  int tform_of[8] = {};            // per sweep op: the tuned kernel form (0: one node per warp)
+  // region-owned sweeps (fsb_region.cu)
+  TileMap tplan[kTilePlans];  // per tile side
   bool region_enabled = true;  // use them when the plan and a cooperative launch allow
-  signed char region_ok[8] = {};  // per sweep op: 0 unchecked, 1 usable, -1 not on this device
-  void* rl_line = nullptr;     // one 128-byte line per tile-major slot
-  double* rl_val = nullptr;    // 2 doubles per slot: area, or (h, water)
-  unsigned char* rl_cnt0 = nullptr;  // initial counters, one byte per slot
-  int* rl_xcnt = nullptr;      // cross-tile inputs per slot
-  int* rl_inbox = nullptr;     // per tile: nodes whose cross-tile inputs are all in
-  unsigned* rl_itail = nullptr;
-  int rl_icap = 0;
+  signed char region_ok[8] = {};  // per sweep op: 0 unchecked, 1 usable, -1 not
+  unsigned short* rl_wmeta = nullptr;  // per node: inputs to wait for | dependents' directions << 8
+  unsigned* rl_flags = nullptr;        // rim_words per tile
+  double* rl_mbox = nullptr;           // rim_cells mailbox cells of up to 16 bytes per tile
+  long long* rl_queue = nullptr;       // ready nodes: natural index << 32 | index within the CTA
   unsigned* la_ctl = nullptr;  // head, tail, done count
   int* s_scan2 = nullptr;
   // sweeps
@@ -232,7 +222,7 @@ void flux_mfd(Ctx& c, double* flux);                  // compute_fluxes' flux, m
 // tridiagonal systems s0..s1-1, element t of system s at [t*L + s], F solved in place
 // region-owned multiple-flow sweeps (fsb_region.cu); false: not usable, the
 // queue engine of fsb_flow.cu runs instead
-int plan_tiles(int nx, int ny, int sms, TileMap* out, int max_plans);
+TileMap plan_tiles(int nx, int ny, int lt, int sms);
 bool region_accumulate(Ctx& c);
 bool region_stream_power(Ctx& c);
 void thomas_lines(Ctx& c, int N, int L, int s0, int s1, const double* A, const double* B, const double* C, double* F,

@@ -8,25 +8,35 @@
 //
 // Both sweeps are recurrences along the receiver DAG whose critical path is
 // about three grid sides long, so their time is the number of hops on that
-// path times the latency of one hop.  Here the grid is cut into 2^a x 2^b
-// tiles, one co-resident CTA per tile (cooperative launch), and nodes are
-// numbered tile-major (a tile's nodes are contiguous).  A CTA keeps its
-// tile's dependency counters (one byte per node, four to a word) and its
-// ready queue in shared memory: a hop between two nodes of one tile is a
-// shared-memory atomic and loads that the SM's L1 serves, not an L2 round
-// trip.  Every node's value lands once in a tile-major value array, from
-// which its dependents gather it, so no input slots need resetting.  A
-// dependency that crosses a tile boundary goes through a global counter; its
-// last producer posts the node into the owning CTA's inbox (release/acquire
-// at GPU scope), which one lane of the CTA polls.  The arithmetic of a node,
-// including the order of its sums, is that of the queue engine in
+// path times the latency of one hop, plus what the nodes of the wave front
+// cost the SMs that own them.  The grid is cut into square tiles dealt out
+// over one CTA per SM (cooperative launch, all co-resident), so that the
+// front, wherever it runs, is spread over all SMs.  A CTA keeps its nodes'
+// dependency counters in shared memory and hands ready nodes to its warps
+// through a queue that its L1 serves; one lane computes one node.  What a
+// node needs beyond its inputs' values is one 96-byte record, built in
+// parallel before the sweep and brought into L1 by the nodes it waits for.
+// A value that crosses a tile edge is written into a mailbox cell of the
+// neighbouring tile, whose CTA polls a flag bit per cell: the value itself
+// says whether it has arrived, so no fence beyond CTA scope runs during a
+// sweep (a fence at GPU scope would empty the SM's L1).  The arithmetic of a
+// node, including the order of its sums, is that of the queue engine in
 // fsb_flow.cu, so both engines give bit-identical results.
+//
+// What bounds them (2049^2, B200, a trace of every node's start and end
+// followed back from the last one): the path is about 6,000 hops, 90 % of
+// them continuations inside one warp.  A stream-power hop is about 750 cycles
+// for each Newton iteration (a root, two exchanges, sixteen additions in
+// order, a quotient) and about 800 between the value and the next node's
+// start; an area hop about 950 (records come from DRAM there) and 500.  150
+// hops cross a tile, at 4,000 to 6,000 cycles each.  DRAM is idle.  Against the form
+// with one tile per CTA, a warp per node and inboxes behind GPU-scope fences:
+// area 6.9 -> 5.8 ms, stream power 12.0 -> 6.9 ms; 4097^2 (which took the
+// queue engine) 36.1 -> 17.1 and 54.9 -> 20.6 ms with their records; 2049x1537
+// closed basins, n = 1: 7.6 -> 6.1 and 24.0 -> 7.3 ms.
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
-#include <map>
-#include <mutex>
-#include <tuple>
 #include <type_traits>
 
 #include "fsb_kernels.cuh"
@@ -35,392 +45,338 @@ namespace fsb {
 
 namespace {
 
-// Co-resident sweep CTAs per SM the tile plan counts on.  The threads of a
-// sweep CTA (warp 0 polls the inbox, the others compute nodes) are the op's
-// kThreads: 512 where its registers allow two such CTAs per SM -- more
-// worker warps per tile measured faster at 2049^2 (stream-power sweep 32 ->
-// 16 ms against 256 threads).
-constexpr int kRegionCtasPerSm = 2;
-constexpr unsigned short kQEmpty = 0xFFFF;
+constexpr unsigned FULL = 0xffffffffu;
 constexpr unsigned long long kRegionTimeLimitNs = 4000000000ull;  // a sweep giving up: 4 s
+
+// Threads of a sweep CTA (warp 0 polls the flag words, the others compute
+// nodes).  2049^2, B200: 384 threads 5.9 + 7.9 ms (area + stream power), 512
+// threads 5.8 + 7.3, 768 threads 5.8 + 7.5.
+constexpr int kThreads = 512;
+// grids whose records (96 bytes a node) L2 does not keep
+constexpr int kL2Records = 1 << 20;
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-// weak load that the SM's L1 may serve (values written by this CTA)
-__device__ __forceinline__ double ld_l1(const double* p) {
+// Loads under a predicate, without a branch (0 where it is off); the SM's L1
+// may serve them (values written by this CTA)
+__device__ __forceinline__ double ld_l1_if(const double* p, bool on) {
   double v;
-  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+  asm volatile(
+      "{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n mov.f64 %0, 0d0000000000000000;\n @q ld.global.f64 %0, [%1];\n}"
+      : "=d"(v)
+      : "l"(p), "r"((unsigned)on)
+      : "memory");
   return v;
 }
-__device__ __forceinline__ double2 ld_l1(const double2* p) {
-  double2 v;
-  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
-  return v;
-}
-// load from L2 (values written by other SMs, after an acquire)
-__device__ __forceinline__ double ld_l2(const double* p) {
-  double v;
-  asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ double2 ld_l2(const double2* p) {
-  double2 v;
-  asm volatile("ld.global.cg.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ float ld_l1f(const float* p) {
+__device__ __forceinline__ float ld_l1_if(const float* p, bool on) {
   float v;
-  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n mov.f32 %0, 0f00000000;\n @q ld.global.f32 %0, [%1];\n}"
+               : "=f"(v)
+               : "l"(p), "r"((unsigned)on)
+               : "memory");
   return v;
 }
-__device__ __forceinline__ float ld_l2f(const float* p) {
-  float v;
-  asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
-  return v;
+// the same for data written before the kernel; v keeps its value where the
+// predicate is off
+__device__ __forceinline__ void ldg_if(int4& v, const int4* p, bool on) {
+  asm("{\n .reg .pred q;\n setp.ne.u32 q, %5, 0;\n @q ld.global.nc.v4.s32 {%0, %1, %2, %3}, [%4];\n}"
+      : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
+      : "l"(p), "r"((unsigned)on));
 }
-__device__ __forceinline__ void st_globalf(float* p, float v) {
-  asm volatile("st.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
+__device__ __forceinline__ void ldg_if(double& v, const double* p, bool on) {
+  asm("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n @q ld.global.nc.f64 %0, [%1];\n}" : "+d"(v) : "l"(p), "r"((unsigned)on));
 }
-__device__ __forceinline__ void st_global(double* p, double v) {
+__device__ __forceinline__ void ldg_if(float& v, const float* p, bool on) {
+  asm("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n @q ld.global.nc.f32 %0, [%1];\n}" : "+f"(v) : "l"(p), "r"((unsigned)on));
+}
+__device__ __forceinline__ void st_value(double* p, double v) {
   asm volatile("st.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
 }
-__device__ __forceinline__ void st_global(double2* p, double2 v) {
+__device__ __forceinline__ void st_value(float* p, float v) {
+  asm volatile("st.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
+}
+__device__ __forceinline__ void st_value(double2* p, double2 v) {
   asm volatile("st.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(v.x), "d"(v.y) : "memory");
 }
-__device__ __forceinline__ void st_relaxed_gpu_int(int* p, int v) {
-  asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+// queue entries: written and polled by one CTA, so L1 may hold them
+__device__ __forceinline__ long long ld_queue(const long long* p) {
+  long long v;
+  asm volatile("ld.relaxed.cta.global.s64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
 }
-__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+__device__ __forceinline__ void st_queue(long long* p, long long v) {
+  asm volatile("st.relaxed.cta.global.s64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+// Brings the 32-byte sector at p into L1: a 16-byte copy whose destination
+// nobody reads (prefetch.global.L1 left the sector in L2 only: the consumer's
+// load still took an L2 round trip)
+__device__ __forceinline__ void touch_l1_if(unsigned scratch, const void* p, bool on) {
+  asm volatile(
+      "{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n @q cp.async.ca.shared.global [%0], [%1], 16;\n}" ::"r"(scratch),
+      "l"(p), "r"((unsigned)on)
+      : "memory");
+}
 
-__device__ inline unsigned short prio16(int size) { return (unsigned short)(__float_as_uint((float)size) >> 16); }
+// brings a record into L2
+__device__ __forceinline__ void prefetch_l2_if(const void* p, bool on) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %1, 0;\n @q cp.async.bulk.prefetch.L2.global [%0], 64;\n}" ::"l"(p),
+               "r"((unsigned)on)
+               : "memory");
+}
 
-// Inserts node v of priority p into dep[0..n) / pr[0..n) (n < 8), kept in
-// decreasing priority with ties in insertion order (registers only).
-__device__ inline void insert_by_priority(int (&dep)[8], unsigned (&pr)[8], int n, int v, unsigned p) {
-  int pos = 0;
-#pragma unroll
-  for (int t = 0; t < 8; ++t) pos += (t < n && pr[t] >= p) ? 1 : 0;
-#pragma unroll
-  for (int t = 7; t > 0; --t)
-    if (t > pos && t <= n) {
-      dep[t] = dep[t - 1];
-      pr[t] = pr[t - 1];
-    }
-#pragma unroll
-  for (int t = 0; t < 8; ++t)
-    if (t == pos) {
-      dep[t] = v;
-      pr[t] = p;
-    }
+// four flag words
+__device__ __forceinline__ void ld_flags(const unsigned* p, unsigned (&v)[4]) {
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+               : "l"(p)
+               : "memory");
+}
+
+// mailbox cells: every word is all ones until its value has arrived
+__device__ __forceinline__ bool mail_read(const double* p, double& v) {
+  v = ld_relaxed_gpu(p);
+  return __double_as_longlong(v) != -1ll;
+}
+__device__ __forceinline__ bool mail_read(const float* p, float& v) {
+  v = __int_as_float(ld_relaxed_gpu(reinterpret_cast<const int*>(p)));
+  return __float_as_int(v) != -1;
+}
+__device__ __forceinline__ bool mail_read(const double2* p, double2& v) {
+  const double* d = reinterpret_cast<const double*>(p);
+  v.x = ld_relaxed_gpu(d);
+  v.y = ld_relaxed_gpu(d + 1);
+  return __double_as_longlong(v.x) != -1ll && __double_as_longlong(v.y) != -1ll;
+}
+// a NaN whose bits are all ones travels as another NaN
+__device__ __forceinline__ double mail_word(double v) {
+  return __double_as_longlong(v) == -1ll ? __longlong_as_double(0x7ff8000000000000ll) : v;
+}
+__device__ __forceinline__ void mail_write(double* p, double v) { st_relaxed_gpu(p, mail_word(v)); }
+__device__ __forceinline__ void mail_write(float* p, float v) {
+  const int b = __float_as_int(v);
+  asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(b == -1 ? 0x7fc00000 : b) : "memory");
+}
+__device__ __forceinline__ void mail_write(double2* p, double2 v) {
+  double* d = reinterpret_cast<double*>(p);
+  st_relaxed_gpu(d, mail_word(v.x));
+  st_relaxed_gpu(d + 1, mail_word(v.y));
+}
+
+// The eight neighbours in the order of the reference's loops (jj outer, ii
+// inner, FlowRouting.f90:200-236): direction t, and 7 - t is its opposite.
+// dir_code packs the offset as (dj + 1) << 2 | (di + 1).
+__host__ __device__ constexpr int dir_di(int t) { return (t + (t >> 2)) % 3 - 1; }
+__host__ __device__ constexpr int dir_dj(int t) { return (t + (t >> 2)) / 3 - 1; }
+__host__ __device__ constexpr unsigned dir_code(int t) { return (unsigned)((dir_dj(t) + 1) << 2 | (dir_di(t) + 1)); }
+// direction of offset (di, dj), not (0, 0)
+__device__ __forceinline__ int dir_of(int di, int dj) {
+  const int c = 3 * (dj + 1) + di + 1;
+  return c - (c > 4 ? 1 : 0);
+}
+
+// One record per node: a 16-byte header, then the coefficients of its present
+// inputs (at most 8, in input order).
+//   codes  offset of input s (dir_code) in bits 4s..4s+3
+//   meta   bits 0-3 number of inputs (stream power: kNoRec a root, kNoMrec no
+//          receivers); 4-7 tile edges the node lies on (kWest ...); 8-15
+//          directions of the dependents; 16-19 stream power: offset of rec(k)
+//          and 20 whether it lies in another tile; 21-23 the dependent to
+//          continue with; 24-31 inputs that lie in another tile
+//   base   area: dx*dy*precip(k); stream power: ht(k)
+//   c      area: summed weight of the donor's slots targeting k
+//          stream power: kf*dt*(a*w)^m/l^n of the gated receiver slot
+constexpr unsigned kNoMrec = 14, kNoRec = 15;
+constexpr unsigned kWest = 1, kEast = 2, kSouth = 4, kNorth = 8;
+// the edges beyond which the neighbour in direction (di, dj) lies in another tile
+__device__ __forceinline__ unsigned edges_of(int di, int dj) {
+  return (di < 0 ? kWest : di > 0 ? kEast : 0u) | (dj < 0 ? kSouth : dj > 0 ? kNorth : 0u);
 }
 template <class T>
-__device__ inline void set_at(T (&a)[8], int n, T v) {
-#pragma unroll
-  for (int t = 0; t < 8; ++t)
-    if (t == n) a[t] = v;
-}
-template <class T>
-__device__ inline bool contains(const T (&a)[8], int n, T v) {
-  bool f = false;
-#pragma unroll
-  for (int t = 0; t < 8; ++t) f |= t < n && a[t] == v;
-  return f;
-}
+struct __align__(32) RecordT {
+  unsigned codes, meta;
+  double base;
+  T c[8];
+};
+static_assert(sizeof(RecordT<double>) == 96 && sizeof(RecordT<float>) == 64, "whole 32-byte sectors");
 
-// Coordinates of q if it is one of the 3x3 neighbours of (i, j), rows and
-// columns wrapping across the grid's edges; the row is found by range compares
-// (q lies in row j-1, j or j+1, or in a wrapped edge row), so the common
-// case needs no integer division.  False if q is not a neighbour.
-__device__ inline bool nbr_of(int i, int j, int q, int nx, int ny, int& qi, int& qj) {
-  const int r0 = j * nx;
-  int y;
-  if (q >= r0 && q < r0 + nx) y = j;
-  else if (q < r0 && q >= r0 - nx) y = j - 1;
-  else if (q >= r0 + nx && q < r0 + 2 * nx) y = j + 1;
-  else if (q >= 0 && q < nx) y = 0;
-  else if (q >= (ny - 1) * nx && q < ny * nx) y = ny - 1;
-  else return false;
-  const int x = q - y * nx;
-  int di = x - i, dj = y - j;
-  if (di > 1) di -= nx; else if (di < -1) di += nx;
-  if (dj > 1) dj -= ny; else if (dj < -1) dj += ny;
-  if (di < -1 || di > 1 || dj < -1 || dj > 1 || (di == 0 && dj == 0)) return false;
-  qi = x;
-  qj = y;
+// ---- record builders --------------------------------------------------------
+
+// neighbour of (i, j) in direction t; false when it lies beyond a non-cyclic edge
+__device__ __forceinline__ bool nbr_at(const Bounds& bd, int i, int j, int t, int& q) {
+  int x = i + dir_di(t), y = j + dir_dj(t);
+  if (x < 0) { if (!bd.xcyc) return false; x += bd.nx; }
+  if (x >= bd.nx) { if (!bd.xcyc) return false; x -= bd.nx; }
+  if (y < 0) { if (!bd.ycyc) return false; y += bd.ny; }
+  if (y >= bd.ny) { if (!bd.ycyc) return false; y -= bd.ny; }
+  q = x + y * bd.nx;
   return true;
 }
 
-// tile-major index of receiver q of (i, j), reporting a non-neighbour
-__device__ inline int nbr_g(const TileMap& tm, int i, int j, int q, int nx, int ny, int* err) {
-  int qi, qj;
-  if (!nbr_of(i, j, q, nx, ny, qi, qj)) {
+// direction of q from k = (i, j), reporting a node that is no neighbour (-1)
+__device__ inline int dir_to(const Bounds& bd, int i, int j, int q, int* err) {
+  const int qj = q / bd.nx, qi = q - qj * bd.nx;
+  int di = qi - i, dj = qj - j;
+  if (di > 1) di -= bd.nx; else if (di < -1) di += bd.nx;
+  if (dj > 1) dj -= bd.ny; else if (dj < -1) dj += bd.ny;
+  if (di < -1 || di > 1 || dj < -1 || dj > 1 || (di == 0 && dj == 0)) {
     atomicExch(err, DEV_NOT_ADJACENT);
-    qi = q % nx;
-    qj = q / nx;
+    return -1;
   }
-  return tm.g(qi, qj);
+  return dir_of(di, dj);
 }
 
-// The slots of d's receiver row that hold k, as bits (rows are padded with -1
-// past mnrec, so all eight slots are compared: two 16-byte loads)
-__device__ inline unsigned row_hits(const int* __restrict__ mrec, int d, int k) {
-  const int4* r = reinterpret_cast<const int4*>(mrec + (size_t)d * 8);
-  const int4 a = __ldg(r), b = __ldg(r + 1);
-  return (unsigned)(a.x == k) | (unsigned)(a.y == k) << 1 | (unsigned)(a.z == k) << 2 | (unsigned)(a.w == k) << 3 |
-         (unsigned)(b.x == k) << 4 | (unsigned)(b.y == k) << 5 | (unsigned)(b.z == k) << 6 | (unsigned)(b.w == k) << 7;
+// the edges of its tile (or of the grid) that (i, j) lies on
+__device__ __forceinline__ unsigned tile_edges(const Bounds& bd, int ts, int i, int j) {
+  const int x = i & (ts - 1), y = j & (ts - 1);
+  return (x == 0 ? kWest : 0u) | (x == ts - 1 || i == bd.nx - 1 ? kEast : 0u) | (y == 0 ? kSouth : 0u) |
+         (y == ts - 1 || j == bd.ny - 1 ? kNorth : 0u);
 }
 
-// One record line per node, tile-major: the inputs a node gathers, their
-// coefficients, and its dependents (tile-major indices, -1 past the last;
-// dependents largest priority first).
-//   area:          c[t] = summed weight of input (donor) t's slots targeting k
-//   stream power:  c[t] = kf*dt*(a*w)^m/l^n of gated receiver slot t
-// The coefficients are double in the plain form and float in the mixed one.
+// mmask[k] (k_mfd_receivers): bits 0-7 the loop directions that hold a
+// receiver slot, in slot order; bits 8-15 the directions of the distinct
+// receivers.  The two differ only beside a free, non-cyclic edge, where the
+// reference lists a clamped neighbour again.
+
+// Area: inputs are k's distinct donors in direction order with the summed
+// weight of their slots targeting k; dependents are k's distinct receivers.
 template <class T>
-struct __align__(128) RegionLineT {
-  T c[8];
-  int dep[8];
-  int inp[8];
-};
-using RegionLine = RegionLineT<double>;
-using RegionLineF = RegionLineT<float>;
-static_assert(sizeof(RegionLine) == 128 && sizeof(RegionLineF) == 128, "one line per node");
-
-// a line in registers: the words that hold data (128 bytes, or 96 with float
-// coefficients), read through the read-only path
-template <class T>
-struct LineRegsT {
-  static constexpr int kWords = (8 * (int)sizeof(T) + 64) / 16;
-  static constexpr int kDep = 2 * (int)sizeof(T);  // int index of dep[0]
-  union {
-    int4 v[kWords];
-    T c[8];
-    int s[4 * kWords];
-  };
-  __device__ explicit LineRegsT(const RegionLineT<T>* p) {
+__global__ void __launch_bounds__(256) k_acc_records(Bounds bd, int ts, double dxdy, const int* __restrict__ mmask,
+                                                     const int* __restrict__ mrec, const double* __restrict__ mwrec,
+                                                     const double* __restrict__ precip, RecordT<T>* __restrict__ rec,
+                                                     unsigned short* __restrict__ wmeta) {
+  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
+  if (i >= bd.nx || j >= bd.ny) return;
+  const int k = i + j * bd.nx;
+  const unsigned edges = tile_edges(bd, ts, i, j);
+  unsigned codes = 0, far = 0;
+  int n = 0;
+  RecordT<T>* r = rec + k;
 #pragma unroll
-    for (int t = 0; t < kWords; ++t) v[t] = __ldg(reinterpret_cast<const int4*>(p) + t);
-  }
-  __device__ int dep(int t) const { return s[kDep + t]; }
-  __device__ int inp(int t) const { return s[kDep + 8 + t]; }
-};
-using LineRegs = LineRegsT<double>;
-
-// stream-power node metadata kept in the value array's water word until the
-// node is computed: rec (tile-major, or -1 for a root) and whether mnrec > 0
-__device__ inline double pack_meta(int rec_g, bool has_mrec) {
-  const long long v = (long long)(unsigned)rec_g | (has_mrec ? (1ll << 40) : 0ll);
-  return __longlong_as_double(v);
-}
-__device__ inline void unpack_meta(double w, int& rec_g, bool& has_mrec) {
-  const long long v = __double_as_longlong(w);
-  rec_g = (int)(unsigned)(v & 0xffffffffll);
-  has_mrec = (v >> 40) & 1;
-}
-
-// ---- line builders (natural node order in, tile-major out) ------------------
-
-// Area: inputs are k's distinct donors among its 3x3 neighbours (jj outer, ii
-// inner, as FlowRouting.f90's neighbour loops) with the summed weight of
-// their slots targeting k; dependents are k's distinct receivers.  cnt0 gets
-// the in-tile input count plus one if any input lies in another tile (that
-// token is released by the inbox); xcnt the number of cross-tile inputs.
-template <class T>
-__global__ void k_acc_lines_t(Bounds bd, TileMap tm, double dxdy, const int* __restrict__ mrec,
-                              const int* __restrict__ mnrec, const double* __restrict__ mwrec,
-                              const double* __restrict__ precip, const int* __restrict__ prio,
-                              RegionLineT<T>* __restrict__ line, T* __restrict__ val,
-                              unsigned char* __restrict__ cnt0, int* __restrict__ xcnt, int* err) {
-  const int nx = bd.nx, ny = bd.ny, nn = nx * ny;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
-    const int i = k % nx, j = k / nx;
-    const int gk = tm.g(i, j);
-    const int tile = gk >> tm.lr();
-    const size_t o = (size_t)k * 8;
-    const int nr = mnrec[k];
-    int mr[8], dep[8];
-    unsigned pr[8];
-    {  // the row past mnrec holds -1
-      const int4 ra = __ldg(reinterpret_cast<const int4*>(mrec + o)), rb = __ldg(reinterpret_cast<const int4*>(mrec + o) + 1);
-      mr[0] = ra.x; mr[1] = ra.y; mr[2] = ra.z; mr[3] = ra.w;
-      mr[4] = rb.x; mr[5] = rb.y; mr[6] = rb.z; mr[7] = rb.w;
-    }
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      dep[t] = -1;
-      pr[t] = 0u;
-    }
-    int rn = 0;
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      if (t >= nr) break;
-      const int q = mr[t];
-      if (contains(mr, t, q)) continue;
-      insert_by_priority(dep, pr, rn++, nbr_g(tm, i, j, q, nx, ny, err), prio16(prio[q]));
-    }
-    int inp[8], seen[8];
-    double aw[8];
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      aw[t] = 0.0;
-      inp[t] = -1;
-    }
-    int an = 0, ns = 0, nin = 0, nx_in = 0;
-#pragma unroll
-    for (int jj = -1; jj <= 1; ++jj) {
-      int y = j + jj;
-      if (y < 0) { if (!bd.ycyc) continue; y += ny; }
-      if (y >= ny) { if (!bd.ycyc) continue; y -= ny; }
-#pragma unroll
-      for (int ii = -1; ii <= 1; ++ii) {
-        int x = i + ii;
-        if (x < 0) { if (!bd.xcyc) continue; x += nx; }
-        if (x >= nx) { if (!bd.xcyc) continue; x -= nx; }
-        const int d = x + y * nx;
-        if (d == k || contains(seen, ns, d)) continue;
-        set_at(seen, ns++, d);
-        const unsigned hm = row_hits(mrec, d, k);
-        double wsum = 0.0;
-        int hits = 0;
-#pragma unroll
-        for (int t = 0; t < 8; ++t)
-          if (hm >> t & 1u) {
-            const double w = mwrec[(size_t)d * 8 + t];
-            wsum = hits ? wsum + w : w;
-            ++hits;
-          }
-        if (hits && an < 8) {
-          const int gd = tm.g(x, y);
-          set_at(inp, an, gd);
-          set_at(aw, an++, wsum);
-          if ((gd >> tm.lr()) == tile) ++nin; else ++nx_in;
+  for (int t = 0; t < 8; ++t) {
+    int d;
+    if (!nbr_at(bd, i, j, t, d)) continue;
+    const int m = __ldg(&mmask[d]);
+    const int ot = 7 - t;
+    if (!((m >> (8 + ot)) & 1)) continue;
+    const size_t o = (size_t)d * 8;
+    double w;
+    if ((m & 255) == (m >> 8)) {
+      w = __ldg(&mwrec[o + __popc(m & ((1 << ot) - 1))]);
+    } else {  // beside a free edge: d may list k twice
+      const int nr = __popc(m & 255);
+      int hits = 0;
+      w = 0.0;
+      for (int s = 0; s < nr; ++s)
+        if (mrec[o + s] == k) {
+          const double ws = mwrec[o + s];
+          w = hits ? w + ws : ws;
+          ++hits;
         }
-      }
     }
-    RegionLineT<T> L;
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      L.c[t] = (T)aw[t];
-      L.dep[t] = dep[t];
-      L.inp[t] = inp[t];
-    }
-    line[gk] = L;
-    val[gk] = (T)(dxdy * precip[k]);
-    cnt0[gk] = (unsigned char)(nin + (nx_in > 0 ? 1 : 0));
-    xcnt[gk] = nx_in;
+    codes |= dir_code(t) << (4 * n);
+    far |= ((edges & edges_of(dir_di(t), dir_dj(t))) ? 1u : 0u) << n;
+    r->c[n++] = (T)w;
   }
+  const unsigned deps = (unsigned)(mmask[k] >> 8) & 255u;
+  r->codes = codes;
+  r->meta = (unsigned)n | (edges << 4) | (deps << 8) | (far << 24);
+  r->base = dxdy * precip[k];
+  wmeta[k] = (unsigned short)((unsigned)n | (deps << 8));
 }
 
 // Stream power: inputs are k's gated receiver slots (ht(k) >= ht(q) for n = 1,
 // > otherwise: the terms StreamPowerLaw.f90:108-114 / 152-158 include), in
 // mrec slot order, duplicates kept; the counter also waits for rec(k), whose
 // water the node compares against.  Dependents are the donors that read
-// k's new elevation (gated) or its water (rec == k).  The value array starts
-// as (ht, metadata) and ends as (h, water).
+// k's new elevation (gated) or its water (rec == k).
 template <class T>
-__global__ void k_spl_lines_t(Bounds bd, TileMap tm, int n_is_one, double kfsed, double dt, double m, double n,
-                              const int* __restrict__ rec, const int* __restrict__ mrec,
-                              const int* __restrict__ mnrec, const double* __restrict__ mwrec,
-                              const double* __restrict__ mlrec, const double* __restrict__ h,
-                              const double* __restrict__ b, const double* __restrict__ kf,
-                              const double* __restrict__ a, const int* __restrict__ prio,
-                              const double* __restrict__ ltab, const T* __restrict__ lpow,
-                              RegionLineT<T>* __restrict__ line, double2* __restrict__ hw,
-                              unsigned char* __restrict__ cnt0, int* __restrict__ xcnt, int* err) {
-  const int nx = bd.nx, ny = bd.ny, nn = nx * ny;
-  const double l_diag = __ldg(&ltab[0]), l_dy = __ldg(&ltab[1]);
-  const T lp_diag = __ldg(&lpow[0]), lp_dy = __ldg(&lpow[1]), lp_dx = __ldg(&lpow[3]);
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
-    const int i = k % nx, j = k / nx;
-    const int gk = tm.g(i, j);
-    const int tile = gk >> tm.lr();
-    const size_t o = (size_t)k * 8;
-    const double htk = h[k];
-    const int nr = mnrec[k];
-    const int r = rec[k];
+__global__ void __launch_bounds__(256) k_spl_records(
+    Bounds bd, int ts, int n_is_one, double kfsed, double dt, double m, const int* __restrict__ recv,
+    const int* __restrict__ mmask, const int* __restrict__ mrec, const double* __restrict__ mwrec,
+    const double* __restrict__ mlrec, const double* __restrict__ h, const double* __restrict__ b,
+    const double* __restrict__ kf, const double* __restrict__ a, const double* __restrict__ ltab,
+    const T* __restrict__ lpow, RecordT<T>* __restrict__ rec, unsigned short* __restrict__ wmeta, int* err) {
+  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
+  if (i >= bd.nx || j >= bd.ny) return;
+  const int k = i + j * bd.nx;
+  const double htk = h[k];
+  const int mk = mmask[k];
+  const int r = recv[k];
+  const unsigned edges = tile_edges(bd, ts, i, j);
+  unsigned codes = 0, waits = 0, far = 0, rcode = 0;
+  int n = 0;
+  RecordT<T>* out = rec + k;
+  if (r != k) {
     const double kk = ((kfsed > 0.0 && (htk - b[k]) > 1.0) ? kfsed : kf[k]) * dt;
     const double ak = a[k];
-    int qv[8], inp[8], dep[8];
-    unsigned pr[8];
-    T fact[8];
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      qv[t] = -1;
-      inp[t] = -1;
-      dep[t] = -1;
-      pr[t] = 0u;
-      fact[t] = 0;
-    }
-    int nq = 0;
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      if (t >= nr) break;
-      const int q = mrec[o + t];
-      if (n_is_one ? (htk >= h[q]) : (htk > h[q])) {
-        const double w = mwrec[o + t], l = mlrec[o + t];
-        // l^n from the table of the neighbour lengths: l is one of its three
-        // values (diagonal at 0, dy at 1, dx at 3; equal values have equal powers)
-        const T ln = l == l_diag ? lp_diag : l == l_dy ? lp_dy : lp_dx;
-        if constexpr (sizeof(T) == sizeof(double)) {
-          set_at(fact, nq, n_is_one ? kk * pow(ak * w, m) / l : kk * pow(ak * w, m) / ln);
-        } else {  // mixed precision: the erosion factor in FP32
-          const float kf32 = (float)kk, aw32 = (float)(ak * w), l32 = (float)l;
-          set_at(fact, nq, n_is_one ? kf32 * powf(aw32, (float)m) / l32 : kf32 * powf(aw32, (float)m) / ln);
-        }
-        set_at(inp, nq, nbr_g(tm, i, j, q, nx, ny, err));
-        set_at(qv, nq++, q);
+    const int nr = __popc(mk & 255);
+    const size_t o = (size_t)k * 8;
+    const bool plain = (mk & 255) == (mk >> 8);
+    int dirs = mk & 255;
+    for (int s = 0; s < nr; ++s) {
+      int t = __ffs(dirs) - 1;  // the loop direction of slot s
+      dirs &= dirs - 1;
+      int q;
+      double l;
+      if (plain) {
+        nbr_at(bd, i, j, t, q);
+        l = __ldg(&ltab[t + (t >> 2)]);
+      } else {  // a clamped neighbour keeps the length of its loop direction
+        q = mrec[o + s];
+        l = mlrec[o + s];
+        t = dir_to(bd, i, j, q, err);
+        if (t < 0) continue;
       }
-    }
-    // distinct inputs: gated receivers and rec(k), split by tile
-    int nin = 0, nx_in = 0;
-    const int rg = r != k ? nbr_g(tm, i, j, r, nx, ny, err) : -1;
-    if (r != k) {
-#pragma unroll
-      for (int t = 0; t < 8; ++t)
-        if (t < nq && !contains(qv, t, qv[t])) {
-          if ((inp[t] >> tm.lr()) == tile) ++nin; else ++nx_in;
-        }
-      if (!contains(qv, nq, r)) {
-        if ((rg >> tm.lr()) == tile) ++nin; else ++nx_in;
+      if (!(n_is_one ? (htk >= h[q]) : (htk > h[q]))) continue;
+      const double w = mwrec[o + s];
+      // l^n from the table of the neighbour lengths: l is one of its three
+      // values (diagonal at 0, dy at 1, dx at 3; equal values have equal powers)
+      const T ln = l == __ldg(&ltab[0]) ? __ldg(&lpow[0]) : l == __ldg(&ltab[1]) ? __ldg(&lpow[1]) : __ldg(&lpow[3]);
+      T f;
+      if constexpr (sizeof(T) == sizeof(double)) {
+        f = n_is_one ? kk * pow(ak * w, m) / l : kk * pow(ak * w, m) / ln;
+      } else {  // mixed precision: the erosion factor in FP32
+        const float kf32 = (float)kk, aw32 = (float)(ak * w), l32 = (float)l;
+        f = n_is_one ? kf32 * powf(aw32, (float)m) / l32 : kf32 * powf(aw32, (float)m) / ln;
       }
+      codes |= dir_code(t) << (4 * n);
+      far |= ((edges & edges_of((t + (t >> 2)) % 3 - 1, (t + (t >> 2)) / 3 - 1)) ? 1u : 0u) << n;
+      waits |= 1u << t;
+      out->c[n++] = f;
     }
-    int dn = 0, ns = 0;
-    int seen[8];
-#pragma unroll
-    for (int jj = -1; jj <= 1; ++jj) {
-      int y = j + jj;
-      if (y < 0) { if (!bd.ycyc) continue; y += ny; }
-      if (y >= ny) { if (!bd.ycyc) continue; y -= ny; }
-#pragma unroll
-      for (int ii = -1; ii <= 1; ++ii) {
-        int x = i + ii;
-        if (x < 0) { if (!bd.xcyc) continue; x += nx; }
-        if (x >= nx) { if (!bd.xcyc) continue; x -= nx; }
-        const int d = x + y * nx;
-        if (d == k || contains(seen, ns, d)) continue;
-        set_at(seen, ns++, d);
-        const int rd = rec[d];
-        if (rd == d) continue;
-        const bool hits = row_hits(mrec, d, k) != 0u;
-        const bool gated = hits && (n_is_one ? (h[d] >= htk) : (h[d] > htk));
-        if ((gated || rd == k) && dn < 8) insert_by_priority(dep, pr, dn++, tm.g(x, y), prio16(prio[d]));
-      }
+    const int rd = dir_to(bd, i, j, r, err);
+    if (rd >= 0) {
+      rcode = dir_code(rd) | ((edges & edges_of((rd + (rd >> 2)) % 3 - 1, (rd + (rd >> 2)) / 3 - 1)) ? 16u : 0u);
+      waits |= 1u << rd;
     }
-    RegionLineT<T> L;
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      L.c[t] = fact[t];
-      L.dep[t] = dep[t];
-      L.inp[t] = inp[t];
-    }
-    line[gk] = L;
-    hw[gk] = make_double2(htk, pack_meta(rg, nr > 0));
-    cnt0[gk] = (unsigned char)(nin + (nx_in > 0 ? 1 : 0));
-    xcnt[gk] = nx_in;
   }
+  unsigned deps = 0, prefer = 0;
+  double amax = -1.0;  // the dependent with the largest area has the longest way up behind it
+#pragma unroll
+  for (int t = 0; t < 8; ++t) {
+    int d;
+    if (!nbr_at(bd, i, j, t, d)) continue;
+    const int rd = __ldg(&recv[d]);
+    if (rd == d) continue;
+    const bool hits = (__ldg(&mmask[d]) >> (15 - t)) & 1;
+    const bool gated = hits && (n_is_one ? (h[d] >= htk) : (h[d] > htk));
+    if (gated || rd == k) {
+      deps |= 1u << t;
+      const double ad = __ldg(&a[d]);
+      if (ad > amax) {
+        amax = ad;
+        prefer = (unsigned)t;
+      }
+    }
+  }
+  out->codes = codes;
+  const unsigned ni = r == k ? kNoRec : (mk & 255) ? (unsigned)n : kNoMrec;
+  out->meta = ni | (edges << 4) | (deps << 8) | (rcode << 16) | (prefer << 21) | (far << 24);
+  out->base = htk;
+  wmeta[k] = (unsigned short)((unsigned)__popc(waits) | (deps << 8));
 }
 
 // l^n for the nine neighbour lengths of find_receiver / find_mult_rec, with
@@ -434,497 +390,354 @@ __global__ void k_length_pow(const double* __restrict__ ltab, double n, double* 
   }
 }
 
-// ---- node operations: a warp segment per node -------------------------------------
-// A node is computed by a segment of W = 32 / NPW lanes of a warp (NPW nodes
-// per warp).  Lane t < 8 of the segment holds slot t of the node's line
-// (coefficient, input, dependent), loads input t and forms term t; the
-// node's sums then run over the present slots in slot order -- the order of
-// the queue engine in fsb_flow.cu -- with every lane of the segment doing the
-// same scalar arithmetic on shuffled terms.  The area sums issue all eight
-// shuffles and mask absent slots in the adds (an early exit serialised the
-// shuffles and measured slower); the one-node Newton loop of the stream power
-// law stops at the last present slot (measured faster: it runs once per
-// iteration).  All segments of a warp execute
-// the same instruction stream: a segment without a node, or whose node needs
-// fewer Newton iterations, runs along without effect, so warp-collective
-// shuffles and ballots stay convergent.  Lane 0 of a segment stores the
-// node's value.  run() returns the dependent in this lane's slot (-1 for
-// none).
-constexpr unsigned FULL = 0xffffffffu;
+// ---- node operations: eight lanes per node -------------------------------------
+// A node is computed by a segment of eight lanes of a warp: lane t holds input
+// t of the node's record, loads its value and forms term t; the terms then
+// meet in the warp's row of shared memory (two 16-byte accesses per term
+// instead of shuffling the halves of two doubles) and every lane adds them up
+// in input order -- the order of the queue engine in fsb_flow.cu -- so all
+// eight do the same scalar arithmetic.  All segments of a warp execute the
+// same instruction stream: a segment without a node, or whose node needs
+// fewer Newton iterations, runs along without effect.
+//
+// Inputs of this tile are read through L1 (a store updates the line, which
+// the node's inputs bring in before it is computed), those of other tiles
+// from this tile's mailbox.
+constexpr int kSegLanes = 8, kSegs = 32 / kSegLanes;
+constexpr int kRowStride = 8 * 16 + 16;  // bytes of a segment's terms, padded against bank conflicts
 
-__device__ __forceinline__ float ld_l1(const float* p) { return ld_l1f(p); }
-__device__ __forceinline__ float ld_l2(const float* p) { return ld_l2f(p); }
+// a tile of this CTA: its first node, its size
+struct TileInfo {
+  int x0, y0, w, h;
+};
 
-// An input's value: this tile's nodes through L1, other tiles' (which arrive
-// through the inbox, after an acquire at GPU scope) from L2.  Measured on
-// B200: a shared-memory cache of produced values in front of these loads
-// was slower (its fences and the L1 capacity it took cost more than the
-// round trips it saved).
-struct TileLoc {
-  int tile, lr;
-  template <class V>
-  __device__ V load(const V* arr, int q) const {
-    return (q >> lr) == tile ? ld_l1(arr + q) : ld_l2(arr + q);
+// Cells of the rim around a w x h tile of side 2^LT: the row above, the row
+// below, then the left and the right column.
+template <int LT>
+struct Rim {
+  static constexpr int kTS = 1 << LT;
+  static constexpr int kCells = rim_cells(LT), kWords = rim_words(LT);
+  __device__ static __forceinline__ int index(int x, int y, int w, int h) {
+    if (y < 0) return x + 1;
+    if (y >= h) return kTS + 3 + x;
+    return 2 * (kTS + 2) + (x < 0 ? y : kTS + y);
+  }
+  // false for a cell that a w x h tile does not have
+  __device__ static __forceinline__ bool coords(int c, int w, int h, int& x, int& y) {
+    if (c < kTS + 2) { x = c - 1; y = -1; return x <= w; }
+    if (c < 2 * (kTS + 2)) { x = c - (kTS + 3); y = h; return x <= w; }
+    if (c < 2 * (kTS + 2) + kTS) { x = -1; y = c - 2 * (kTS + 2); return y < h; }
+    x = w; y = c - 2 * (kTS + 2) - kTS;
+    return c < 4 * kTS + 4 && y < h;
   }
 };
 
-// A lane's segment: its lane within the segment and the segment's first lane.
-struct Seg {
-  int sl, base;
-  __device__ double shfl(double v, int s) const { return __shfl_sync(FULL, v, base + s); }
-  __device__ float shfl(float v, int s) const { return __shfl_sync(FULL, v, base + s); }
-  // bit t: predicate of lane t (< 8) of this segment
-  __device__ unsigned slots(bool p) const { return (__ballot_sync(FULL, p) >> base) & 0xffu; }
+// What a lane knows about its segment's node: natural index k, local index id
+// (tile of this CTA << 2*LT | y << LT | x), and where cross-tile inputs lie.
+template <class V, int LT>
+struct NodeCtx {
+  int k, id, nx;
+  int sl;                // lane within the segment
+  unsigned char* row;    // the segment's terms in shared memory
+  const TileInfo* tab;   // shared memory
+  const V* mbox;         // all tiles' cells
+  int tile0, tile_step;
+  __device__ __forceinline__ int near(unsigned code) const {
+    return k + ((int)(code >> 2) - 1) * nx + (int)(code & 3u) - 1;
+  }
+  __device__ __forceinline__ const V* far(unsigned code) const {
+    const int slot = id >> (2 * LT);
+    const int lx = id & ((1 << LT) - 1), ly = (id >> LT) & ((1 << LT) - 1);
+    const TileInfo ti = tab[slot];
+    return mbox + (size_t)(tile0 + slot * tile_step) * Rim<LT>::kCells +
+           Rim<LT>::index(lx + (int)(code & 3u) - 1, ly + (int)(code >> 2) - 1, ti.w, ti.h);
+  }
+  // every lane's term(s), in input order
+  template <class T, class F>
+  __device__ __forceinline__ void exchange(T a, F add) const {
+    T* r = reinterpret_cast<T*>(row);
+    __syncwarp();
+    r[sl] = a;
+    __syncwarp();
+    struct __align__(16) Quad { T v[16 / sizeof(T)]; } v[8 * sizeof(T) / 16];
+#pragma unroll
+    for (int i = 0; i < (int)(8 * sizeof(T) / 16); ++i) v[i] = reinterpret_cast<const Quad*>(row)[i];
+#pragma unroll
+    for (int s = 0; s < 8; ++s) add(v[s / (16 / sizeof(T))].v[s % (16 / sizeof(T))]);
+  }
+  template <class T, class F>
+  __device__ __forceinline__ void exchange(T a, T b, F add) const {
+    struct __align__(2 * sizeof(T)) Pair { T a, b; };
+    Pair* r = reinterpret_cast<Pair*>(row);
+    __syncwarp();
+    r[sl] = Pair{a, b};
+    __syncwarp();
+    Pair v[8];
+#pragma unroll
+    for (int s = 0; s < 8; ++s) v[s] = r[s];
+#pragma unroll
+    for (int s = 0; s < 8; ++s) add(v[s].a, v[s].b);
+  }
 };
 
-// The slot fields of a node's line for this lane (nothing for an idle segment).
+// The record of this lane's node (without inputs and dependents for an idle
+// segment).  It is loaded as soon as the node is known, before the previous
+// node's bookkeeping is finished.
 template <class T>
 struct Slot {
+  int4 hd = {0, 0, 0, 0};
   T c = 0;
-  int d = -1, q = -1;
-  bool owner = false;  // lane < 8 of the segment: the slot is this lane's
-  __device__ Slot(const RegionLineT<T>* line, int g, const Seg& sg) {
-    if (g >= 0) {  // lanes 8.. of a wide segment read the same slots (one line, coalesced)
-      const RegionLineT<T>* L = line + g;
-      const int t = sg.sl & 7;
-      c = __ldg(&L->c[t]);
-      d = __ldg(&L->dep[t]);
-      q = __ldg(&L->inp[t]);
-      owner = sg.sl < 8;
-    }
+  unsigned codes, meta;
+  double base;
+  __device__ __forceinline__ void load(const RecordT<T>* r, bool on, int sl) {
+    ldg_if(hd, reinterpret_cast<const int4*>(r), on);
+    ldg_if(c, &r->c[sl], on);
   }
-  // the dependent's line (lanes 0-7) and its own entry (lanes 8-15, or the
-  // same lanes in 8-lane segments) into L1
-  template <class E>
-  __device__ void prefetch(const void* lines, const E* entries, const Seg& sg, int w) const {
-    if (d < 0) return;
-    if (sg.sl < 8) prefetch_l1(reinterpret_cast<const RegionLineT<T>*>(lines) + d);
-    if (w > 8 ? (sg.sl >= 8 && sg.sl < 16) : true) prefetch_l1(entries + d);
+  __device__ __forceinline__ void open(bool on) {
+    codes = (unsigned)hd.x;
+    meta = on ? (unsigned)hd.y : kNoRec;
+    base = __hiloint2double(hd.w, hd.z);
   }
+  // inputs of the node; whether this lane has one, its offset, whether it lies in another tile
+  __device__ __forceinline__ unsigned n() const { return meta & 15u; }
+  __device__ __forceinline__ bool mine(int sl) const { return (unsigned)sl < n() && n() < kNoMrec; }
+  __device__ __forceinline__ unsigned code(int sl) const { return (codes >> (4 * sl)) & 15u; }
+  __device__ __forceinline__ bool far(int sl) const { return (meta >> (24 + sl)) & 1u; }
 };
 
 // a(k) = dx*dy*precip(k) + sum over donors of a(d)*w(d->k) (FlowRouting.f90:109-115)
-template <class T, int NPW>
-struct AccRegionOpT {
-  using Value = T;
-  static constexpr int kThreads = 512, kNpw = NPW, kId = sizeof(T) == sizeof(double) ? 0 : 3;
-  const RegionLineT<T>* line;
+template <class T_>
+struct AccOp {
+  using T = T_;
+  using Value = T_;
+  static constexpr int kId = sizeof(T_) == sizeof(double) ? 0 : 1;
+  static constexpr bool kPrefer = false;  // records name a dependent to continue with
+  const RecordT<T>* rec;
   T* val;
-  __device__ int run(int g, const Seg& sg, const TileLoc& vc) const {
-    const Slot<T> sl(line, g, sg);
-    const bool mine = sl.owner && sl.q >= 0;
-    T x = 0;
-    if (mine) x = vc.load(val, sl.q);
-    sl.prefetch(line, val, sg, 32 / NPW);
-    const T term = x * sl.c;
-    const unsigned present = sg.slots(mine);
-    const int npres = __popc(present);  // slots fill from 0: the present ones are 0..npres-1
-    T acc = g >= 0 ? ld_l1(val + g) : T(0);  // dx*dy*precip(k), stored by the line builder
-#pragma unroll
-    for (int s = 0; s < 8; ++s) {
-      const T v = sg.shfl(term, s);
-      if (s < npres) acc = acc + v;
-    }
-    if (g >= 0 && sg.sl == 0) {
-      if constexpr (sizeof(T) == sizeof(double)) st_global(val + g, acc);
-      else st_globalf(val + g, acc);
-    }
-    return sl.owner ? sl.d : -1;
-  }
-};
-template <int NPW> using AccRegionOpN = AccRegionOpT<double, NPW>;
-template <int NPW> using AccRegionOpFN = AccRegionOpT<float, NPW>;
-
-// x^n and x^(n-1) for the Newton update (as NewtonPow in fsb_flow.cu): for
-// n = 1.5 as x*sqrt(x) and sqrt(x); otherwise x*x^(n-1) with one pow for x > 0.
-struct RegionPow {
-  double n;
-  int half3;
-  __device__ void eval(double x, double& pn, double& pn1) const {
-    if (half3) {
-      const double r = sqrt(x);
-      pn = x * r;
-      pn1 = r;
-    } else if (x > 0.0) {
-      pn1 = pow(x, n - 1.0);
-      pn = x * pn1;
-    } else {
-      pn = pow(x, n);
-      pn1 = pow(x, n - 1.0);
-    }
+  template <int LT, class Touch>
+  __device__ __forceinline__ unsigned run(const NodeCtx<T, LT>& nc, const Slot<T>& sl, bool on, T& out, Touch touch) const {
+    const unsigned code = sl.code(nc.sl);
+    const bool mine = sl.mine(nc.sl), far = mine && sl.far(nc.sl);
+    T x = ld_l1_if(val + nc.near(code), mine && !far);
+    if (far) mail_read(nc.far(code), x);
+    touch(sl.meta);
+    T acc = (T)sl.base;
+    nc.exchange(mine ? x * sl.c : T(0), [&](T a) { acc = acc + a; });
+    if (on && nc.sl == 0) st_value(val + nc.k, acc);
+    out = acc;
+    return sl.meta;
   }
 };
 
 // implicit stream power law over the multiple receivers with g == 0
-// (StreamPowerLaw.f90:92-177): hw[g] = (new h, water).  For n = 1.5 each
-// Newton iteration evaluates the receivers' x*sqrt(x) in parallel, one per
-// lane; for other n lane 0 of the segment iterates with pow (a shuffle in a
-// loop with pow does not compile).
-template <bool HALF3, int NPW>
-struct SplRegionOpN {
+// (StreamPowerLaw.f90:92-177): hw[k] = (new h, water).  MODE 0: n = 1, closed
+// form; 1: n = 1.5, whose powers are x*sqrt(x) and sqrt(x) (sqrt is correctly
+// rounded); 2: other n, x*x^(n-1) with one pow for x > 0.
+//
+// T = double: the reference's arithmetic.  T = float (mixed precision): the
+// solve for the increment d = h - ht in FP32.  Elevations, water levels and
+// the h update stay FP64; the distances to the receivers' new elevations,
+// ht(k) - h(q), are taken in FP64 and rounded once.  n = 1: d =
+// -sum f*(ht - hq) / (1 + sum f), the closed form of StreamPowerLaw.f90:108-118
+// rewritten for the increment; otherwise Newton on d (x = max(0, ht - hq + d),
+// :146-162) with the reference's tolerance and relaxation.
+// x^n and x^(n-1) for x >= 0
+template <int MODE>
+__device__ __forceinline__ void newton_pow(double x, double n, double& pn, double& pn1) {
+  pn1 = MODE == 1 ? sqrt(x) : pow(x, n - 1.0);
+  pn = MODE == 1 || x > 0.0 ? x * pn1 : pow(x, n);
+}
+template <int MODE>
+__device__ __forceinline__ void newton_pow(float x, float n, float& pn, float& pn1) {
+  pn1 = MODE == 1 ? sqrtf(x) : powf(x, n - 1.0f);
+  pn = MODE == 1 || x > 0.0f ? x * pn1 : powf(x, n);
+}
+
+template <class T_, int MODE>
+struct SplOp {
+  using T = T_;
   using Value = double2;
-  static constexpr int kThreads = HALF3 ? 512 : 256, kNpw = NPW, kId = HALF3 ? 1 : 2;
-  const RegionLine* line;
-  double2* hw;
-  RegionPow np;
-  double omega;
-  int n_is_one;
+  static constexpr bool kPrefer = true;
+  static constexpr int kId = 2 + MODE + (sizeof(T_) == sizeof(double) ? 0 : 3);
+  const RecordT<T>* rec;
+  double2* val;
+  T n, omega;
   int* err;
-  __device__ int run(int g, const Seg& sg, const TileLoc& vc) const {
-    const Slot<double> sl(line, g, sg);
-    int rg = -1;
-    bool has_mrec = false;
-    double ht = 0.0;
-    if (g >= 0) {
-      const double2 self = ld_l1(hw + g);
-      unpack_meta(self.y, rg, has_mrec);
-      ht = self.x;
+  template <int LT, class Touch>
+  __device__ __forceinline__ unsigned run(const NodeCtx<double2, LT>& nc, const Slot<T>& sl, bool on, double2& out,
+                                             Touch touch) const {
+    constexpr bool kInc = sizeof(T) == sizeof(float);  // solve for the increment
+    const unsigned ni = sl.n(), code = sl.code(nc.sl), rc = (sl.meta >> 16) & 15u;
+    const bool has_rec = ni != kNoRec, mine = sl.mine(nc.sl);
+    const bool far = mine && sl.far(nc.sl), rfar = (sl.meta >> 20) & 1u;
+    const double ht = sl.base;
+    double hq = ld_l1_if(&val[nc.near(code)].x, mine && !far);
+    double wr = ld_l1_if(&val[nc.near(rc)].y, has_rec && !rfar);
+    if (far || (has_rec && rfar)) {
+      if (far) hq = ld_relaxed_gpu(&nc.far(code)->x);
+      if (has_rec && rfar) wr = ld_relaxed_gpu(&nc.far(rc)->y);
     }
-    const bool mine = sl.owner && sl.q >= 0;
-    const unsigned present = sg.slots(mine);
-    const int npres = __popc(present);
-    double hq = 0.0, w = 0.0;
-    if (rg >= 0) {
-      if (mine) hq = vc.load(hw, sl.q).x;
-      if (sg.sl == 0) w = vc.load(hw, rg).y;
-    }
-    const double wr = sg.shfl(w, 0);
-    sl.prefetch(line, hw, sg, 32 / NPW);  // the dependent's line and own entry (ht, rec)
-    const double elev = ht;
-    const bool solve = rg >= 0 && elev > wr && has_mrec;
-    double hk = ht;
-    if (n_is_one) {
-      const double tf = sl.c * hq;
-      double f = elev, df = 1.0;
-#pragma unroll
-      for (int s = 0; s < 8; ++s) {
-        const double a = sg.shfl(tf, s), b = sg.shfl(sl.c, s);
-        if (s < npres) {
+    touch(sl.meta);
+    const bool above = has_rec && ht > wr;
+    const bool solve = above && ni != kNoMrec;
+    // the unknown: h itself, or its increment over ht; q: h or ht - h of the receiver
+    T u = kInc ? T(0) : (T)ht;
+    const T q = kInc ? (T)(ht - hq) : (T)hq;
+    if constexpr (MODE == 0) {
+      T f = kInc ? T(0) : (T)ht, df = 1;
+      nc.exchange(mine ? sl.c * q : T(0), mine ? sl.c : T(0), [&](T a, T b) {
+        f = f + a;
+        df = df + b;
+      });
+      if (solve) u = kInc ? -f / df : f / df;
+    } else {
+      const T tolp = (T)1.0e-3;
+      bool go = solve;
+      int guard = 0;
+      while (__any_sync(FULL, go)) {
+        if (go && ++guard > kNewtonLimit) {
+          if (nc.sl == 0) atomicExch(err, DEV_NEWTON_LIMIT);
+          go = false;
+        }
+        T x = 1, pn, pn1;  // lanes without an input run on 1: a root of 0 takes a slow path
+        if (mine) {
+          if constexpr (kInc) x = fmaxf(0.0f, q + u);
+          else x = fmax(0.0, u - q);
+        }
+        newton_pow<MODE>(x, n, pn, pn1);
+        T f = kInc ? u : u - (T)ht, df = 1;
+        const T tf = mine ? sl.c * pn : T(0), tdf = mine ? sl.c * n * pn1 : T(0);
+        nc.exchange(tf, tdf, [&](T a, T b) {
           f = f + a;
           df = df + b;
-        }
-      }
-      if (solve) hk = f / df;
-    } else if constexpr (HALF3 && NPW == 1) {
-      // one node per warp: solve and npres are warp-uniform, so the loop is
-      // the reference's and the sums stop at the last present slot
-      if (solve) {
-        const double tolp = 1.0e-3;
-        double errp = 2.0 * tolp;
-        int guard = 0;
-        while (errp > tolp) {
-          if (++guard > kNewtonLimit) {
-            if (sg.sl == 0) atomicExch(err, DEV_NEWTON_LIMIT);
-            break;
-          }
-          const double x = fmax(0.0, hk - hq);
-          const double r = sqrt(x);
-          const double tf = sl.c * (x * r), tdf = sl.c * np.n * r;
-          double f = hk - elev, df = 1.0;
-#pragma unroll
-          for (int s = 0; s < 8; ++s) {
-            if (s >= npres) break;
-            const double a = sg.shfl(tf, s), b = sg.shfl(tdf, s);
-            f = f + a;
-            df = df + b;
-          }
-          const double hn = hk - f / df;
-          errp = fabs(hn - hk);
-          hk = hk * (1.0 - omega) + hn * omega;
-        }
-      }
-    } else if constexpr (HALF3) {
-      const double tolp = 1.0e-3;
-      bool go = solve;
-      int guard = 0;
-      while (__any_sync(FULL, go)) {
-        if (go && ++guard > kNewtonLimit) {
-          if (sg.sl == 0) atomicExch(err, DEV_NEWTON_LIMIT);
-          go = false;
-        }
-        const double x = fmax(0.0, hk - hq);
-        const double r = sqrt(x);
-        const double tf = sl.c * (x * r), tdf = sl.c * np.n * r;
-        double f = hk - elev, df = 1.0;
-#pragma unroll
-        for (int s = 0; s < 8; ++s) {
-          const double a = sg.shfl(tf, s), b = sg.shfl(tdf, s);
-          if (s < npres) {
-            f = f + a;
-            df = df + b;
-          }
-        }
+        });
         if (go) {
-          const double hn = hk - f / df;
-          const double errp = fabs(hn - hk);
-          hk = hk * (1.0 - omega) + hn * omega;
+          const T un = u - f / df;
+          const T errp = kInc ? (T)fabsf((float)(un - u)) : (T)fabs((double)(un - u));
+          u = u * (T(1) - omega) + un * omega;
           go = errp > tolp;
         }
       }
-    } else {
-      double fs[8], qs[8];
-#pragma unroll
-      for (int s = 0; s < 8; ++s) {
-        fs[s] = sg.shfl(sl.c, s);
-        qs[s] = sg.shfl(hq, s);
-      }
-      if (sg.sl == 0 && solve) {
-        const double tolp = 1.0e-3;
-        double errp = 2.0 * tolp;
-        int guard = 0;
-        while (errp > tolp) {
-          if (++guard > kNewtonLimit) {
-            atomicExch(err, DEV_NEWTON_LIMIT);
-            break;
-          }
-          double f = hk - elev, df = 1.0;
-#pragma unroll
-          for (int s = 0; s < 8; ++s)
-            if (s < npres) {
-              const double x = fmax(0.0, hk - qs[s]);
-              double pn, pn1;
-              np.eval(x, pn, pn1);
-              f = f + fs[s] * pn;
-              df = df + fs[s] * np.n * pn1;
-            }
-          const double hn = hk - f / df;
-          errp = fabs(hn - hk);
-          hk = hk * (1.0 - omega) + hn * omega;
-        }
-      }
-      hk = sg.shfl(hk, 0);
-    }
-    double wk = ht;
-    if (rg >= 0) {
-      if (elev > wr) {
-        if (hk < wr) hk = wr;
-      } else {
-        hk = elev;
-      }
-      wk = fmax(wr, hk);
-    }
-    if (g >= 0 && sg.sl == 0) st_global(hw + g, make_double2(hk, wk));
-    return sl.owner ? sl.d : -1;
-  }
-};
-
-// Mixed precision: the stream-power solve for the increment d = h - ht in FP32.
-// Elevations, water levels and the h update stay FP64; the distances to the
-// receivers' new elevations, ht(k) - h(q), are taken in FP64 and rounded once.
-// n = 1: d = -sum f*(ht - hq) / (1 + sum f), the closed form of
-// StreamPowerLaw.f90:108-118 rewritten for the increment; otherwise Newton on
-// d (x = max(0, ht - hq + d), :146-162) with the reference's tolerance and
-// relaxation.
-template <bool HALF3, int NPW>
-struct SplRegionOpMN {
-  using Value = double2;
-  static constexpr int kThreads = HALF3 ? 512 : 256, kNpw = NPW, kId = HALF3 ? 4 : 5;
-  const RegionLineF* line;
-  double2* hw;
-  float n;
-  int half3;
-  float omega;
-  int n_is_one;
-  int* err;
-  __device__ int run(int g, const Seg& sg, const TileLoc& vc) const {
-    const Slot<float> sl(line, g, sg);
-    int rg = -1;
-    bool has_mrec = false;
-    double ht = 0.0;
-    if (g >= 0) {
-      const double2 self = ld_l1(hw + g);
-      unpack_meta(self.y, rg, has_mrec);
-      ht = self.x;
-    }
-    const bool mine = sl.owner && sl.q >= 0;
-    const unsigned present = sg.slots(mine);
-    const int npres = __popc(present);
-    double hq = 0.0, w = 0.0;
-    if (rg >= 0) {
-      if (mine) hq = vc.load(hw, sl.q).x;
-      if (sg.sl == 0) w = vc.load(hw, rg).y;
-    }
-    const double wr = sg.shfl(w, 0);
-    sl.prefetch(line, hw, sg, 32 / NPW);
-    const bool solve = rg >= 0 && ht > wr && has_mrec;
-    const float dist = mine ? (float)(ht - hq) : 0.0f;
-    float d = 0.0f;
-    if (n_is_one) {
-      const float tf = sl.c * dist;
-      float num = 0.0f, den = 1.0f;
-#pragma unroll
-      for (int s = 0; s < 8; ++s) {
-        const float a = sg.shfl(tf, s), b = sg.shfl(sl.c, s);
-        if (s < npres) {
-          num = num + a;
-          den = den + b;
-        }
-      }
-      d = -num / den;
-    } else if constexpr (HALF3 && NPW == 1) {  // warp-uniform, as in SplRegionOpN
-      if (solve) {
-        const float tolp = 1.0e-3f;
-        float errp = 2.0f * tolp;
-        int guard = 0;
-        while (errp > tolp) {
-          if (++guard > kNewtonLimit) {
-            if (sg.sl == 0) atomicExch(err, DEV_NEWTON_LIMIT);
-            break;
-          }
-          const float x = fmaxf(0.0f, dist + d);
-          const float r = sqrtf(x);
-          const float tf = sl.c * (x * r), tdf = sl.c * n * r;
-          float f = d, df = 1.0f;
-#pragma unroll
-          for (int s = 0; s < 8; ++s) {
-            if (s >= npres) break;
-            const float a = sg.shfl(tf, s), b = sg.shfl(tdf, s);
-            f = f + a;
-            df = df + b;
-          }
-          const float dn = d - f / df;
-          errp = fabsf(dn - d);
-          d = d * (1.0f - omega) + dn * omega;
-        }
-      }
-    } else if constexpr (HALF3) {
-      const float tolp = 1.0e-3f;
-      bool go = solve;
-      int guard = 0;
-      while (__any_sync(FULL, go)) {
-        if (go && ++guard > kNewtonLimit) {
-          if (sg.sl == 0) atomicExch(err, DEV_NEWTON_LIMIT);
-          go = false;
-        }
-        const float x = fmaxf(0.0f, dist + d);
-        const float r = sqrtf(x);
-        const float tf = sl.c * (x * r), tdf = sl.c * n * r;
-        float f = d, df = 1.0f;
-#pragma unroll
-        for (int s = 0; s < 8; ++s) {
-          const float a = sg.shfl(tf, s), b = sg.shfl(tdf, s);
-          if (s < npres) {
-            f = f + a;
-            df = df + b;
-          }
-        }
-        if (go) {
-          const float dn = d - f / df;
-          const float errp = fabsf(dn - d);
-          d = d * (1.0f - omega) + dn * omega;
-          go = errp > tolp;
-        }
-      }
-    } else {
-      float fs[8], ds[8];
-#pragma unroll
-      for (int s = 0; s < 8; ++s) {
-        fs[s] = sg.shfl(sl.c, s);
-        ds[s] = sg.shfl(dist, s);
-      }
-      if (sg.sl == 0 && solve) {
-        const float tolp = 1.0e-3f;
-        float errp = 2.0f * tolp;
-        int guard = 0;
-        while (errp > tolp) {
-          if (++guard > kNewtonLimit) {
-            atomicExch(err, DEV_NEWTON_LIMIT);
-            break;
-          }
-          float f = d, df = 1.0f;
-#pragma unroll
-          for (int s = 0; s < 8; ++s)
-            if (s < npres) {
-              const float x = fmaxf(0.0f, ds[s] + d);
-              float pn, pn1;
-              if (x > 0.0f) {
-                pn1 = powf(x, n - 1.0f);
-                pn = x * pn1;
-              } else {
-                pn = powf(x, n);
-                pn1 = powf(x, n - 1.0f);
-              }
-              f = f + fs[s] * pn;
-              df = df + fs[s] * n * pn1;
-            }
-          const float dn = d - f / df;
-          errp = fabsf(dn - d);
-          d = d * (1.0f - omega) + dn * omega;
-        }
-      }
-      d = sg.shfl(d, 0);
     }
     double hk = ht, wk = ht;
-    if (rg >= 0) {
-      if (ht > wr) {
-        if (has_mrec) hk = ht + (double)d;
+    if (has_rec) {
+      if (above) {
+        if (solve) hk = kInc ? ht + (double)u : (double)u;
         if (hk < wr) hk = wr;
-      } else {
-        hk = ht;
       }
       wk = fmax(wr, hk);
     }
-    if (g >= 0 && sg.sl == 0) st_global(hw + g, make_double2(hk, wk));
-    return sl.owner ? sl.d : -1;
+    out = make_double2(hk, wk);
+    if (on && nc.sl == 0) st_value(val + nc.k, out);
+    return sl.meta;
   }
 };
 
-// Nodes per warp: each sweep runs as two kernels, one node per warp (the
-// shortest latency per node, best where the critical path dominates) and four
-// per warp (8-lane segments, more nodes in flight, best on large grids); the
-// tuner below picks one per grid size class.  Single-node ops (n != 1.5 SPL)
-// have one form.
-constexpr int kNpwWide = 4;
-
 // ---- the sweep kernel ------------------------------------------------------------
-// One CTA per tile.  Shared memory: the tile's counters (bytes, four per word)
-// and its ready queue (local indices, filled once each, never wrapped).
-// Warp 0's lane 0 polls the tile's inbox; every other warp computes up to
-// NPW nodes at a time, one per segment: after a node, its lanes release the
-// node's dependents (one per lane), the segment continues with the first one
-// made ready (they come largest priority first) and queues the others.  A
-// segment without a node claims the next queue slot and waits for it to be
-// filled.  A CTA ends when all nodes of its tile are done; every wait is
-// bounded by a 4 s limit, after which the sweep reports DEV_SPIN_LIMIT.
-template <class Op>
-__global__ void __launch_bounds__(Op::kThreads, kRegionCtasPerSm)
-    k_region_sweep(Op op, TileMap tm, const unsigned char* __restrict__ cnt0, int* xcnt, int* inbox, int icap,
-                   unsigned* itail, int* err) {
+// One CTA per SM; CTA c owns tiles c, c + C, c + 2C, ...  Shared memory: a
+// counter byte per node, the directions in which each rim cell's node has
+// dependents in the tile, the flag words already seen.  Warp 0 polls the flag
+// words of the CTA's tiles; every segment of the other warps computes one node
+// at a time: its lanes release the node's dependents (lane t the one in
+// direction t), it continues with the first one made ready and queues the
+// others.  A warp without work claims one queue
+// entry ahead and waits for it, so that a new entry wakes an idle warp at
+// once; entries beyond those that idle warps wait for are taken by whichever
+// warp comes round next, up to four at a time.  A CTA ends when all its
+// nodes are done; every wait is bounded by a 4 s limit, after which the sweep
+// reports DEV_SPIN_LIMIT.
+template <class Op, int LT>
+__global__ void __launch_bounds__(kThreads, 1)
+    k_region_sweep(Op op, TileMap tm, const unsigned short* __restrict__ wmeta, long long* queue,
+                   typename Op::Value* mbox, unsigned* flags, int* err) {
+  using V = typename Op::Value;
+  using R = Rim<LT>;
+  constexpr int kTS = 1 << LT, kNodes = kTS * kTS;
   extern __shared__ __align__(16) unsigned char smem[];
-  const int lr = tm.lr();
-  const int R = 1 << lr;
-  unsigned* cnt = reinterpret_cast<unsigned*>(smem);                  // R bytes
-  unsigned short* q = reinterpret_cast<unsigned short*>(smem + R);    // R entries
-  __shared__ int qhead, qtail, ndone, stop;
-  const int tile = blockIdx.x;
-  const int gbase = tile << lr;
-  const int tx = tile % tm.ntx, ty = tile / tm.ntx;
-  const int count = min(1 << tm.ltx, tm.nx - (tx << tm.ltx)) * min(1 << tm.lty, tm.ny - (ty << tm.lty));
+  __shared__ int qhead, qtail, ndone, stop, count_sh;
+  __shared__ __align__(16) int4 scratch;
+  __shared__ __align__(16) unsigned char terms[kThreads / 32][kSegs * kRowStride];
+  const int nC = gridDim.x;
+  const int tiles = tm.tiles();
+  const int ns = (tiles - (int)blockIdx.x + nC - 1) / nC;  // tiles of this CTA
+  unsigned* cnt = reinterpret_cast<unsigned*>(smem);
+  unsigned char* rim = smem + tm.ns * kNodes;                                        // tm.ns * R::kCells
+  unsigned* seen = reinterpret_cast<unsigned*>(rim + tm.ns * R::kCells);            // tm.ns * R::kWords
+  TileInfo* tab = reinterpret_cast<TileInfo*>(seen + tm.ns * R::kWords);  // tm.ns
+  long long* q = queue + (size_t)blockIdx.x * tm.ns * kNodes;
   const unsigned long long t0 = global_ns();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int kWarps = kThreads / 32;
 
   if (threadIdx.x == 0) {
     qhead = 0;
     qtail = 0;
     ndone = 0;
     stop = 0;
+    count_sh = 0;
   }
-  for (int w = threadIdx.x; w < R / 4; w += blockDim.x)
-    cnt[w] = reinterpret_cast<const unsigned*>(cnt0 + gbase)[w];
-  for (int l = threadIdx.x; l < R; l += blockDim.x) q[l] = kQEmpty;
   __syncthreads();
-  const TileLoc vc{tile, lr};
-  for (int l = threadIdx.x; l < R; l += blockDim.x)
-    if (cnt0[gbase + l] == 0) q[atomicAdd(&qtail, 1)] = (unsigned short)l;
+  for (int s = threadIdx.x; s < ns; s += kThreads) {
+    const int t = (int)blockIdx.x + s * nC;
+    TileInfo ti;
+    ti.x0 = (t % tm.ntx) * kTS;
+    ti.y0 = (t / tm.ntx) * kTS;
+    ti.w = min(kTS, tm.nx - ti.x0);
+    ti.h = min(kTS, tm.ny - ti.y0);
+    tab[s] = ti;
+    atomicAdd(&count_sh, ti.w * ti.h);
+  }
+  __syncthreads();
+  const int count = count_sh;
+  for (int row = warp; row < ns * kTS; row += kWarps) {
+    const int s = row >> LT, y = row & (kTS - 1);
+    const TileInfo ti = tab[s];
+    if (y >= ti.h) continue;
+    for (int xb = 0; xb < ti.w; xb += 32) {
+      const int x = xb + lane;
+      const int k = ti.x0 + x + (ti.y0 + y) * tm.nx;
+      int c = 255;
+      if (x < ti.w) {
+        c = wmeta[k] & 255;
+        smem[(row << LT) + x] = (unsigned char)c;
+      }
+      const unsigned m = __ballot_sync(FULL, c == 0);
+      if (m) {
+        int p = 0;
+        if (lane == 0) p = atomicAdd(&qtail, __popc(m));
+        p = __shfl_sync(FULL, p, 0) + __popc(m & ((1u << lane) - 1u));
+        if (c == 0) st_queue(q + p, (long long)k << 32 | ((row << LT) + x));
+      }
+    }
+  }
+  for (int e = threadIdx.x; e < ns * R::kCells; e += kThreads) {
+    const int s = e / R::kCells, c = e - s * R::kCells;
+    const TileInfo ti = tab[s];
+    int x, y;
+    unsigned m = 0;
+    if (R::coords(c, ti.w, ti.h, x, y)) {
+      // a cell beyond a non-cyclic edge names a node on the other side, which
+      // has no dependents in the directions that lead here
+      int X = ti.x0 + x, Y = ti.y0 + y;
+      X += X < 0 ? tm.nx : (X >= tm.nx ? -tm.nx : 0);
+      Y += Y < 0 ? tm.ny : (Y >= tm.ny ? -tm.ny : 0);
+      const unsigned deps = wmeta[X + Y * tm.nx] >> 8;
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        const int ax = x + dir_di(t), ay = y + dir_dj(t);
+        if (((deps >> t) & 1u) && ax >= 0 && ax < ti.w && ay >= 0 && ay < ti.h) m |= 1u << t;
+      }
+    }
+    rim[e] = (unsigned char)m;
+  }
+  for (int e = threadIdx.x; e < ns * R::kWords; e += kThreads) seen[e] = 0u;
   __syncthreads();
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  auto push = [&](int l) {
-    __threadfence_block();
-    const int p = atomicAdd(&qtail, 1);
-    if (p < R) *(volatile unsigned short*)&q[p] = (unsigned short)l;
+  auto push = [&](int p, int k, int id) {
+    if (p < count) st_queue(q + p, (long long)k << 32 | id);
     else atomicExch(err, DEV_OVERFLOW);
   };
-  // decrements node l's counter; true when l became ready
+  // decrements the counter of local node l; true when the node became ready
   auto release = [&](int l) {
     const unsigned sh = 8u * (unsigned)(l & 3);
     const unsigned old = atomicSub(&cnt[l >> 2], 1u << sh);
@@ -948,103 +761,201 @@ __global__ void __launch_bounds__(Op::kThreads, kRegionCtasPerSm)
   };
 
   if (warp == 0) {
-    if (lane != 0) return;
-    int ih = 0, ticks = 0;
-    int* box = inbox + (size_t)tile * icap;
+    int ticks = 0;
     for (;;) {
-      if (ih < icap) {
-        const int d = ld_relaxed_gpu(&box[ih]);
-        if (d >= 0) {
-          ++ih;
-          __threadfence();  // acquire: the cross-tile producers' values
-          if (release(d - gbase)) push(d - gbase);
-          continue;
+      bool any = false;
+      for (int e0 = 0; e0 < ns * (R::kWords / 4); e0 += 32) {
+        const int e = e0 + lane;
+        unsigned nw[4] = {0u, 0u, 0u, 0u};
+        if (e < ns * (R::kWords / 4)) {
+          const int s = e / (R::kWords / 4), w4 = e - s * (R::kWords / 4);
+          ld_flags(flags + ((size_t)blockIdx.x + (size_t)s * nC) * R::kWords + 4 * w4, nw);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) nw[i] &= ~seen[4 * e + i];
         }
-      }
-      if (*(volatile int*)&ndone >= count) return;
-      if (should_stop(ticks)) return;
-      __nanosleep(64);
-    }
-  }
-  constexpr int W = 32 / Op::kNpw;  // lanes per node
-  const Seg sg{lane % W, lane - lane % W};
-  const unsigned segmask = (W == 32 ? 0xffffffffu : ((1u << W) - 1u)) << sg.base;
-  int cur = -1, slot = -1, ticks = 0, back = 32;
-  for (;;) {
-    // segments without a node try their queue slot (the segment's lane 0);
-    // a one-segment warp that continues with a dependent skips the poll
-    if (W < 32 || cur < 0) {
-      int got = -1;
-      if (cur < 0 && sg.sl == 0) {
-        if (slot < 0) slot = atomicAdd(&qhead, 1);
-        if (slot < R) {
-          const unsigned short v = *(volatile unsigned short*)&q[slot];
-          if (v != kQEmpty) {
-            got = v;
-            slot = -1;
+        // the warp takes the words with news one after the other, a cell per lane
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          unsigned lanes = __ballot_sync(FULL, nw[i] != 0u);
+          while (lanes) {
+            const int src = __ffs(lanes) - 1;
+            lanes &= lanes - 1u;
+            const unsigned bits = __shfl_sync(FULL, nw[i], src);
+            const int word = 4 * (e0 + src) + i;
+            bool got = false;
+            if ((bits >> lane) & 1u) {
+              const int s = word / R::kWords, c = 32 * (word - s * R::kWords) + lane;
+              V v;
+              got = mail_read(mbox + ((size_t)blockIdx.x + (size_t)s * nC) * R::kCells + c, v);  // or the flag overtook it
+              if (got) {
+                const TileInfo ti = tab[s];
+                int x, y;
+                R::coords(c, ti.w, ti.h, x, y);
+                unsigned m = rim[s * R::kCells + c];
+                __threadfence_block();
+                while (m) {
+                  const int t = __ffs(m) - 1;
+                  m &= m - 1u;
+                  const int c3 = t + (t >> 2);
+                  const int lx = x + c3 % 3 - 1, ly = y + c3 / 3 - 1;
+                  const int id = (s << (2 * LT)) | (ly << LT) | lx;
+                  if (release(id)) {
+                    __threadfence_block();
+                    push(atomicAdd(&qtail, 1), ti.x0 + lx + (ti.y0 + ly) * tm.nx, id);
+                  }
+                }
+              }
+            }
+            const unsigned in = __ballot_sync(FULL, got);
+            if (lane == 0) seen[word] |= in;
+            any |= in != 0u;
           }
         }
+        __syncwarp();
       }
-      got = __shfl_sync(FULL, got, sg.base);
-      if (cur < 0) cur = got;
-      if (!__any_sync(FULL, cur >= 0)) {
+      if (!any) {
         int quit = 0;
         if (lane == 0) quit = *(volatile int*)&ndone >= count || should_stop(ticks);
         if (__shfl_sync(FULL, quit, 0)) return;
-        // idle warps back off (32 ns doubling to 512 ns): polling warps take
-        // issue slots from the busy ones (stream-power sweep at 2049^2:
-        // 15.9 -> 15.3 ms against a constant 32 ns)
-        __nanosleep(back);
-        if (back < 512) back <<= 1;
-        continue;
+        __nanosleep(20);
       }
-      back = 32;
-      __threadfence_block();  // acquire: the producers' values
     }
-    const int d = op.run(cur >= 0 ? gbase + cur : -1, sg, vc);
-    __syncwarp();
-    __threadfence_block();  // release: the node's value before its dependents' counters
-    bool ready = false;
-    if (d >= 0) {
-      if ((d >> lr) == tile) {
-        ready = release(d - gbase);
-      } else {
-        __threadfence();  // release at GPU scope before a cross-tile counter
-        if (atomicSub(&xcnt[d], 1) == 1) {
-          __threadfence();
-          const int owner = d >> lr;
-          const unsigned p = atomicAdd(&itail[owner], 1u);
-          if (p < (unsigned)icap) st_relaxed_gpu_int(&inbox[(size_t)owner * icap + p], d);
-          else atomicExch(err, DEV_OVERFLOW);
+  }
+
+  const unsigned scr = (unsigned)__cvta_generic_to_shared(&scratch);
+  const int sl = lane & (kSegLanes - 1), base = lane - sl;
+  const int di = (sl + (sl >> 2)) % 3 - 1, dj = (sl + (sl >> 2)) / 3 - 1;  // this lane's direction
+  const int kstep = dj * tm.nx + di, lstep = dj * kTS + di;
+  const unsigned my_edges = edges_of(di, dj);
+  const int nn = tm.nx * tm.ny;
+  const bool far_ahead = nn > kL2Records;
+  int k = 0, id = -1, slot = -1, ticks = 0;  // the same in all lanes of a segment
+  int backlog = 0;  // entries queued beyond the claims, as last seen (the same in all lanes)
+  int hops = 0;
+  int done = 0;     // nodes computed by this segment and not yet counted (its first lane)
+  Slot<typename Op::T> rec;
+  for (;;) {
+    // a warp without work claims one entry ahead; segments of a working warp
+    // take entries that are queued beyond the waiting warps' claims
+    const unsigned busy = __ballot_sync(FULL, id >= 0 || slot >= 0);
+    if (busy == 0u || (backlog > 0 && busy != FULL)) {
+      const unsigned open = ~busy & 0x01010101u;  // one bit per open segment
+      const int want = backlog > 0 ? min(__popc(open), max(1, backlog >> 4)) : 1;
+      int b0 = 0;
+      if (lane == 0) b0 = atomicAdd(&qhead, want);
+      b0 = __shfl_sync(FULL, b0, 0);
+      const int rank = __popc(open & ((1u << base) - 1u));
+      if (((open >> base) & 1u) && rank < want) slot = b0 + rank;
+    }
+    const bool poll = sl == 0 && slot >= 0 && slot < count;  // a segment's first lane looks
+    long long v = -1;
+    if (poll) v = ld_queue(q + slot);
+    if (!__any_sync(FULL, id >= 0)) {  // nothing to do until an entry comes
+      if (done) {
+        atomicAdd(&ndone, done);
+        done = 0;
+      }
+      const int mine = __reduce_max_sync(FULL, slot);
+      int tries = 0;
+      while (!__any_sync(FULL, v >= 0)) {
+        // the next pushes fill the entries right after the tail: warps that
+        // wait further ahead look less often
+        const int ahead = mine - *(volatile int*)&qtail;
+        if (ahead > 2) __nanosleep(ahead > 6 ? 200 : 40);
+        if ((++tries & 7) == 0) {
+          int quit = 0;
+          if (lane == 0) quit = *(volatile int*)&ndone >= count || should_stop(ticks);
+          if (__shfl_sync(FULL, quit, 0)) {
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            return;
+          }
         }
+        if (poll) v = ld_queue(q + slot);
       }
     }
-    const unsigned rm = __ballot_sync(FULL, ready) & segmask;
-    const int first = rm ? __ffs(rm) - 1 : lane;
-    const int nxt_l = __shfl_sync(FULL, d - gbase, first);
-    if (ready && lane != first) push(d - gbase);
-    if (rm) __threadfence_block();  // acquire for the continuation
-    if (sg.sl == 0 && cur >= 0) atomicAdd(&ndone, 1);
-    cur = rm ? nxt_l : -1;
+    v = __shfl_sync(FULL, v, base);
+    if (v >= 0) {
+      k = (int)(v >> 32);
+      id = (int)v;
+      slot = -1;
+      rec.load(op.rec + k, true, sl);
+    }
+    const bool waiting = __any_sync(FULL, slot >= 0);
+    bool go;
+    do {  // chains of nodes, while nothing waits for this warp's idle segments
+      __threadfence_block();  // acquire: the producers' values
+      const bool on = id >= 0;
+      V out;
+      rec.open(on);
+      const NodeCtx<V, LT> nc{k, id, tm.nx, sl, &terms[warp][(lane >> 3) * kRowStride], tab, mbox, (int)blockIdx.x, nC};
+      const unsigned meta = op.run(nc, rec, on, out, [&](unsigned m) {
+        // bring what the dependents will read into L1
+        const bool t = ((m >> (8 + sl)) & 1u) && !((m >> 4) & my_edges);
+        const char* p = reinterpret_cast<const char*>(op.rec + (k + kstep));
+        touch_l1_if(scr, p, t);
+        touch_l1_if(scr, p + 32, t);
+        if (sizeof(typename Op::T) == 8) touch_l1_if(scr, p + 64, t);
+        if (!Op::kPrefer && far_ahead) {  // the area's nodes wait long for their last input: L2 may have lost what comes after
+          const char* p2 = reinterpret_cast<const char*>(op.rec + (k + 2 * kstep));
+          prefetch_l2_if(p2, t && (unsigned)(k + 2 * kstep) < (unsigned)nn);
+        }
+        touch_l1_if(scr, reinterpret_cast<const void*>(reinterpret_cast<size_t>(op.val + (k + kstep)) & ~(size_t)15), t);
+      });
+      __syncwarp();
+      __threadfence_block();  // release: the node's value before its dependents' counters
+      const bool dep = on && ((meta >> (8 + sl)) & 1u), cross = (meta >> 4) & my_edges;
+      const unsigned prefer = (meta >> 21) & 7u;
+      bool ready = false;
+      if (dep && !cross) ready = release(id + lstep);
+      const unsigned all = __ballot_sync(FULL, ready);
+      unsigned rm = (all >> base) & 0xffu;
+      if (Op::kPrefer && ((rm >> prefer) & 1u)) rm = 1u << prefer;
+      const int first = (base + __ffs(rm) - 1) & 31;  // any lane where none is ready
+      const bool queued = ready && lane != first;
+      int qp = 0;
+      if (queued) {
+        __threadfence_block();  // the other producers' values too
+        qp = atomicAdd(&qtail, 1);
+      }
+      const int nk = __shfl_sync(FULL, k + kstep, first), nid = __shfl_sync(FULL, id + lstep, first);
+      rec.load(op.rec + nk, rm != 0u, sl);
+      if (queued) push(qp, k + kstep, id + lstep);
+      if (dep && cross) {  // the value into the neighbouring tile's cell, then its flag
+        const TileInfo ti = tab[id >> (2 * LT)];
+        int X = ti.x0 + (id & (kTS - 1)) + di, Y = ti.y0 + ((id >> LT) & (kTS - 1)) + dj;
+        X += X < 0 ? tm.nx : (X >= tm.nx ? -tm.nx : 0);
+        Y += Y < 0 ? tm.ny : (Y >= tm.ny ? -tm.ny : 0);
+        const int ox = X >> LT, oy = Y >> LT;
+        const int ow = min(kTS, tm.nx - ox * kTS), oh = min(kTS, tm.ny - oy * kTS);
+        const int c = R::index((X & (kTS - 1)) - di, (Y & (kTS - 1)) - dj, ow, oh);
+        const size_t tile = (size_t)oy * tm.ntx + ox;
+        mail_write(mbox + tile * R::kCells + c, out);
+        atomicOr(&flags[tile * R::kWords + (c >> 5)], 1u << (c & 31));
+      }
+      done += on && sl == 0;
+      k = nk;
+      id = rm ? nid : -1;
+      // on with the chains while every segment has a node, or none of the idle
+      // ones has anything to do (looked up every fourth node)
+      const bool full = (all & 0xffu) && (all & 0xff00u) && (all & 0xff0000u) && (all & 0xff000000u);
+      go = full || (all && !waiting && ((++hops & 3) || !__any_sync(FULL, *(volatile int*)&qtail > *(volatile int*)&qhead)));
+    } while (go);
+    backlog = __shfl_sync(FULL, *(volatile int*)&qtail - *(volatile int*)&qhead, 0);
   }
 }
 
-// natural-order copies of the sweeps' results
-template <class T>
-__global__ void k_untile_area(int nx, int ny, TileMap tm, const T* __restrict__ val, double* __restrict__ a) {
-  const int nn = nx * ny;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x)
-    a[k] = (double)val[tm.g(k % nx, k / nx)];
+// natural-order FP64 area from the mixed form's FP32 values
+__global__ void k_widen(int nn, const float* __restrict__ v, double* __restrict__ a) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) a[k] = (double)v[k];
 }
 
 // StreamPowerLaw.f90:380-393 with g == 0: b=min(h,b), etot=etot+ht-h,
-// erate=(ht-h)/dt, Sedflux=ht-h, from the tile-major (h, water) pairs
-__global__ void k_spl_finish_t(int nx, int ny, TileMap tm, double dt, const double2* __restrict__ hw,
-                               double* __restrict__ h, double* __restrict__ b, double* __restrict__ etot,
-                               double* __restrict__ erate, double* __restrict__ sedflux) {
-  const int nn = nx * ny;
+// erate=(ht-h)/dt, Sedflux=ht-h, from the (h, water) pairs
+__global__ void k_spl_finish_hw(int nn, double dt, const double2* __restrict__ hw, double* __restrict__ h,
+                                double* __restrict__ b, double* __restrict__ etot, double* __restrict__ erate,
+                                double* __restrict__ sedflux) {
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
-    const double ht = h[k], hn = hw[tm.g(k % nx, k / nx)].x;
+    const double ht = h[k], hn = hw[k].x;
     b[k] = fmin(hn, b[k]);
     etot[k] = etot[k] + ht - hn;
     erate[k] = (ht - hn) / dt;
@@ -1053,20 +964,21 @@ __global__ void k_spl_finish_t(int nx, int ny, TileMap tm, double dt, const doub
   }
 }
 
+constexpr int kMaxSmem = 212 * 1024;  // dynamic shared memory of a sweep CTA at most
 
-template <class Op>
-size_t region_smem(const TileMap& tm) {
-  return (size_t)3 << tm.lr();
+int region_smem(const TileMap& tm) {
+  return tm.ns * ((1 << 2 * tm.lt) + rim_cells(tm.lt) + 4 * rim_words(tm.lt) + (int)sizeof(TileInfo));
 }
 
-// whether every tile's CTA of this sweep kernel can be co-resident
-template <class Op>
+// whether every CTA of this sweep kernel can be co-resident
+template <class Op, int LT>
 bool region_fits(const TileMap& tm) {
-  const size_t smem = region_smem<Op>(tm);
-  auto kern = k_region_sweep<Op>;
-  // the permitted maximum covers every plan (3 bytes per node, 32768 nodes per
-  // tile), so instances with different plans never undo each other's setting
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * 32768) != cudaSuccess) {
+  const int smem = region_smem(tm);
+  if (smem > kMaxSmem) return false;
+  auto kern = k_region_sweep<Op, LT>;
+  // the permitted maximum covers every plan, so instances with different
+  // plans never undo each other's setting
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
@@ -1074,256 +986,128 @@ bool region_fits(const TileMap& tm) {
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, Op::kThreads, smem) != cudaSuccess) {
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, (size_t)smem) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  return per_sm * sms >= tm.tiles();
+  return per_sm * sms >= tm.nctas;
 }
 
-// whether the sweep of op Op can run on one of the instance's tile plans
-// (checked once per instance and op)
-template <class Op>
-bool region_usable(Ctx& c) {
-  if (!c.region_enabled || c.ntplans == 0) return false;
+// whether the sweep of Op can run on the plan (checked once per instance)
+template <class Op, int LT>
+bool region_usable(Ctx& c, const TileMap& tm) {
+  if (!c.region_enabled || tm.ntx == 0) return false;
   signed char& st = c.region_ok[Op::kId];
-  if (st == 0) {
-    st = -1;
-    for (int i = 0; i < c.ntplans; ++i)
-      if (region_fits<Op>(c.tplans[i])) st = 1;
-  }
+  if (st == 0) st = region_fits<Op, LT>(tm) ? 1 : -1;
   return st > 0;
 }
 
-template <class Op>
-bool launch_region(Ctx& c, Op op, const TileMap& tm) {
-  const int tiles = tm.tiles();
-  const size_t smem = region_smem<Op>(tm);
-  auto kern = k_region_sweep<Op>;
-  cudaMemsetAsync(c.rl_inbox, 0xff, sizeof(int) * (size_t)tiles * c.rl_icap, c.stream);
-  cudaMemsetAsync(c.rl_itail, 0, sizeof(unsigned) * (size_t)tiles, c.stream);
-  const unsigned char* cnt0 = c.rl_cnt0;
-  int* xcnt = c.rl_xcnt;
-  int* inbox = c.rl_inbox;
-  int icap = c.rl_icap;
-  unsigned* itail = c.rl_itail;
+// Launches the sweep of op; false when the launch is refused (the queue engine
+// of fsb_flow.cu then runs).
+template <int LT, class Op>
+bool launch_region(Ctx& c, const TileMap& plan, Op op) {
+  using V = typename Op::Value;
+  TileMap tm = plan;
+  const size_t tiles = (size_t)tm.tiles();
+  cudaMemsetAsync(c.rl_queue, 0xff, sizeof(long long) * tm.queue_entries(), c.stream);
+  cudaMemsetAsync(c.rl_flags, 0, sizeof(unsigned) * tiles * rim_words(LT), c.stream);
+  cudaMemsetAsync(c.rl_mbox, 0xff, sizeof(V) * tiles * rim_cells(LT), c.stream);
+  const unsigned short* wmeta = c.rl_wmeta;
+  long long* queue = c.rl_queue;
+  V* mbox = reinterpret_cast<V*>(c.rl_mbox);
+  unsigned* flags = c.rl_flags;
   int* err = c.d_err;
-  TileMap tmv = tm;
-  void* args[] = {&op, &tmv, &cnt0, &xcnt, &inbox, &icap, &itail, &err};
-  const int timer = Op::kId == 0 || Op::kId == 3 ? KT_AREA_SWEEP : KT_SPL_SWEEP;
+  void* args[] = {&op, &tm, &wmeta, &queue, &mbox, &flags, &err};
+  const int timer = Op::kPrefer ? KT_SPL_SWEEP : KT_AREA_SWEEP;
   stage_begin(c, timer);
-  const cudaError_t e =
-      cudaLaunchCooperativeKernel((const void*)kern, dim3(tiles), dim3(Op::kThreads), args, smem, c.stream);
+  const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_region_sweep<Op, LT>, dim3(tm.nctas), dim3(kThreads),
+                                                    args, (size_t)region_smem(tm), c.stream);
   stage_end(c, timer);
   c.count_launch();
-  if (e != cudaSuccess) {  // e.g. the GPU is shared and the tiles no longer fit
+  if (e != cudaSuccess) {  // e.g. the GPU is shared and the CTAs no longer fit
     cudaGetLastError();
+    c.region_ok[Op::kId] = -1;
     return false;
   }
   return true;
 }
 
-// ---- the tile-plan tuner ------------------------------------------------------
-// The tile shape decides how a sweep's work is split between co-resident CTAs
-// and how often its critical path crosses a tile boundary, and the nodes per
-// warp trade latency per node for nodes in flight; which pair is fastest
-// depends on the grid.  The first sweep of an op on an instance whose grid
-// size class has not been seen by the process runs twice on each candidate
-// (every candidate plan -- the smallest tiles that fit the co-resident CTAs
-// and up to two coarser ones -- with each form of the kernel), timed with
-// CUDA events, and keeps the fastest, also for every later instance of that
-// size class.  Every run is a complete, correct sweep: a node's arithmetic
-// depends neither on the plan nor on the form, so each run gives the same
-// values and the last one's output is used.  A cached choice applies to a
-// later grid of the same size class when its candidate list holds that tile
-// shape.
-std::mutex g_tune_mu;
-// (size class, aspect class, op) -> (ltx, lty, form); a size class spans a
-// factor sqrt(2) in nodes, so a stream of requests of many sizes (the served
-// form) tunes once per class, not once per size
-std::map<std::tuple<int, int, int>, std::tuple<int, int, int>> g_tuned;
-std::tuple<int, int, int> tune_key(const Ctx& c, int op) {
-  const int size_class = (int)std::floor(2.0 * std::log2((double)c.nx * (double)c.ny));
-  const int aspect_class = (int)std::lround(std::log2((double)c.nx / (double)c.ny));
-  return std::make_tuple(size_class * 64 + aspect_class, 0, op);
-}
+dim3 grid2d(const Ctx& c) { return dim3((c.nx + 31) / 32, (c.ny + 7) / 8); }
 
-// Runs run(plan, form) on op id's tuned plan and form (0 <= form < nforms),
-// tuning first where needed; fits(plan, form) says whether the form's CTAs
-// are co-resident on the plan.  Returns the plan of the last complete run, or
-// nullptr when no plan could run.
-template <class Fits, class Run>
-const TileMap* run_tuned(Ctx& c, int id, int nforms, Fits fits, Run run) {
-  TileMap& chosen = c.tplan_of[id];
-  int& form = c.tform_of[id];
-  if (chosen.ntx == 0) {
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    auto it = g_tuned.find(tune_key(c, id));
-    if (it != g_tuned.end() && std::get<2>(it->second) < nforms)
-      for (int i = 0; i < c.ntplans; ++i)
-        if (c.tplans[i].ltx == std::get<0>(it->second) && c.tplans[i].lty == std::get<1>(it->second)) {
-          chosen = c.tplans[i];
-          form = std::get<2>(it->second);
-        }
-  }
-  if (chosen.ntx != 0) {
-    if (fits(chosen, form) && run(chosen, form)) return &chosen;
-    c.region_ok[id] = -1;  // the queue engine runs from now on
-    return nullptr;
-  }
-  cudaEvent_t e0 = nullptr, e1 = nullptr;
-  cudaEventCreate(&e0);
-  cudaEventCreate(&e1);
-  const TileMap* last = nullptr;
-  float best_ms = 0.f;
-  int best = -1, best_form = 0;
-  for (int i = 0; i < c.ntplans; ++i)
-    for (int f = 0; f < nforms; ++f) {
-      if (!fits(c.tplans[i], f)) continue;
-      float cand_ms = -1.f;  // the better of two runs of each candidate
-      for (int rep = 0; rep < 2; ++rep) {
-        cudaEventRecord(e0, c.stream);
-        const bool ok = run(c.tplans[i], f);
-        cudaEventRecord(e1, c.stream);
-        float ms = 0.f;
-        if (!ok || cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) {
-          cudaGetLastError();
-          cand_ms = -1.f;
-          break;
-        }
-        last = &c.tplans[i];
-        if (cand_ms < 0.f || ms < cand_ms) cand_ms = ms;
-      }
-      if (cand_ms >= 0.f && (best < 0 || cand_ms < best_ms)) {
-        best = i;
-        best_form = f;
-        best_ms = cand_ms;
-      }
-    }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  if (best < 0) c.region_ok[id] = -1;  // no plan ran: the queue engine from now on
-  if (best >= 0) {
-    chosen = c.tplans[best];
-    form = best_form;
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tuned[tune_key(c, id)] = std::make_tuple(chosen.ltx, chosen.lty, form);
-  }
-  return last;
-}
-
-// area sweep of value type T on plan p with NPW nodes per warp
-template <class T, int NPW>
-bool acc_run(Ctx& c, const TileMap& p) {
-  using Op = AccRegionOpT<T, NPW>;
-  RegionLineT<T>* line = static_cast<RegionLineT<T>*>(c.rl_line);
-  T* val = reinterpret_cast<T*>(c.rl_val);
-  cudaMemsetAsync(c.rl_cnt0, 0xff, (size_t)p.padded(), c.stream);  // padding slots never run
-  k_acc_lines_t<T><<<grid1d(c.nn), kBlock, 0, c.stream>>>(c.bd, p, c.dx * c.dy, c.mrec, c.mnrec, c.mwrec, c.precip,
-                                                          c.size, line, val, c.rl_cnt0, c.rl_xcnt, c.d_err);
+template <class T, int LT>
+bool accumulate_t(Ctx& c) {
+  using Op = AccOp<T>;
+  const TileMap& tm = c.tplan[LT - kLogTileMin];
+  if (!region_usable<Op, LT>(c, tm)) return false;
+  RecordT<T>* rec = static_cast<RecordT<T>*>(c.mfd_line);
+  T* val = sizeof(T) == sizeof(double) ? reinterpret_cast<T*>(c.a) : reinterpret_cast<T*>(c.hw);
+  k_acc_records<T><<<grid2d(c), dim3(32, 8), 0, c.stream>>>(c.bd, 1 << LT, c.dx * c.dy, c.mdmask, c.mrec, c.mwrec,
+                                                            c.precip, rec, c.rl_wmeta);
   c.count_launch();
-  return launch_region<Op>(c, Op{line, val}, p);
+  if (!launch_region<LT>(c, tm, Op{rec, val})) return false;
+  if (sizeof(T) == sizeof(float)) {
+    k_widen<<<grid1d(c.nn), kBlock, 0, c.stream>>>(c.nn, reinterpret_cast<float*>(c.hw), c.a);
+    c.count_launch();
+  }
+  return true;
 }
 
-template <class T>
-bool region_accumulate_t(Ctx& c) {
-  using Op1 = AccRegionOpT<T, 1>;
-  using OpW = AccRegionOpT<T, kNpwWide>;
-  if (!region_usable<Op1>(c)) return false;
-  const TileMap* tm = run_tuned(
-      c, Op1::kId, 2, [&](const TileMap& p, int f) { return f ? region_fits<OpW>(p) : region_fits<Op1>(p); },
-      [&](const TileMap& p, int f) { return f ? acc_run<T, kNpwWide>(c, p) : acc_run<T, 1>(c, p); });
-  if (!tm) return false;
-  k_untile_area<T><<<grid1d(c.nn), kBlock, 0, c.stream>>>(c.nx, c.ny, *tm, reinterpret_cast<T*>(c.rl_val), c.a);
+template <class T, int MODE, int LT>
+bool stream_power_t(Ctx& c) {
+  using Op = SplOp<T, MODE>;
+  const TileMap& tm = c.tplan[LT - kLogTileMin];
+  if (!region_usable<Op, LT>(c, tm)) return false;
+  RecordT<T>* rec = static_cast<RecordT<T>*>(c.mfd_line);
+  double2* hw = reinterpret_cast<double2*>(c.hw);
+  double* lpow = c.ltab + 16;
+  float* lpowf = reinterpret_cast<float*>(c.ltab + 32);
+  const T* lp;
+  if constexpr (sizeof(T) == sizeof(double)) lp = lpow; else lp = lpowf;
+  k_length_pow<<<1, 32, 0, c.stream>>>(c.ltab, c.n, lpow, lpowf);
+  k_spl_records<T><<<grid2d(c), dim3(32, 8), 0, c.stream>>>(c.bd, 1 << LT, MODE == 0, c.kfsed, c.dt, c.m, c.rec,
+                                                            c.mdmask, c.mrec, c.mwrec, c.mlrec, c.h, c.b, c.kf, c.a,
+                                                            c.ltab, lp, rec, c.rl_wmeta, c.d_err);
+  c.count_launch(2);
+  if (!launch_region<LT>(c, tm, Op{rec, hw, (T)c.n, (T)(0.875 / c.n), c.d_err})) return false;
+  k_spl_finish_hw<<<grid1d(c.nn), kBlock, 0, c.stream>>>(c.nn, c.dt, hw, c.h, c.b, c.etot, c.erate, c.sedflux);
   c.count_launch();
   return true;
 }
 
-// stream-power sweep: op1 (one node per warp) and opw (its wide form, the
-// same type where the op has one form only: nforms = 1)
-template <class Op1, class OpW, class T>
-const TileMap* spl_sweep(Ctx& c, const Op1& op1, const OpW& opw, int nforms, RegionLineT<T>* line,
-                         const T* lpow) {
-  const int n1 = fabs(c.n - 1.0) < DBL_MIN;
-  double2* hw = reinterpret_cast<double2*>(c.rl_val);
-  return run_tuned(
-      c, Op1::kId, nforms, [&](const TileMap& p, int f) { return f ? region_fits<OpW>(p) : region_fits<Op1>(p); },
-      [&](const TileMap& p, int f) {
-        cudaMemsetAsync(c.rl_cnt0, 0xff, (size_t)p.padded(), c.stream);
-        k_spl_lines_t<T><<<grid1d(c.nn), kBlock, 0, c.stream>>>(c.bd, p, n1, c.kfsed, c.dt, c.m, c.n, c.rec, c.mrec,
-                                                                c.mnrec, c.mwrec, c.mlrec, c.h, c.b, c.kf, c.a,
-                                                                c.size, c.ltab, lpow, line, hw, c.rl_cnt0,
-                                                                c.rl_xcnt, c.d_err);
-        c.count_launch();
-        return f ? launch_region<OpW>(c, opw, p) : launch_region<Op1>(c, op1, p);
-      });
+template <class T>
+bool stream_power_n(Ctx& c) {
+  if (fabs(c.n - 1.0) < DBL_MIN) return stream_power_t<T, 0, 5>(c);
+  return c.n == 1.5 ? stream_power_t<T, 1, 5>(c) : stream_power_t<T, 2, 5>(c);
 }
 
 }  // namespace
 
-// Tile plans: tiles of 2^a x 2^b nodes (32 x 32 at least, 32768 nodes at
-// most, width >= height) whose count fits the co-resident CTAs
-// (kRegionCtasPerSm per SM) -- the smallest such tiles and up to two coarser
-// ones, for the tuner.  None fits -> the queue engine runs.
-int plan_tiles(int nx, int ny, int sms, TileMap* out, int max_plans) {
-  const int max_ctas = kRegionCtasPerSm * std::max(1, sms);
-  static const int cand[][2] = {{5, 5}, {6, 5}, {6, 6}, {7, 6}, {7, 7}, {8, 7}};
-  int n = 0;
-  for (const auto& cd : cand) {
-    const int ntx = (nx + (1 << cd[0]) - 1) >> cd[0], nty = (ny + (1 << cd[1]) - 1) >> cd[1];
-    if (ntx * nty <= max_ctas && n < max_plans) {
-      TileMap& tm = out[n++];
-      tm.nx = nx;
-      tm.ny = ny;
-      tm.ltx = cd[0];
-      tm.lty = cd[1];
-      tm.ntx = ntx;
-      tm.nty = nty;
-    }
-  }
-  return n;
+// Tile plan: the grid's tiles of side 2^lt over at most one CTA per SM.  Tiles
+// so many that a CTA's counters exceed its shared memory leave ntx at 0: the
+// queue engine runs.
+TileMap plan_tiles(int nx, int ny, int lt, int sms) {
+  TileMap tm;
+  tm.nx = nx;
+  tm.ny = ny;
+  tm.lt = lt;
+  tm.ntx = (nx + (1 << lt) - 1) >> lt;
+  tm.nty = (ny + (1 << lt) - 1) >> lt;
+  tm.nctas = std::min(std::max(1, sms), tm.tiles());
+  tm.ns = (tm.tiles() + tm.nctas - 1) / tm.nctas;
+  if (region_smem(tm) > kMaxSmem) tm.ntx = 0;
+  return tm;
 }
 
+// Tile sides.  Smaller tiles spread the front over more SMs and halve the
+// nodes that share an SM; larger ones have fewer crossings, and the area's
+// nodes, all sources at once, are spread anyway.  B200, side 32 / 64: area
+// 257^2 0.48 / 0.53 ms, 1025x769 3.05 / 2.88, 2049^2 6.4 / 5.8; stream power
+// (n = 1.5) 0.69 / 0.84, 3.98 / 4.27, 6.9 / 7.3, 4097^2 18.0 / 18.0.
 bool region_accumulate(Ctx& c) {
-  return c.mixed ? region_accumulate_t<float>(c) : region_accumulate_t<double>(c);
+  if (c.nn <= 1 << 18) return c.mixed ? accumulate_t<float, 5>(c) : accumulate_t<double, 5>(c);
+  return c.mixed ? accumulate_t<float, 6>(c) : accumulate_t<double, 6>(c);
 }
 
-bool region_stream_power(Ctx& c) {
-  const bool h3 = c.n == 1.5;
-  const bool ok = c.mixed ? (h3 ? region_usable<SplRegionOpMN<true, 1>>(c) : region_usable<SplRegionOpMN<false, 1>>(c))
-                          : (h3 ? region_usable<SplRegionOpN<true, 1>>(c) : region_usable<SplRegionOpN<false, 1>>(c));
-  if (!ok) return false;
-  const int n1 = fabs(c.n - 1.0) < DBL_MIN;
-  double2* hw = reinterpret_cast<double2*>(c.rl_val);
-  double* lpow = c.ltab + 16;
-  float* lpowf = reinterpret_cast<float*>(c.ltab + 32);
-  k_length_pow<<<1, 32, 0, c.stream>>>(c.ltab, c.n, lpow, lpowf);
-  c.count_launch();
-  const TileMap* tm;
-  const double omega = 0.875 / c.n;
-  if (c.mixed) {
-    RegionLineF* line = static_cast<RegionLineF*>(c.rl_line);
-    const float nf = (float)c.n, of = (float)omega;
-    if (h3)
-      tm = spl_sweep(c, SplRegionOpMN<true, 1>{line, hw, nf, 1, of, n1, c.d_err},
-                     SplRegionOpMN<true, kNpwWide>{line, hw, nf, 1, of, n1, c.d_err}, 2, line, lpowf);
-    else
-      tm = spl_sweep(c, SplRegionOpMN<false, 1>{line, hw, nf, 0, of, n1, c.d_err},
-                     SplRegionOpMN<false, 1>{line, hw, nf, 0, of, n1, c.d_err}, 1, line, lpowf);
-  } else {
-    RegionLine* line = static_cast<RegionLine*>(c.rl_line);
-    if (h3)
-      tm = spl_sweep(c, SplRegionOpN<true, 1>{line, hw, RegionPow{c.n, 1}, omega, n1, c.d_err},
-                     SplRegionOpN<true, kNpwWide>{line, hw, RegionPow{c.n, 1}, omega, n1, c.d_err}, 2, line, lpow);
-    else
-      tm = spl_sweep(c, SplRegionOpN<false, 1>{line, hw, RegionPow{c.n, 0}, omega, n1, c.d_err},
-                     SplRegionOpN<false, 1>{line, hw, RegionPow{c.n, 0}, omega, n1, c.d_err}, 1, line, lpow);
-  }
-  if (!tm) return false;
-  k_spl_finish_t<<<grid1d(c.nn), kBlock, 0, c.stream>>>(c.nx, c.ny, *tm, c.dt, hw, c.h, c.b, c.etot, c.erate,
-                                                        c.sedflux);
-  c.count_launch();
-  return true;
-}
+bool region_stream_power(Ctx& c) { return c.mixed ? stream_power_n<float>(c) : stream_power_n<double>(c); }
 
 }  // namespace fsb
