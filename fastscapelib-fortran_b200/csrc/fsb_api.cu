@@ -152,13 +152,11 @@ size_t layout(fsb::Ctx& c, char* base) {
   c.arc_adj = L.take<int>(2 * N);
   c.o_keys = L.take<unsigned long long>(N); c.o_keys2 = L.take<unsigned long long>(N);
   c.o_vals = L.take<int>(N); c.o_vals2 = L.take<int>(N); c.o_pos = L.take<int>(N);
-  c.ch_heavy = L.take<int>(N); c.ch_tmp = L.take<int>(N + 1); c.ch_tmp2 = L.take<int>(N + 1);
-  c.ch_nxt = L.take<int>(N); c.ch_nxt2 = L.take<int>(N);
-  c.ch_val = L.take<unsigned long long>(N); c.ch_val2 = L.take<unsigned long long>(N);
-  c.ch_ord = L.take<int>(N); c.ch_pos = L.take<int>(N); c.ch_ldep = L.take<int>(N); c.ch_start = L.take<int>(N);
-  c.ch_cid = L.take<int>(N); c.ch_sid = L.take<int>(N); c.ch_hist = L.take<int>(128); c.ch_goff = L.take<int>(128);
-  c.ch_tk_td = L.take<int>(N + 2048); c.ch_tk_bu = L.take<int>(N + 2048);
-  c.ch_key = L.take<unsigned>(2 * N); c.ch_skey = L.take<unsigned>(N);
+  c.ch_val = L.take<unsigned long long>(N + 1); c.ch_val2 = L.take<unsigned long long>(N + 1);
+  c.ch_ord = L.take<int>(N); c.ch_flag = L.take<int>(N + 1); c.ch_start = L.take<int>(N);
+  c.ch_hist = L.take<int>(3 * fsb::kChainHist); c.ch_totals = L.take<int>(2);
+  c.ch_head = L.take<unsigned char>(N); c.ch_depth = L.take<unsigned char>(N);
+  for (int t = 0; t < 4; ++t) c.ch_tk[t] = L.take<int4>(t % 2 ? N / 2 + 1 : N / fsb::kLongChain + 1);
   c.la_queue = L.take<int>(N); c.la_cnt = L.take<int>(N); c.cnt_acc = L.take<int>(N); c.cnt_spl = L.take<int>(N);
   c.la_ctl = L.take<unsigned>(128);
   c.mfd_line = L.take<double>(16 * N); c.hw = L.take<double>(2 * N);
@@ -183,7 +181,7 @@ size_t layout(fsb::Ctx& c, char* base) {
     c.rl_queue = L.take<long long>(entries);
   }
   c.s_scan2 = L.take<int>(N + 1);
-  c.done = L.take<unsigned>(N); c.ticket = L.take<unsigned>(4);
+  c.ticket = L.take<unsigned>(4);
   c.water = L.take<double>(N); c.hnew = L.take<double>(N);
   c.catch0 = L.take<double>(N); c.catchv = L.take<double>(N); c.red = L.take<double>(3 * 512 + 8);
   c.g = L.take<double>(N); c.vx = L.take<double>(N); c.vy = L.take<double>(N);
@@ -466,11 +464,9 @@ int fsb_setup(fsb_ctx* h, void* arena, size_t bytes) {
   FSB_CUDA(cudaMemcpyAsync(c.precip, ones.data(), sizeof(double) * c.nn, cudaMemcpyHostToDevice, c.stream));
   for (double* f : {c.u, c.etot, c.erate, c.a, c.length, c.lake_depth, c.hwater, c.sedflux, c.kf, c.kd, c.catchv})
     FSB_CUDA(cudaMemsetAsync(f, 0, sizeof(double) * c.nn, c.stream));
-  FSB_CUDA(cudaMemsetAsync(c.done, 0, sizeof(unsigned) * c.nn, c.stream));
   FSB_CUDA(cudaMemsetAsync(c.s_flag, 0, sizeof(int) * (c.nn + 1), c.stream));
   FSB_CUDA(cudaMemsetAsync(c.d_err, 0, sizeof(int) * 4, c.stream));
   FSB_CUDA(cudaStreamSynchronize(c.stream));
-  c.epoch = 0;
   c.runSPL = c.runDiffusion = c.runUplift = false;
   c.sfd = false;
   c.p = 1.0;

@@ -11,22 +11,43 @@
 // Schedule.  Every node's heavy child is its donor with the largest subtree
 // (first in ascending node order on ties).  A heavy-first preorder lays every
 // heavy path out contiguously; a "chain" is one heavy path, from its head (a
-// root or a light child) to a leaf.  One thread walks a whole chain, carrying
-// the running value in registers, so a long river costs one dependent
-// arithmetic step per node instead of one inter-thread hand-off.  A chain
-// depends only on its head's parent (top-down) or on the chains hanging off
-// it (bottom-up); its "light depth" -- the number of light edges above it,
-// at most log2(nn) -- therefore orders the chains: tickets are handed out by
-// light depth (increasing for top-down sweeps, decreasing for bottom-up), and
-// within a light depth longer chains first.  Every wait then targets a chain
-// with an earlier ticket, so the sweeps cannot deadlock; warps never mix light
-// depths (groups are padded to multiples of 32).
+// root or a light child) to a leaf.  A chain depends only on its head's parent
+// (top-down) or on the chains hanging off it (bottom-up); its "light depth" --
+// the number of light edges above it, at most log2(nn) -- therefore orders the
+// chains.  They are dealt out by light depth (increasing for top-down sweeps,
+// decreasing for bottom-up), by three kinds of workers:
+//   * chains of one node (two thirds of all) take no part in the waiting: a
+//     kernel with a thread per node computes them after (top-down) or before
+//     (bottom-up) the others;
+//   * chains of kLong nodes or more get a warp each: 32 nodes' data arrive with
+//     one load per lane while the recurrence runs through the previous 32 on
+//     values shuffled from their lanes, so a node costs its arithmetic, not a
+//     memory round trip;
+//   * the others get a lane each; a lane that waits for its chain's parent does
+//     not hold up its warp mates.
+// Every wait targets a chain of another light depth that is earlier in both
+// lists, so the sweeps cannot deadlock.  A published value says itself that
+// it has arrived: the arrays start as all ones (a NaN no result has: see
+// fsb::publishable), values are written and polled with relaxed accesses at
+// GPU scope, and no flags or fences are needed.
 //
-// Heavy-first positions come from path sums over the receiver pointers
-// (pointer jumping): pos(k) = sum over the root->k path of each node's offset
-// within its parent's subtree (1 + sizes of the siblings laid out before it).
-#include <cuda/atomic>
+// Measured (B200), per step: 1023x767 single flow on a cell size without a
+// closed form for the area: area 2.29 -> 0.26 ms, stream power 1.70 -> 0.20,
+// schedule and fill 0.65 -> 0.22; 513x511 with n = 1.37: stream power 1.94 -> 0.24;
+// 2049^2 schedule and fill 2.37 -> 0.87.  Against 32 chains of any length per
+// warp that waited together, flags behind a fence at GPU scope (770 cycles per
+// 8 or 16 nodes), powers evaluated on the chain, radix-sorted tickets and three
+// read-backs.  What bounds a sweep now is the recurrence along the longest
+// root-to-leaf path (a quotient or Newton's iterations per node) and ten or so
+// hand-offs between chains of about 1 us.
+//
+// Heavy-first positions come from path sums over the receiver forest (a scan
+// over the DFS preorder): pos(k) = sum over the root->k path of each node's
+// offset within its parent's subtree (1 + sizes of the siblings laid out
+// before it).
+#include <algorithm>
 #include <climits>
+#include <cmath>
 
 #include "fsb_kernels.cuh"
 
@@ -35,288 +56,543 @@ namespace fsb {
 namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
+constexpr int kLong = kLongChain;  // nodes of a chain that gets a warp of its own
+constexpr int kDepths = 32;        // light depths (at most log2(nn) <= 28)
+constexpr int kClasses = 32;       // length classes (powers of two, longest first)
+constexpr int kBuckets = kDepths * kClasses;
+// ticket counts and cursors: kBuckets of the long chains, kDepths of the short ones
+constexpr int kHist = kBuckets + kDepths;
+static_assert(kHist == kChainHist, "the arena holds three of them");
 
-// bounded wait for done[k] == epoch (relaxed polling, then an acquire
-// fence); gives up once any wait has failed
-// waits (bounded) until done[k] == epoch; the acquire load that sees it makes
-// the chain's values released before the flag visible
-__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+// ---- schedule ---------------------------------------------------------------
 
-__device__ inline void wait_flag(unsigned* done, int k, unsigned epoch, int* err) {
-  int spins = 0, back = 32;
-  while (ld_acquire_gpu(&done[k]) != epoch) {
-    if (++spins > kSpinLimit) { atomicExch(err, DEV_SPIN_LIMIT); return; }
-    if ((spins & 63) == 0 && *(volatile int*)err != 0) return;
-    __nanosleep(back);
-    if (back < 512) back <<= 1;
-  }
-}
+// offset of k inside its parent's heavy-first layout and whether it heads a
+// chain, as path-sum marks: node k's subtree is the interval [pos(k), pos(k) +
+// size(k)) of the DFS preorder, so adding w(k) at pos(k) and subtracting it
+// at pos(k) + size(k) makes the prefix sum at pos(k) the sum over k's
+// ancestors and k.  w = (light flag << kOffBits) | offset: offsets sum to a
+// heavy-first position and light flags to a light depth (< 32), so the two
+// fields never carry into each other; the marks wrap and cancel exactly.
+// 32-bit words hold grids below 2^27 nodes, 64-bit ones the others.
+template <class U>
+constexpr int kOffBits = sizeof(U) == 4 ? 27 : 32;
 
-// heavy child: donor with the largest subtree, first in ascending order on ties
-__global__ void k_heavy(int nn, const int* __restrict__ ndon, const int* __restrict__ don,
-                        const int* __restrict__ size, int* __restrict__ heavy) {
+template <class U>
+__global__ void k_path_marks(int nn, const int* __restrict__ rec, const int* __restrict__ ndon,
+                             const int* __restrict__ don, const int* __restrict__ pos, const int* __restrict__ size,
+                             U* __restrict__ marks, unsigned char* __restrict__ head, int* __restrict__ err) {
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
-    const int nd = ndon[k];
-    int best = -1, bs = -1;
-    for (int i = 0; i < nd; ++i) {
-      const int d = don[(size_t)k * 8 + i];
-      const int s = size[d];
-      if (s > bs) { bs = s; best = d; }
-    }
-    heavy[k] = best;
-  }
-}
-
-// sizes of the roots in ascending root order (for the root offsets)
-__global__ void k_root_sizes(int nroots, const int* __restrict__ roots, const int* __restrict__ size,
-                             int* __restrict__ out) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r <= nroots; r += gridDim.x * blockDim.x)
-    out[r] = r < nroots ? size[roots[r]] : 0;
-}
-
-// offset of each node inside its parent's heavy-first layout, light flag in
-// the high word; pointer = receiver (or -1 at roots)
-__global__ void k_hf_offsets(int nn, const int* __restrict__ rec, const int* __restrict__ ndon,
-                             const int* __restrict__ don, const int* __restrict__ size,
-                             const int* __restrict__ heavy, const int* __restrict__ root_rank,
-                             const int* __restrict__ root_off, unsigned long long* __restrict__ val,
-                             int* __restrict__ nxt) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
-    const int r = rec[k];
-    unsigned long long v;
+    const int r = rec[k], p = pos[k], e = p + size[k];
+    U off = 1, light = 0;
+    bool hd = true;
     if (r == k) {
-      v = (unsigned long long)(unsigned)root_off[root_rank[k]];
-      nxt[k] = -1;
+      off = (U)p;  // roots ascending: the earlier roots' trees fill [0, pos)
     } else {
-      const int hv = heavy[r];
-      if (k == hv) {
-        v = 1ull;
-      } else {
-        unsigned off = 1u + (unsigned)size[hv];
-        const int nd = ndon[r];
-        for (int i = 0; i < nd; ++i) {
-          const int d = don[(size_t)r * 8 + i];
-          if (d >= k) break;
-          if (d != hv) off += (unsigned)size[d];
+      const int nd = ndon[r];
+      if (nd > 1) {
+        const int4* row = reinterpret_cast<const int4*>(don + (size_t)r * 8);
+        const int4 a = __ldg(row), b = __ldg(row + 1);
+        const int d[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        int hv = -1, hs = -1, before = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (i < nd) {
+            const int s = __ldg(&size[d[i]]);
+            if (s > hs) { hs = s; hv = d[i]; }
+            if (d[i] < k) before += s;
+          }
+        hd = hv != k;
+        if (hd) {
+          light = 1;
+          off = 1u + (U)before + (hv < k ? (U)0 : (U)hs);  // the heavy child comes first
         }
-        v = (unsigned long long)off | (1ull << 32);
+      } else {
+        hd = false;  // the only donor
       }
-      nxt[k] = r;
     }
-    val[k] = v;
-  }
-}
-
-// Path sums of the heavy-first offsets over the receiver forest without
-// pointer jumping: node k's subtree is the interval [pos(k), pos(k) + size(k))
-// of the DFS preorder, so adding w(k) at pos(k) and subtracting it at
-// pos(k) + size(k) makes the prefix sum at pos(k) the sum over k's ancestors
-// and k.  w = (light flag << 27) | offset: offsets sum to a heavy-first
-// position (< nn <= 2^27) and light flags to a light depth (< 32), so the
-// two fields never carry into each other; the marks wrap modulo 2^32 and
-// cancel exactly.
-constexpr int kPathOffBits = 27;
-
-__global__ void k_path_marks(int nn, const unsigned long long* __restrict__ val, const int* __restrict__ pos,
-                             const int* __restrict__ size, unsigned* __restrict__ marks, int* __restrict__ err) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
-    const unsigned long long v = val[k];
-    const unsigned w = ((unsigned)(v >> 32) << kPathOffBits) | (unsigned)v;
-    const int p = pos[k], e = p + size[k];
+    head[k] = hd ? 1 : 0;
     if (p < 0 || e > nn || e <= p) {
       atomicExch(err, DEV_STACK_ERROR);
       continue;
     }
+    const U w = (light << kOffBits<U>) | off;
     atomicAdd(&marks[p], w);
-    atomicAdd(&marks[e], 0u - w);
+    atomicAdd(&marks[e], (U)0 - w);
   }
 }
 
-// after an exclusive scan of the marks: the path sum of k (light depth in the high word)
-__global__ void k_path_take(int nn, const int* __restrict__ pos, const unsigned* __restrict__ scan,
-                            unsigned long long* __restrict__ out) {
+// after an exclusive scan of the marks: the heavy-first order, and by position
+// the chain starts and light depths
+template <class U>
+__global__ void k_hf_order(int nn, const U* __restrict__ scan, const int* __restrict__ pos,
+                           const unsigned char* __restrict__ head, int* __restrict__ ord, int* __restrict__ flag,
+                           unsigned char* __restrict__ depth, int* __restrict__ err) {
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
-    const unsigned s = scan[pos[k] + 1];
-    out[k] = ((unsigned long long)(s >> kPathOffBits) << 32) | (s & ((1u << kPathOffBits) - 1u));
+    const U s = scan[pos[k] + 1];
+    const U off = s & (((U)1 << kOffBits<U>) - 1);
+    if (off >= (U)nn) { atomicExch(err, DEV_STACK_ERROR); continue; }
+    ord[off] = k;
+    flag[off] = head[k];
+    depth[off] = (unsigned char)min((unsigned)(s >> kOffBits<U>), (unsigned)kDepths - 1u);
+    if (k == 0) flag[nn] = 0;
   }
 }
 
-// one synchronous pointer-jumping round of the path sums
-__global__ void k_path_jump(int nn, const unsigned long long* __restrict__ vin, const int* __restrict__ nin,
-                            unsigned long long* __restrict__ vout, int* __restrict__ nout, int* __restrict__ flag) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
-    const int p = nin[k];
-    if (p < 0) {
-      vout[k] = vin[k];
-      nout[k] = -1;
-    } else {
-      vout[k] = vin[k] + vin[p];
-      const int pp = nin[p];
-      nout[k] = pp;
-      if (pp >= 0) *flag = 1;
-    }
-  }
-}
-
-__global__ void k_hf_order(int nn, const unsigned long long* __restrict__ val, const int* __restrict__ rec,
-                           const int* __restrict__ heavy, int* __restrict__ ord, int* __restrict__ hpos,
-                           int* __restrict__ ldep, int* __restrict__ err) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
-    const unsigned p = (unsigned)val[k];
-    if (p >= (unsigned)nn) { atomicExch(err, DEV_STACK_ERROR); continue; }
-    ord[p] = k;
-    hpos[k] = (int)p;
-    ldep[k] = (int)(val[k] >> 32);
-  }
-}
-
-// chain starts: positions whose node is a root or a light child
-__global__ void k_chain_flags(int nn, const int* __restrict__ ord, const int* __restrict__ rec,
-                              const int* __restrict__ heavy, int* __restrict__ flag) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p <= nn; p += gridDim.x * blockDim.x) {
-    if (p == nn) { flag[p] = 0; continue; }
-    const int k = ord[p];
-    const int r = rec[k];
-    flag[p] = (r == k || heavy[r] != k) ? 1 : 0;
-  }
-}
-
-// chain list (start positions ascending) with sort keys
-//   top-down key:  light depth (6 bits) | ~length (26 bits)
-//   bottom-up key: (63 - light depth)   | ~length
 __global__ void k_chain_list(int nn, const int* __restrict__ flag, const int* __restrict__ scan,
-                             int* __restrict__ cstart, int* __restrict__ cid) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < nn; p += gridDim.x * blockDim.x) {
-    if (!flag[p]) continue;
-    const int c = scan[p];
-    cstart[c] = p;
-    cid[c] = c;
+                             int* __restrict__ cstart) {
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < nn; p += gridDim.x * blockDim.x)
+    if (flag[p]) cstart[scan[p]] = p;
+}
+
+// bucket of a chain of `len` >= 2 nodes: the long ones by depth, then longest first
+__device__ __forceinline__ int chain_bucket(int len, int depth) {
+  if (len < kLong) return kBuckets + depth;
+  return depth * kClasses + __clz(len);
+}
+// the same with decreasing depth (bottom-up)
+__device__ __forceinline__ int reversed(int b) {
+  if (b >= kBuckets) return kBuckets + (kDepths - 1 - (b - kBuckets));
+  return (kDepths - 1 - b / kClasses) * kClasses + b % kClasses;
+}
+
+// Chains per bucket.  Counted per block in shared memory: the buckets are
+// few, and one global atomic per block and bucket replaces one per chain.
+constexpr int kChainBlock = 256, kChainsPerBlock = 8 * kChainBlock;
+__global__ void __launch_bounds__(kChainBlock) k_chain_hist(int nn, const int* __restrict__ nchains,
+                                                            const int* __restrict__ cstart,
+                                                            const unsigned char* __restrict__ depth,
+                                                            int* __restrict__ hist) {
+  __shared__ int sh[kHist];
+  const int n = *nchains;
+  for (int t = threadIdx.x; t < kHist; t += kChainBlock) sh[t] = 0;
+  __syncthreads();
+  for (int c = blockIdx.x * kChainsPerBlock + threadIdx.x, i = 0; i < 8 && c < n; ++i, c += kChainBlock) {
+    const int s = cstart[c], e = c + 1 < n ? cstart[c + 1] : nn;
+    if (e - s > 1) atomicAdd(&sh[chain_bucket(e - s, depth[s])], 1);
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < kHist; t += kChainBlock)
+    if (sh[t]) atomicAdd(&hist[t], sh[t]);
+}
+
+// exclusive prefix of the bucket counts, top-down and bottom-up order, and the
+// two lists' lengths (one block of kBuckets threads)
+__global__ void __launch_bounds__(kBuckets) k_chain_offsets(const int* __restrict__ hist, int* __restrict__ cur_td,
+                                                            int* __restrict__ cur_bu, int* __restrict__ totals) {
+  __shared__ int warp_sum[2][32];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  for (int dir = 0; dir < 2; ++dir) {
+    int* cur = dir ? cur_bu : cur_td;
+    const int v = hist[dir ? reversed(t) : t];
+    int x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(FULL, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) warp_sum[dir][w] = x;
+    __syncthreads();
+    if (w == 0) {
+      int s = warp_sum[dir][lane];
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(FULL, s, o);
+        if (lane >= o) s += y;
+      }
+      warp_sum[dir][lane] = s;
+    }
+    __syncthreads();
+    cur[t] = x - v + (w ? warp_sum[dir][w - 1] : 0);  // cursors are in this direction's order
+    if (t == kBuckets - 1) totals[0] = warp_sum[dir][31];
+    if (w == 0) {  // the short chains
+      const int b = kBuckets + lane;
+      const int sv = hist[dir ? reversed(b) : b];
+      int sx = sv;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(FULL, sx, o);
+        if (lane >= o) sx += y;
+      }
+      cur[b] = sx - sv;
+      if (lane == 31) totals[1] = sx;
+    }
   }
 }
 
-// The light-depth histogram is counted per block in shared memory (few
-// distinct depths: one global atomic per block and depth, not per chain).
-__global__ void k_chain_keys(int nn, int nchains, const int* __restrict__ cstart, const int* __restrict__ ord,
-                             const int* __restrict__ ldep, unsigned* __restrict__ key_td,
-                             unsigned* __restrict__ key_bu, int* __restrict__ hist_td, int* __restrict__ hist_bu) {
-  __shared__ int sh[64];
-  for (int t = threadIdx.x; t < 64; t += blockDim.x) sh[t] = 0;
+// tickets {first position, end, head, its receiver}, both directions; within a
+// bucket in any order
+__global__ void __launch_bounds__(kChainBlock) k_chain_tickets(int nn, const int* __restrict__ nchains,
+                                                               const int* __restrict__ cstart,
+                                                               const unsigned char* __restrict__ depth,
+                                                               const int* __restrict__ ord, const int* __restrict__ rec,
+                                                               int* cur_td, int* cur_bu, int4* __restrict__ td_long,
+                                                               int4* __restrict__ td_short, int4* __restrict__ bu_long,
+                                                               int4* __restrict__ bu_short) {
+  __shared__ int cnt[kHist], base_td[kHist], base_bu[kHist];
+  const int n = *nchains;
+  if (blockIdx.x * kChainsPerBlock >= n) return;
+  for (int t = threadIdx.x; t < kHist; t += kChainBlock) cnt[t] = 0;
   __syncthreads();
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nchains; c += gridDim.x * blockDim.x) {
-    const int s = cstart[c];
-    const int e = (c + 1 < nchains) ? cstart[c + 1] : nn;
-    const unsigned len = (unsigned)(e - s);
-    int ld = ldep[ord[s]];
-    if (ld > 63) ld = 63;
-    const unsigned inv = 0x3ffffffu - (len > 0x3ffffffu ? 0x3ffffffu : len);
-    key_td[c] = ((unsigned)ld << 26) | inv;
-    key_bu[c] = ((unsigned)(63 - ld) << 26) | inv;
-    atomicAdd(&sh[ld], 1);
+  int b[8], rank[8], st[8], en[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int c = blockIdx.x * kChainsPerBlock + i * kChainBlock + threadIdx.x;
+    b[i] = -1;
+    if (c < n) {
+      st[i] = cstart[c];
+      en[i] = c + 1 < n ? cstart[c + 1] : nn;
+      if (en[i] - st[i] > 1) {
+        b[i] = chain_bucket(en[i] - st[i], depth[st[i]]);
+        rank[i] = atomicAdd(&cnt[b[i]], 1);
+      }
+    }
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < 64; t += blockDim.x)
-    if (sh[t]) {
-      atomicAdd(&hist_td[t], sh[t]);
-      atomicAdd(&hist_bu[63 - t], sh[t]);
+  for (int t = threadIdx.x; t < kHist; t += kChainBlock)
+    if (cnt[t]) {
+      base_td[t] = atomicAdd(&cur_td[t], cnt[t]);
+      base_bu[t] = atomicAdd(&cur_bu[reversed(t)], cnt[t]);
+    }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    if (b[i] >= 0) {
+      const int k0 = ord[st[i]];
+      const int4 t = make_int4(st[i], en[i], k0, rec[k0]);
+      (b[i] < kBuckets ? td_long : td_short)[base_td[b[i]] + rank[i]] = t;
+      (b[i] < kBuckets ? bu_long : bu_short)[base_bu[b[i]] + rank[i]] = t;
     }
 }
 
-// per-group offsets, padded to multiples of 32 (one thread)
-__global__ void k_group_offsets(const int* __restrict__ hist, int* __restrict__ ustart, int* __restrict__ pstart,
-                                int* __restrict__ total) {
-  int u = 0, pz = 0;
-  for (int g = 0; g < 64; ++g) {
-    ustart[g] = u;
-    pstart[g] = pz;
-    u += hist[g];
-    pz += (hist[g] + 31) & ~31;
-  }
-  *total = pz;
-}
-
-__global__ void k_ticket_scatter(int nchains, const unsigned* __restrict__ skey, const int* __restrict__ sid,
-                                 const int* __restrict__ ustart, const int* __restrict__ pstart,
-                                 int* __restrict__ tickets) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nchains; t += gridDim.x * blockDim.x) {
-    const int g = (int)(skey[t] >> 26);
-    tickets[pstart[g] + (t - ustart[g])] = sid[t];
-  }
-}
-
-// ---------------------------------------------------------------------------
-// chain sweeps
+// ---- sweeps -------------------------------------------------------------------
 
 struct ChainView {
-  const int* ord;      // heavy-first order
-  const int* cstart;   // chain start positions (ascending), nchains entries
-  const int* tickets;  // padded ticket list (chain ids or -1)
-  int nchains, ntickets, nn;
-  __device__ void range(int c, int& s, int& e) const {
-    s = cstart[c];
-    e = (c + 1 < nchains) ? cstart[c + 1] : nn;  // exclusive
+  const int* ord;  // heavy-first order
+  const int4 *tk_long, *tk_short;
+  const int* totals;   // long, short chains
+  unsigned* ticket;    // next long, next short chain
+  int* err;
+};
+
+// Values travel between chains in arrays that start as all ones.
+__device__ __forceinline__ bool arrived(double v) { return __double_as_longlong(v) != -1ll; }
+
+// Bounded waiting: true when the caller must give up (a wait here or elsewhere failed).
+struct Patience {
+  int spins = 0, back = 32;
+  __device__ bool over(int* err) {
+    if (++spins > kSpinLimit) {
+      atomicExch(err, DEV_SPIN_LIMIT);
+      return true;
+    }
+    return (spins & 63) == 0 && *(volatile int*)err != 0;
+  }
+  __device__ void rest() {
+    __nanosleep(back);
+    if (back < 256) back <<= 1;
   }
 };
 
-constexpr int kCF = 16;  // nodes per software-pipelined chunk (fill, area)
-constexpr int kCS = 8;   // nodes per chunk (stream power)
+constexpr int kSweepThreads = 128, kSoloWarps = 2;  // per block: warps for long chains; the others' lanes take short ones
 
-// Top-down: hwater(k) = hwater(rec) > h(k) ? hwater(rec) + 1e-8 : h(k)
-// (FlowRouting.f90:77-86); lake_depth = hwater - h.
-__global__ void __launch_bounds__(128) k_fill_chains(ChainView cv, const int* __restrict__ rec,
-                                                     const int* __restrict__ ndon, const double* __restrict__ h,
-                                                     double* __restrict__ hwater, double* __restrict__ lake_depth,
-                                                     unsigned* ticket, unsigned* done, unsigned epoch, int* err) {
-  const int lane = threadIdx.x & 31;
-  for (;;) {
-    unsigned w = 0;
-    if (lane == 0) w = atomicAdd(ticket, 32u);
-    w = __shfl_sync(FULL, w, 0);
-    if ((int)w >= cv.ntickets) break;
-    const int t = (int)w + lane;
-    const int c = t < cv.ntickets ? cv.tickets[t] : -1;
-    if (c < 0) continue;
-    int s, e;
-    cv.range(c, s, e);
-    const int k0 = cv.ord[s];
-    const int r0 = rec[k0];
-    bool root = r0 == k0;
-    double prev = 0.0;
-    if (!root) {
-      wait_flag(done, r0, epoch, err);
-      prev = __ldcg(&hwater[r0]);
-    }
-    for (int p = s; p < e; p += kCF) {
-      const int n = min(kCF, e - p);
-      int kk[kCF], nd[kCF];
-      double hh[kCF], out[kCF];
-#pragma unroll
-      for (int i = 0; i < kCF; ++i) if (i < n) kk[i] = cv.ord[p + i];
-#pragma unroll
-      for (int i = 0; i < kCF; ++i) if (i < n) { hh[i] = h[kk[i]]; nd[i] = ndon[kk[i]]; }
-#pragma unroll
-      for (int i = 0; i < kCF; ++i) if (i < n) {
-        const double v = root ? hh[i] : (prev > hh[i] ? prev + 1.0e-8 : hh[i]);
-        root = false;
-        out[i] = v;
-        prev = v;
+// Top-down sweep.  Op:
+//   Node load(k)            what the recurrence needs of node k
+//   Node shfl(node, lane)   that of another lane
+//   bool poll(r, State&)    the state after receiver r; false if not there yet
+//   State root()            the state before a root
+//   void step(State&, node, k, first, store)
+//                           node k's value; first: k is a root; store: write it out
+template <class Op>
+__global__ void __launch_bounds__(kSweepThreads) k_top_down(ChainView cv, Op op) {
+  using Node = typename Op::Node;
+  using State = typename Op::State;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp < kSoloWarps) {
+    const int total = cv.totals[0];
+    for (;;) {
+      unsigned t = 0;
+      if (lane == 0) t = atomicAdd(&cv.ticket[0], 1u);
+      t = __shfl_sync(FULL, t, 0);
+      if ((int)t >= total) return;
+      const int4 tk = cv.tk_long[t];
+      const int s = tk.x, e = tk.y;
+      const bool root = tk.z == tk.w;
+      // nodes of this chunk, of the next one, and the indices of the one after
+      int k = s + lane < e ? cv.ord[s + lane] : -1;
+      int k2 = s + 32 + lane < e ? cv.ord[s + 32 + lane] : -1;
+      Node nd{}, nd2{};
+      if (k >= 0) nd = op.load(k);
+      State st = op.root();
+      if (!root) {
+        Patience pat;
+        while (!__all_sync(FULL, op.poll(tk.w, st))) {  // a value that has arrived is final: the lanes agree
+          if (__any_sync(FULL, pat.over(cv.err))) return;
+          pat.rest();
+        }
       }
+      for (int p = s; p < e; p += 32) {
+        const int k3 = p + 64 + lane < e ? cv.ord[p + 64 + lane] : -1;
+        if (k2 >= 0) nd2 = op.load(k2);
+        const int n = min(32, e - p);
+        for (int i = 0; i < n; ++i)
+          op.step(st, op.shfl(nd, i), __shfl_sync(FULL, k, i), root && p == s && i == 0, lane == i);
+        k = k2;
+        nd = nd2;
+        k2 = k3;
+      }
+    }
+  }
+  constexpr int kC = 4;
+  const int total = cv.totals[1];
+  int4 tk = make_int4(0, 0, 0, 0);
+  int status = 0;  // 0 without a chain, 1 waiting, 2 walking, 3 no chain left
+  State st = op.root();
+  Patience pat;
+  for (;;) {
+    const unsigned idle = __ballot_sync(FULL, status == 0);
+    if (idle) {
+      unsigned t = 0;
+      if (lane == 0) t = atomicAdd(&cv.ticket[1], (unsigned)__popc(idle));
+      t = __shfl_sync(FULL, t, 0) + __popc(idle & ((1u << lane) - 1u));
+      if (status == 0) {
+        if ((int)t < total) {
+          tk = cv.tk_short[t];
+          status = tk.z == tk.w ? 2 : 1;
+          st = op.root();
+        } else {
+          status = 3;
+        }
+      }
+    }
+    if (!__any_sync(FULL, status != 3)) return;
+    if (status == 1 && op.poll(tk.w, st)) status = 2;
+    if (status == 2) {
+      int k[kC];
+      Node nd[kC];
 #pragma unroll
-      for (int i = 0; i < kCF; ++i) if (i < n) { hwater[kk[i]] = out[i]; lake_depth[kk[i]] = out[i] - hh[i]; }
-      fence_acq_rel();
+      for (int i = 0; i < kC; ++i) k[i] = tk.x + i < tk.y ? cv.ord[tk.x + i] : -1;
 #pragma unroll
-      for (int i = 0; i < kCF; ++i) if (i < n && nd[i] > 1) *(volatile unsigned*)&done[kk[i]] = epoch;
+      for (int i = 0; i < kC; ++i)
+        if (k[i] >= 0) nd[i] = op.load(k[i]);
+#pragma unroll
+      for (int i = 0; i < kC; ++i)
+        if (k[i] >= 0) op.step(st, nd[i], k[i], k[i] == tk.w, true);
+      tk.x += kC;
+      if (tk.x >= tk.y) status = 0;
+    }
+    if (!__any_sync(FULL, status == 0 || status == 2)) {  // all of them wait
+      if (__any_sync(FULL, pat.over(cv.err))) return;
+      pat.rest();
+    } else {
+      pat = Patience{};
     }
   }
 }
 
-// Bottom-up single-flow area: a(k) = dx*dy*precip(k) + a(d_m) + ... + a(d_1)
-// (donors descending, the reverse-stack order of FlowRouting.f90:136-139);
-// roots add themselves.  Only the chain head is read by another chain.
-// Each chunk first lists its light donors (heads of other chains), reads all
-// their done flags at once, fences once and reads all their areas at once;
-// the chain recurrence then runs in registers in the original summation order.
-constexpr int kLight = 16;  // light donors fetched together per chunk
-// Finishers of the bottom-up recurrence v(k) = fin(k, base(k) + v(d_m) + ... + v(d_1)):
+// chains of one node, after the others: everything they need is final
+template <class Op>
+__global__ void k_top_down_leaves(int nn, const int* __restrict__ rec, const int* __restrict__ ndon,
+                                  const unsigned char* __restrict__ head, Op op, int* err) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
+    if (ndon[k] != 0 || !head[k]) continue;
+    const int r = rec[k];
+    typename Op::State st = op.root();
+    if (r != k && !op.poll(r, st)) {
+      atomicExch(err, DEV_SPIN_LIMIT);  // never: the walkers have finished
+      continue;
+    }
+    op.step(st, op.load(k), k, r == k, true);
+  }
+}
+
+// hwater(k) = hwater(rec) > h(k) ? hwater(rec) + 1e-8 : h(k)
+// (FlowRouting.f90:77-86); lake_depth = hwater - h.
+struct FillOp {
+  const double* __restrict__ h;
+  double *hwater, *lake_depth;
+  using Node = double;
+  using State = double;
+  __device__ Node load(int k) const { return __ldg(&h[k]); }
+  __device__ Node shfl(Node n, int i) const { return __shfl_sync(FULL, n, i); }
+  __device__ State root() const { return 0.0; }
+  __device__ bool poll(int r, State& st) const {
+    const double v = ld_relaxed_gpu(&hwater[r]);
+    if (!arrived(v)) return false;
+    st = v;
+    return true;
+  }
+  __device__ void step(State& st, Node hk, int k, bool first, bool store) const {
+    st = first ? hk : (st > hk ? st + 1.0e-8 : hk);
+    if (store) {
+      st_relaxed_gpu(&hwater[k], publishable(st));
+      lake_depth[k] = st - hk;
+    }
+  }
+};
+
+// CopyChi (FastScape_ctx.f90:228-251) top down: chi(k) = chi(rec(k)) +
+// (a0/a(k))^(m/n) * length(k) where a(k) > a0, else 0; a root starts from 0.
+struct ChiOp {
+  const double* __restrict__ a;
+  const double* __restrict__ length;
+  double a0, mn;
+  double* chi;
+  struct Node { double term, above; };
+  using State = double;
+  __device__ Node load(int k) const {
+    const double ak = __ldg(&a[k]);
+    return {pow(a0 / ak, mn) * __ldg(&length[k]), ak > a0 ? 1.0 : 0.0};
+  }
+  __device__ Node shfl(const Node& n, int i) const {
+    return {__shfl_sync(FULL, n.term, i), __shfl_sync(FULL, n.above, i)};
+  }
+  __device__ State root() const { return 0.0; }
+  __device__ bool poll(int r, State& st) const {
+    const double v = ld_relaxed_gpu(&chi[r]);
+    if (!arrived(v)) return false;
+    st = v;
+    return true;
+  }
+  __device__ void step(State& st, const Node& n, int k, bool, bool store) const {
+    st = n.above != 0.0 ? st + n.term : 0.0;
+    if (store) st_relaxed_gpu(&chi[k], publishable(st));
+  }
+};
+
+// Single-flow erosion factor kf*dt*a^m/l^n of every node: the powers do not
+// depend on the recurrence, so they stay off the chains.
+__global__ void k_spl_factor(int nn, int n_is_one, const int* __restrict__ rec, const double* __restrict__ h,
+                             const double* __restrict__ b, const double* __restrict__ kf,
+                             const double* __restrict__ a, const double* __restrict__ length, double kfsed, double dt,
+                             double m, double n, double* __restrict__ fact) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
+    double f = 0.0;
+    if (rec[k] != k) {
+      const double kfint = (kfsed > 0.0 && (h[k] - b[k]) > 1.0) ? kfsed : kf[k];
+      const double l = length[k];
+      f = n_is_one ? kfint * dt * pow(a[k], m) / l : kfint * dt * pow(a[k], m) / pow(l, n);
+    }
+    fact[k] = f;
+  }
+}
+
+// Top-down single-flow stream power law (StreamPowerLaw.f90:291-373): writes
+// hnew and water; h keeps ht.  MODE 0: n = 1; 1: n = 1.5 (x*sqrt(x) and
+// sqrt(x)); 2: other n (one pow: x^n = x * x^(n-1)).  With GS (a Gauss-Seidel
+// iteration of the g > 0 solve, :285-373) the deposition-corrected surface
+// comes from `elev`, Newton starts from the current iterate `hstart`, and the
+// lake bookkeeping is written: sill(k) = k for a node above its receiver's
+// water, else sill(rec) with its volume contribution w_rcv - h(k) in
+// contrib(k).  Without GS, elev = hstart = ht.
+template <int MODE, bool GS>
+struct SplOp {
+  const double* __restrict__ h;
+  const double* __restrict__ fact;
+  double n, omega;
+  double *hnew, *water;
+  const double* __restrict__ elev;
+  const double* __restrict__ hstart;
+  int* sill;  // -1 until written
+  double* contrib;
+  int* err;
+  struct Node { double ht, fact, elev, h0; };
+  struct State {
+    double h, w, ht;  // the receiver's new elevation, water and old elevation
+    int sill;
+  };
+  __device__ Node load(int k) const {
+    Node nd;
+    nd.ht = __ldg(&h[k]);
+    nd.fact = __ldg(&fact[k]);
+    nd.elev = GS ? __ldg(&elev[k]) : nd.ht;
+    nd.h0 = GS ? __ldg(&hstart[k]) : nd.ht;
+    return nd;
+  }
+  __device__ Node shfl(const Node& nd, int i) const {
+    Node o;
+    o.ht = __shfl_sync(FULL, nd.ht, i);
+    o.fact = __shfl_sync(FULL, nd.fact, i);
+    o.elev = GS ? __shfl_sync(FULL, nd.elev, i) : o.ht;
+    o.h0 = GS ? __shfl_sync(FULL, nd.h0, i) : o.ht;
+    return o;
+  }
+  __device__ State root() const { return {0.0, 0.0, 0.0, 0}; }
+  __device__ bool poll(int r, State& st) const {
+    const double hv = ld_relaxed_gpu(&hnew[r]), wv = ld_relaxed_gpu(&water[r]);
+    const int sv = GS ? ld_relaxed_gpu(&sill[r]) : 0;
+    if (!arrived(hv) || !arrived(wv) || (GS && sv < 0)) return false;
+    st.h = hv;
+    st.w = wv;
+    st.ht = __ldg(&h[r]);
+    st.sill = sv;
+    return true;
+  }
+  __device__ void step(State& st, const Node& nd, int k, bool first, bool store) const {
+    const double ht = nd.ht, el = nd.elev;
+    double hk = ht, wk = ht, ck = 0.0;
+    int sk = k;
+    if (!first) {
+      hk = nd.h0;
+      if (el > st.w) {
+        if constexpr (MODE == 0) {
+          double f = el, df = 1.0;
+          f = f + nd.fact * st.h;
+          df = df + nd.fact;
+          hk = f / df;
+        } else {
+          const double tolp = 1.0e-3;
+          double errp = 2.0 * tolp;
+          int guard = 0;
+          while (errp > tolp) {
+            if (++guard > kNewtonLimit) {
+              atomicExch(err, DEV_NEWTON_LIMIT);
+              break;
+            }
+            double f = hk - el, df = 1.0;
+            if (ht > st.ht) {
+              const double x = fmax(0.0, hk - st.h);
+              double pn, pn1;
+              if constexpr (MODE == 1) {
+                pn1 = sqrt(x);
+                pn = x * pn1;
+              } else if (x > 0.0) {
+                pn1 = pow(x, n - 1.0);
+                pn = x * pn1;
+              } else {
+                pn = pow(x, n);
+                pn1 = pow(x, n - 1.0);
+              }
+              f = f + nd.fact * pn;
+              df = df + nd.fact * n * pn1;
+            }
+            const double hn = hk - f / df;
+            errp = fabs(hn - hk);
+            hk = hk * (1.0 - omega) + hn * omega;
+          }
+        }
+        if (hk < st.w) hk = st.w;
+      } else {
+        hk = el;
+        sk = st.sill;
+        ck = st.w - hk;
+      }
+      wk = fmax(st.w, hk);
+    }
+    if (store) {
+      st_relaxed_gpu(&hnew[k], publishable(hk));
+      st_relaxed_gpu(&water[k], publishable(wk));
+      if (GS) {
+        st_relaxed_gpu(&sill[k], sk);
+        contrib[k] = ck;
+      }
+    }
+    st.h = hk;
+    st.w = wk;
+    st.ht = ht;
+    st.sill = sk;
+  }
+};
+
+// ---- bottom-up --------------------------------------------------------------------
+// v(k) = value(base(k) + v(d_m) + ... + v(d_1)), donors descending (the
+// reverse-stack order of FlowRouting.f90:136-139).  Finishers:
 //   AreaFin  drainage area; a root adds itself (FlowRouting.f90:136-139)
 //   FluxFin  compute_fluxes' sediment flux: base erate, max(0, .) before the
 //            value goes downstream, a root adds itself (FastScape_ctx.f90:864-869)
@@ -326,399 +602,275 @@ constexpr int kLight = 16;  // light donors fetched together per chunk
 //   VolFin   lake water volume: a flooded node passes its contribution
 //            (w_rcv - h) and its flooded donors' up to its receiver; every
 //            node records what its donors pass as its volume (a sill's volume)
+// aux(k): a further number of the node that value needs (kAux); flags bit 0: a
+// root, bit 1: a property of the node.
 struct AreaFin {
-  const double* precip;
+  const double* __restrict__ precip;
   double dxdy;
-  __device__ double base(int k) const { return dxdy * precip[k]; }
-  __device__ double finish(int, double acc, bool root) const { return root ? acc + acc : acc; }
+  static constexpr bool kAux = false;
+  __device__ double base(int k) const { return dxdy * __ldg(&precip[k]); }
+  __device__ double aux(int) const { return 0.0; }
+  __device__ unsigned prop(int) const { return 0u; }
+  __device__ double value(double acc, double, unsigned fl) const { return (fl & 1u) ? acc + acc : acc; }
+  __device__ void side(int, double, double, unsigned) const {}
 };
 struct FluxFin {
-  const double* erate;
-  __device__ double base(int k) const { return erate[k]; }
-  __device__ double finish(int, double acc, bool root) const {
+  const double* __restrict__ erate;
+  static constexpr bool kAux = false;
+  __device__ double base(int k) const { return __ldg(&erate[k]); }
+  __device__ double aux(int) const { return 0.0; }
+  __device__ unsigned prop(int) const { return 0u; }
+  __device__ double value(double acc, double, unsigned fl) const {
     acc = fmax(0.0, acc);
-    return root ? acc + acc : acc;
+    return (fl & 1u) ? acc + acc : acc;
   }
+  __device__ void side(int, double, double, unsigned) const {}
 };
 struct GsFin {
-  const double *ht, *hp;
-  const int* sill;
+  const double* __restrict__ ht;
+  const double* __restrict__ hp;
+  const int* __restrict__ sill;
   double* lsed;
-  __device__ double base(int k) const { return ht[k] - hp[k]; }
-  __device__ double finish(int k, double acc, bool root) const {
-    if (root) { lsed[k] = acc; return acc; }
-    const double e = ht[k] - hp[k];
+  static constexpr bool kAux = true;
+  __device__ double base(int k) const { return __ldg(&ht[k]) - __ldg(&hp[k]); }
+  __device__ double aux(int k) const { return base(k); }
+  __device__ unsigned prop(int k) const { return __ldg(&sill[k]) == k ? 2u : 0u; }
+  __device__ double value(double acc, double e, unsigned fl) const {
+    if (fl & 1u) return acc;
     const double t = acc - e;
-    if (sill[k] == k) lsed[k] = t <= 0.0 ? 0.0 : t;
     return t + e;
+  }
+  __device__ void side(int k, double acc, double e, unsigned fl) const {
+    if (fl & 1u) {
+      lsed[k] = acc;
+    } else if (fl & 2u) {
+      const double t = acc - e;
+      lsed[k] = t <= 0.0 ? 0.0 : t;
+    }
   }
 };
 struct VolFin {
-  const int* sill;
-  const double* contrib;
+  const int* __restrict__ sill;
+  const double* __restrict__ contrib;
   double* vol;
+  static constexpr bool kAux = true;
   __device__ double base(int) const { return 0.0; }
-  __device__ double finish(int k, double acc, bool root) const {
-    vol[k] = acc;
-    return (!root && sill[k] != k) ? contrib[k] + acc : 0.0;
+  __device__ double aux(int k) const { return __ldg(&contrib[k]); }
+  __device__ unsigned prop(int k) const { return __ldg(&sill[k]) != k ? 2u : 0u; }
+  __device__ double value(double acc, double cb, unsigned fl) const { return fl == 2u ? cb + acc : 0.0; }
+  __device__ void side(int k, double acc, double, unsigned) const { vol[k] = acc; }
+};
+
+// A node's donors: the sum down to the heavy one (descending) and the lighter
+// values that follow it.
+struct Gather {
+  double first;    // base and the donors above the heavy child
+  double rest[7];  // the donors below it, in order
+  int nrest;
+  // false while a value has not arrived
+  __device__ __forceinline__ bool take(int k, int nd, int heavy, double base, const int* __restrict__ don,
+                                       const double* a) {
+    first = base;
+    nrest = 0;
+    if (nd < 2) return true;
+    const int4* row = reinterpret_cast<const int4*>(don + (size_t)k * 8);
+    const int4 x = __ldg(row), y = __ldg(row + 1);
+    const int d[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+    double v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (i < nd && d[i] != heavy) v[i] = ld_relaxed_gpu(&a[d[i]]);
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (i < nd && d[i] != heavy) ok &= arrived(v[i]);
+    if (!ok) return false;
+    bool below = false;
+#pragma unroll
+    for (int i = 7; i >= 0; --i)
+      if (i < nd) {
+        if (d[i] == heavy) {
+          below = true;
+        } else if (!below) {
+          first = first + v[i];
+        } else {
+#pragma unroll
+          for (int t = 0; t < 7; ++t)
+            if (t == nrest) rest[t] = v[i];
+          ++nrest;
+        }
+      }
+    return true;
   }
 };
 
 template <class Fin>
-__global__ void __launch_bounds__(128) k_area_chains(ChainView cv, const int* __restrict__ rec,
-                                                     const int* __restrict__ ndon, const int* __restrict__ don,
-                                                     Fin fin, double* __restrict__ a, unsigned* ticket,
-                                                     unsigned* done, unsigned epoch, int* err) {
-  const int lane = threadIdx.x & 31;
-  for (;;) {
-    // one chain per warp, walked by lane 0: a bottom-up walk waits at every
-    // junction whose light donor is not done, and lanes of one warp waiting
-    // (with back-off) at different junctions slowed each other's walks
-    // (1023^2 single flow: 8.7 -> 5.4 ms with one chain per warp)
-    unsigned w = 0;
-    if (lane == 0) w = atomicAdd(ticket, 1u);
-    w = __shfl_sync(FULL, w, 0);
-    if ((int)w >= cv.ntickets) break;
-    const int c = lane == 0 ? cv.tickets[(int)w] : -1;
-    if (c < 0) continue;
-    int s, e;
-    cv.range(c, s, e);
-    int child = -1;
-    double ac = 0.0;
-    for (int hi = e; hi > s; hi -= kCF) {
-      const int n = min(kCF, hi - s);
-      const int lo = hi - n;
-      int kk[kCF], nd[kCF];
-      double base[kCF];
-#pragma unroll
-      for (int i = 0; i < kCF; ++i) if (i < n) kk[i] = cv.ord[lo + i];
-#pragma unroll
-      for (int i = 0; i < kCF; ++i) if (i < n) {
-        nd[i] = ndon[kk[i]];
-        base[i] = fin.base(kk[i]);
-        if (rec[kk[i]] == kk[i]) nd[i] |= 1 << 8;
-      }
-      // Only nodes with two or more donors have light donors (a node's only
-      // donor is its heavy child, the next node down the chain); their donor
-      // rows are prefetched together before the listing reads them.
-#pragma unroll
-      for (int i = 0; i < kCF; ++i)
-        if (i < n && (nd[i] & 255) >= 2) prefetch_l1(&don[(size_t)kk[i] * 8]);
-      // light donors of the chunk in processing order (i descending, q descending);
-      // the heavy child of kk[i] is the next node down the chain
-      int lid[kLight];
-      double lv[kLight];
-      int nl = 0;
-      for (int i = n - 1; i >= 0; --i) {
-        const int k = kk[i];
-        const int heavy = i + 1 < n ? kk[i + 1] : child;
-        if ((nd[i] & 255) < 2) continue;
-        for (int q = (nd[i] & 255) - 1; q >= 0; --q) {
-          const int d = don[(size_t)k * 8 + q];
-          if (d != heavy && nl < kLight) lid[nl++] = d;
+__global__ void __launch_bounds__(kSweepThreads) k_bottom_up(ChainView cv, const int* __restrict__ rec,
+                                                             const int* __restrict__ ndon,
+                                                             const int* __restrict__ don, Fin fin, double* a) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp < kSoloWarps) {
+    const int total = cv.totals[0];
+    for (;;) {
+      unsigned t = 0;
+      if (lane == 0) t = atomicAdd(&cv.ticket[0], 1u);
+      t = __shfl_sync(FULL, t, 0);
+      if ((int)t >= total) return;
+      const int4 tk = cv.tk_long[t];
+      const int s = tk.x, e = tk.y;
+      double ac = 0.0;
+      // lane i of a chunk holds position hi - 1 - i; its heavy child is the position after
+      int k = e - 1 - lane >= s ? cv.ord[e - 1 - lane] : -1;
+      for (int hi = e; hi > s; hi -= 32) {
+        const int n = min(32, hi - s);
+        const int k2 = hi - 33 - lane >= s ? cv.ord[hi - 33 - lane] : -1;
+        int heavy = __shfl_up_sync(FULL, k, 1);
+        if (lane == 0) heavy = hi < e ? cv.ord[hi] : -1;
+        double base = 0.0, aux = 0.0;
+        int nd = 0;
+        unsigned fl = 0;
+        if (k >= 0) {
+          nd = ndon[k];
+          base = fin.base(k);
+          if (Fin::kAux) aux = fin.aux(k);
+          fl = (rec[k] == k ? 1u : 0u) | fin.prop(k);
         }
-      }
-      if (nl) {
-        bool ready = true;
-        for (int j = 0; j < nl; ++j) ready &= *(volatile unsigned*)&done[lid[j]] == epoch;
-        if (!ready)
-          for (int j = 0; j < nl; ++j) wait_flag(done, lid[j], epoch, err);
-        fence_acq_rel();
-        for (int j = 0; j < nl; ++j) lv[j] = __ldcg(&a[lid[j]]);
-      }
-      int jl = 0;
-#pragma unroll
-      for (int i = kCF - 1; i >= 0; --i) if (i < n) {
-        const int k = kk[i];
-        const int ndk = nd[i] & 255;
-        double acc = base[i];
-        if (ndk == 1) acc = acc + ac;  // the heavy child alone
-        else for (int q = ndk - 1; q >= 0; --q) {
-          const int d = don[(size_t)k * 8 + q];
-          double v;
-          if (d == child) v = ac;
-          else if (jl < kLight) v = lv[jl++];
-          else {  // more light donors than one fetch holds: read this one on its own
-            wait_flag(done, d, epoch, err);
-            v = __ldcg(&a[d]);
+        Gather g;
+        bool ready = k < 0 || g.take(k, nd, heavy, base, don, a);
+        const bool inner = heavy >= 0;  // the chain's leaf has no child
+        double acc_own = 0.0;
+        int i = 0;
+        Patience pat;
+        while (i < n) {
+          const unsigned rb = __ballot_sync(FULL, ready);
+          const int upto = min(n, __ffs(~rb) ? __ffs(~rb) - 1 : 32);
+          if (i >= upto) {  // the next node's donors are not all there
+            if (__any_sync(FULL, pat.over(cv.err))) return;
+            if (pat.spins > 4) pat.rest();
+            if (!ready) ready = g.take(k, nd, heavy, base, don, a);
+            continue;
           }
-          acc = acc + v;
-        }
-        acc = fin.finish(k, acc, (nd[i] >> 8) != 0);
-        a[k] = acc;
-        ac = acc;
-        child = k;
-      }
-    }
-    fence_acq_rel();
-    *(volatile unsigned*)&done[cv.ord[s]] = epoch;
-  }
-}
-
-// CopyChi (FastScape_ctx.f90:228-251) top down: chi(k) = chi(rec(k)) +
-// (a0/a(k))^(m/n) * length(k) where a(k) > a0, else 0; a root starts from 0.
-__global__ void __launch_bounds__(128) k_chi_chains(ChainView cv, const int* __restrict__ rec,
-                                                    const int* __restrict__ ndon, const double* __restrict__ a,
-                                                    const double* __restrict__ length, double a0, double mn,
-                                                    double* __restrict__ chi, unsigned* ticket, unsigned* done,
-                                                    unsigned epoch, int* err) {
-  const int lane = threadIdx.x & 31;
-  for (;;) {
-    unsigned w = 0;
-    if (lane == 0) w = atomicAdd(ticket, 32u);
-    w = __shfl_sync(FULL, w, 0);
-    if ((int)w >= cv.ntickets) break;
-    const int t = (int)w + lane;
-    const int c = t < cv.ntickets ? cv.tickets[t] : -1;
-    if (c < 0) continue;
-    int s, e;
-    cv.range(c, s, e);
-    const int k0 = cv.ord[s];
-    const int r0 = rec[k0];
-    double prev = 0.0;
-    if (r0 != k0) {
-      wait_flag(done, r0, epoch, err);
-      prev = __ldcg(&chi[r0]);
-    }
-    for (int p = s; p < e; p += kCF) {
-      const int n = min(kCF, e - p);
-      int kk[kCF], nd[kCF];
-      double term[kCF], aa[kCF], out[kCF];
+          for (; i < upto; ++i) {
+            double acc = __shfl_sync(FULL, g.first, i);
+            if (__shfl_sync(FULL, (int)inner, i)) acc = acc + ac;
+            const int nr = __shfl_sync(FULL, g.nrest, i);
 #pragma unroll
-      for (int i = 0; i < kCF; ++i) if (i < n) kk[i] = cv.ord[p + i];
-#pragma unroll
-      for (int i = 0; i < kCF; ++i) if (i < n) {
-        aa[i] = a[kk[i]];
-        nd[i] = ndon[kk[i]];
-        term[i] = pow(a0 / aa[i], mn) * length[kk[i]];
-      }
-#pragma unroll
-      for (int i = 0; i < kCF; ++i) if (i < n) {
-        const double v = aa[i] > a0 ? prev + term[i] : 0.0;
-        out[i] = v;
-        prev = v;
-      }
-#pragma unroll
-      for (int i = 0; i < kCF; ++i) if (i < n) chi[kk[i]] = out[i];
-      fence_acq_rel();
-#pragma unroll
-      for (int i = 0; i < kCF; ++i) if (i < n && nd[i] > 1) *(volatile unsigned*)&done[kk[i]] = epoch;
-    }
-  }
-}
-
-// Top-down single-flow stream power law with g == 0 (StreamPowerLaw.f90:291-373):
-// writes hnew and water; h keeps ht.  The per-node factor kf*dt*a^m/l(^n)
-// does not depend on the recurrence and is computed for a whole chunk first.
-// With GS (a Gauss-Seidel iteration of the g > 0 solve, StreamPowerLaw.f90:285-373)
-// the deposition-corrected surface comes from `elev`, Newton starts from the
-// current iterate `hstart`, and the lake bookkeeping is written: sill(k) = k
-// for a node above its receiver's water, else sill(rec) with its volume
-// contribution w_rcv - h(k) in contrib(k).  Without GS, elev = hstart = ht.
-struct GsIo {
-  const double* elev;
-  const double* hstart;
-  int* sill;
-  double* contrib;
-};
-
-template <bool GS>
-__global__ void __launch_bounds__(128) k_spl_chains(ChainView cv, const int* __restrict__ rec,
-                                                    const int* __restrict__ ndon, const double* __restrict__ h,
-                                                    const double* __restrict__ b, const double* __restrict__ kf,
-                                                    const double* __restrict__ a, const double* __restrict__ length,
-                                                    double kfsed, double dt, double m, double n, double omega,
-                                                    int n_is_one, double* __restrict__ hnew,
-                                                    double* __restrict__ water, GsIo gs, unsigned* ticket,
-                                                    unsigned* done, unsigned epoch, int* err) {
-  const int lane = threadIdx.x & 31;
-  for (;;) {
-    unsigned w = 0;
-    if (lane == 0) w = atomicAdd(ticket, 32u);
-    w = __shfl_sync(FULL, w, 0);
-    if ((int)w >= cv.ntickets) break;
-    const int t = (int)w + lane;
-    const int c = t < cv.ntickets ? cv.tickets[t] : -1;
-    if (c < 0) continue;
-    int s, e;
-    cv.range(c, s, e);
-    const int k0 = cv.ord[s];
-    const int r0 = rec[k0];
-    bool root = r0 == k0;
-    double hr = 0.0, wr = 0.0, htr = 0.0;
-    int sr = 0;
-    if (!root) {
-      wait_flag(done, r0, epoch, err);
-      hr = __ldcg(&hnew[r0]);
-      wr = __ldcg(&water[r0]);
-      htr = h[r0];
-      if (GS) sr = __ldcg(&gs.sill[r0]);
-    }
-    for (int p = s; p < e; p += kCS) {
-      const int cn = min(kCS, e - p);
-      int kk[kCS], nd[kCS], so[kCS];
-      double ht[kCS], fact[kCS], ho[kCS], wo[kCS], el[kCS], h0[kCS], co[kCS];
-#pragma unroll
-      for (int i = 0; i < kCS; ++i) if (i < cn) kk[i] = cv.ord[p + i];
-#pragma unroll
-      for (int i = 0; i < kCS; ++i) if (i < cn) {
-        const int k = kk[i];
-        ht[i] = h[k];
-        el[i] = GS ? gs.elev[k] : ht[i];
-        h0[i] = GS ? gs.hstart[k] : ht[i];
-        nd[i] = ndon[k];
-        const double kfint = (kfsed > 0.0 && (ht[i] - b[k]) > 1.0) ? kfsed : kf[k];
-        const double l = length[k];
-        fact[i] = n_is_one ? kfint * dt * pow(a[k], m) / l : kfint * dt * pow(a[k], m) / pow(l, n);
-      }
-#pragma unroll
-      for (int i = 0; i < kCS; ++i) if (i < cn) {
-        double hk = ht[i], wk;
-        int sk = kk[i];
-        double ck = 0.0;
-        if (root) {
-          wk = ht[i];
-          root = false;
-        } else {
-          const double elev = el[i];
-          hk = h0[i];
-          if (elev > wr) {
-            if (n_is_one) {
-              double f = elev, df = 1.0;
-              f = f + fact[i] * hr;
-              df = df + fact[i];
-              hk = f / df;
-            } else {
-              const double tolp = 1.0e-3;
-              double errp = 2.0 * tolp;
-              int guard = 0;
-              while (errp > tolp) {
-                if (++guard > kNewtonLimit) {
-                  atomicExch(err, DEV_NEWTON_LIMIT);
-                  break;
-                }
-                double f = hk - elev, df = 1.0;
-                if (ht[i] > htr) {
-                  const double x = fmax(0.0, hk - hr);
-                  double pn, pn1;
-                  if (n == 1.5) {  // x^1.5 = x*sqrt(x), x^0.5 = sqrt(x)
-                    pn1 = sqrt(x);
-                    pn = x * pn1;
-                  } else if (x > 0.0) {  // one pow: x^n = x * x^(n-1)
-                    pn1 = pow(x, n - 1.0);
-                    pn = x * pn1;
-                  } else {
-                    pn = pow(x, n);
-                    pn1 = pow(x, n - 1.0);
-                  }
-                  f = f + fact[i] * pn;
-                  df = df + fact[i] * n * pn1;
-                }
-                const double hn = hk - f / df;
-                errp = fabs(hn - hk);
-                hk = hk * (1.0 - omega) + hn * omega;
-              }
+            for (int u = 0; u < 7; ++u) {
+              if (u >= nr) break;
+              acc = acc + __shfl_sync(FULL, g.rest[u], i);
             }
-            if (hk < wr) hk = wr;
-          } else {
-            hk = elev;
-            sk = sr;
-            ck = wr - hk;
+            const double ax = Fin::kAux ? __shfl_sync(FULL, aux, i) : 0.0;
+            ac = fin.value(acc, ax, __shfl_sync(FULL, fl, i));
+            if (lane == i) {
+              acc_own = acc;
+              st_relaxed_gpu(&a[k], publishable(ac));
+            }
           }
-          wk = fmax(wr, hk);
         }
-        ho[i] = hk;
-        wo[i] = wk;
-        so[i] = sk;
-        co[i] = ck;
-        hr = hk;
-        wr = wk;
-        htr = ht[i];
-        sr = sk;
+        if (k >= 0) fin.side(k, acc_own, aux, fl);
+        k = k2;
       }
-#pragma unroll
-      for (int i = 0; i < kCS; ++i) if (i < cn) {
-        hnew[kk[i]] = ho[i];
-        water[kk[i]] = wo[i];
-        if (GS) { gs.sill[kk[i]] = so[i]; gs.contrib[kk[i]] = co[i]; }
-      }
-      fence_acq_rel();
-#pragma unroll
-      for (int i = 0; i < kCS; ++i) if (i < cn && nd[i] > 1) *(volatile unsigned*)&done[kk[i]] = epoch;
     }
   }
+  const int total = cv.totals[1];
+  int4 tk = make_int4(0, 0, 0, 0);
+  int status = 0;  // 0 without a chain, 2 walking, 3 no chain left
+  int child = -1;
+  double ac = 0.0;
+  Patience pat;
+  for (;;) {
+    const unsigned idle = __ballot_sync(FULL, status == 0);
+    if (idle) {
+      unsigned t = 0;
+      if (lane == 0) t = atomicAdd(&cv.ticket[1], (unsigned)__popc(idle));
+      t = __shfl_sync(FULL, t, 0) + __popc(idle & ((1u << lane) - 1u));
+      if (status == 0) {
+        if ((int)t < total) {
+          tk = cv.tk_short[t];
+          status = 2;
+          child = -1;
+        } else {
+          status = 3;
+        }
+      }
+    }
+    if (!__any_sync(FULL, status != 3)) return;
+    bool moved = false;
+    if (status == 2) {
+      const int k = cv.ord[tk.y - 1];
+      const int nd = ndon[k];
+      Gather g;
+      if (g.take(k, nd, child, fin.base(k), don, a)) {
+        double acc = g.first;
+        if (child >= 0) acc = acc + ac;
+#pragma unroll
+        for (int u = 0; u < 7; ++u)
+          if (u < g.nrest) acc = acc + g.rest[u];
+        const double ax = Fin::kAux ? fin.aux(k) : 0.0;
+        const unsigned fl = (rec[k] == k ? 1u : 0u) | fin.prop(k);
+        ac = fin.value(acc, ax, fl);
+        fin.side(k, acc, ax, fl);
+        st_relaxed_gpu(&a[k], publishable(ac));
+        child = k;
+        moved = true;
+        if (--tk.y <= tk.x) status = 0;
+      }
+    }
+    if (!__any_sync(FULL, moved)) {
+      if (__any_sync(FULL, pat.over(cv.err))) return;
+      pat.rest();
+    } else {
+      pat = Patience{};
+    }
+  }
+}
+
+// chains of one node, before the others
+template <class Fin>
+__global__ void k_bottom_up_leaves(int nn, const int* __restrict__ rec, const int* __restrict__ ndon,
+                                   const unsigned char* __restrict__ head, Fin fin, double* __restrict__ a) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
+    if (ndon[k] != 0 || !head[k]) continue;
+    const double acc = fin.base(k), ax = Fin::kAux ? fin.aux(k) : 0.0;
+    const unsigned fl = (rec[k] == k ? 1u : 0u) | fin.prop(k);
+    fin.side(k, acc, ax, fl);
+    a[k] = publishable(fin.value(acc, ax, fl));
+  }
+}
+
+template <class U>
+void path_sums(Ctx& c, U* marks, U* scan) {
+  const int nn = c.nn;
+  cudaStream_t st = c.stream;
+  cudaMemsetAsync(marks, 0, sizeof(U) * ((size_t)nn + 1), st);
+  k_path_marks<U><<<grid1d(nn), kBlock, 0, st>>>(nn, c.rec, c.ndon, c.don, c.pos, c.size, marks, c.ch_head, c.d_err);
+  if constexpr (sizeof(U) == 4) exclusive_scan_u32(c, marks, scan, (size_t)nn + 1);
+  else exclusive_scan_u64(c, marks, scan, (size_t)nn + 1);
+  k_hf_order<U><<<grid1d(nn), kBlock, 0, st>>>(nn, scan, c.pos, c.ch_head, c.ch_ord, c.ch_flag, c.ch_depth, c.d_err);
+  c.count_launch(2);
 }
 
 }  // namespace
 
-// Builds the heavy-first order and both ticket lists for the current
-// receiver forest (rec, ndon, don, size, roots must be current).
+// Builds the heavy-first order and both ticket lists for the current receiver
+// forest (rec, ndon, don, stack positions and sizes must be current).
 void build_chains(Ctx& c) {
   const int nn = c.nn;
   cudaStream_t st = c.stream;
-  k_heavy<<<grid1d(nn), kBlock, 0, st>>>(nn, c.ndon, c.don, c.size, c.ch_heavy);
-  cudaMemcpyAsync(c.d_cnt + 15, c.s_scan + nn, sizeof(int), cudaMemcpyDeviceToDevice, st);
-  fetch_counters(c, 20);
-  c.nroots = c.h_cnt[15];
-  const int nroots_h = c.nroots;
-  k_root_sizes<<<grid1d(nroots_h + 1), kBlock, 0, st>>>(nroots_h, c.s_roots, c.size, c.ch_tmp);
-  c.count_launch(2);
-  exclusive_scan_int(c, c.ch_tmp, c.ch_tmp2, nroots_h + 1);
-  k_hf_offsets<<<grid1d(nn), kBlock, 0, st>>>(nn, c.rec, c.ndon, c.don, c.size, c.ch_heavy, c.s_root_rank,
-                                              c.ch_tmp2, c.ch_val, c.ch_nxt);
-  c.count_launch();
-  unsigned long long *va = c.ch_val, *vb = c.ch_val2;
-  if ((size_t)nn < ((size_t)1 << kPathOffBits)) {
-    // a scan over the DFS preorder of the current forest (pos, size)
-    unsigned* marks = reinterpret_cast<unsigned*>(c.ch_tmp);
-    unsigned* scan = reinterpret_cast<unsigned*>(c.ch_tmp2);
-    cudaMemsetAsync(marks, 0, sizeof(unsigned) * (nn + 1), st);
-    k_path_marks<<<grid1d(nn), kBlock, 0, st>>>(nn, va, c.pos, c.size, marks, c.d_err);
-    c.count_launch();
-    exclusive_scan_u32(c, marks, scan, nn + 1);
-    k_path_take<<<grid1d(nn), kBlock, 0, st>>>(nn, c.pos, scan, vb);
-    c.count_launch();
-    std::swap(va, vb);
-  } else {
-    int *na = c.ch_nxt, *nb = c.ch_nxt2;
-    // pointer jumping; the flag read back every 4 rounds says whether any
-    // pointer moved in them (rounds after convergence change nothing)
-    for (int round = 0; round < 20; ++round) {
-      cudaMemsetAsync(c.d_cnt + 16, 0, sizeof(int), st);
-      for (int r = 0; r < 4; ++r) {
-        k_path_jump<<<grid1d(nn), kBlock, 0, st>>>(nn, va, na, vb, nb, c.d_cnt + 16);
-        std::swap(va, vb);
-        std::swap(na, nb);
-      }
-      c.count_launch(4);
-      fetch_counters(c, 20);
-      if (!c.h_cnt[16]) break;
-    }
-  }
-  k_hf_order<<<grid1d(nn), kBlock, 0, st>>>(nn, va, c.rec, c.ch_heavy, c.ch_ord, c.ch_pos, c.ch_ldep, c.d_err);
-  k_chain_flags<<<grid1d(nn + 1), kBlock, 0, st>>>(nn, c.ch_ord, c.rec, c.ch_heavy, c.ch_tmp);
-  c.count_launch(2);
-  exclusive_scan_int(c, c.ch_tmp, c.ch_tmp2, nn + 1);
-  cudaMemcpyAsync(c.d_cnt + 17, c.ch_tmp2 + nn, sizeof(int), cudaMemcpyDeviceToDevice, st);
-  fetch_counters(c, 20);
-  const int nchains = c.h_cnt[17];
-  c.nchains = nchains;
-  k_chain_list<<<grid1d(nn), kBlock, 0, st>>>(nn, c.ch_tmp, c.ch_tmp2, c.ch_start, c.ch_cid);
-  cudaMemsetAsync(c.ch_hist, 0, sizeof(int) * 128, st);
-  k_chain_keys<<<grid1d(nchains), kBlock, 0, st>>>(nn, nchains, c.ch_start, c.ch_ord, c.ch_ldep, c.ch_key,
-                                                   c.ch_key + nchains, c.ch_hist, c.ch_hist + 64);
-  c.count_launch(2);
-  for (int dir = 0; dir < 2; ++dir) {
-    sort_pairs_u32(c, c.ch_key + (size_t)dir * nchains, c.ch_skey, c.ch_cid, c.ch_sid, nchains, 32);
-    k_group_offsets<<<1, 1, 0, st>>>(c.ch_hist + 64 * dir, c.ch_goff, c.ch_goff + 64, c.d_cnt + 18 + dir);
-    int* tk = dir == 0 ? c.ch_tk_td : c.ch_tk_bu;
-    cudaMemsetAsync(tk, 0xff, sizeof(int) * ((size_t)nchains + 64 * 32), st);
-    k_ticket_scatter<<<grid1d(nchains), kBlock, 0, st>>>(nchains, c.ch_skey, c.ch_sid, c.ch_goff, c.ch_goff + 64, tk);
-    c.count_launch(2);
-  }
-  fetch_counters(c, 20);
-  c.ntickets_td = c.h_cnt[18];
-  c.ntickets_bu = c.h_cnt[19];
+  if (nn < 1 << 27) path_sums(c, reinterpret_cast<unsigned*>(c.ch_val), reinterpret_cast<unsigned*>(c.ch_val2));
+  else path_sums(c, c.ch_val, c.ch_val2);
+  int* scan = reinterpret_cast<int*>(c.ch_val);
+  exclusive_scan_int(c, c.ch_flag, scan, (size_t)nn + 1);
+  const int* nchains = scan + nn;
+  k_chain_list<<<grid1d(nn), kBlock, 0, st>>>(nn, c.ch_flag, scan, c.ch_start);
+  int *hist = c.ch_hist, *cur_td = hist + kHist, *cur_bu = cur_td + kHist;
+  cudaMemsetAsync(hist, 0, sizeof(int) * kHist, st);
+  const unsigned blocks = (unsigned)((nn + kChainsPerBlock - 1) / kChainsPerBlock);
+  k_chain_hist<<<blocks, kChainBlock, 0, st>>>(nn, nchains, c.ch_start, c.ch_depth, hist);
+  k_chain_offsets<<<1, kBuckets, 0, st>>>(hist, cur_td, cur_bu, c.ch_totals);
+  k_chain_tickets<<<blocks, kChainBlock, 0, st>>>(nn, nchains, c.ch_start, c.ch_depth, c.ch_ord, c.rec, cur_td, cur_bu,
+                                                  c.ch_tk[0], c.ch_tk[1], c.ch_tk[2], c.ch_tk[3]);
+  c.count_launch(4);
 }
 
 void ensure_chains(Ctx& c) {
@@ -728,109 +880,85 @@ void ensure_chains(Ctx& c) {
   }
 }
 
-static void next_epoch(Ctx& c) {
-  c.epoch += 1;
-  if (c.epoch == 0) {
-    cudaMemsetAsync(c.done, 0, sizeof(unsigned) * c.nn, c.stream);
-    c.epoch = 1;
-  }
-  cudaMemsetAsync(c.ticket, 0, sizeof(unsigned), c.stream);
+// Blocks of a chain sweep: one per 512 nodes up to 4 per SM; a quarter of that
+// beside other instances (fsb_set_concurrency), whose kernels need the SMs that
+// waiting blocks would hold.
+static int sweep_blocks(const Ctx& c) {
+  const int want = c.nn / (512 * c.launch_share) + 1;
+  return std::min(want, 148 * 4);
 }
 
-// Persistent chain sweeps: up to 8 blocks per SM, and one block per 4096
-// tickets below that.  Most chains of a sweep wait for others, so a few
-// threads per thousand chains keep the critical path busy (at 2049^2 the
-// sweeps take the same time as with one thread per chain), and the sweeps of
-// small and mid-size grids leave the GPU to other streams.
-#ifndef FSB_CHAIN_TICKETS_PER_BLOCK
-#define FSB_CHAIN_TICKETS_PER_BLOCK 4096
-#endif
-// bottom-up sweeps take one chain per warp: one block per 512 tickets.  An
-// instance that shares the device with others (fsb_set_concurrency) takes a
-// quarter of the blocks: the persistent blocks of each instance hold SMs
-// while they wait, and fewer of them let more instances run at once (256
-// uneven single-flow grids on 32 workers: 3.22e8 -> 3.8e8 node-steps/s).
-static int chain_blocks_bu(const Ctx& c, int ntickets) {
-  const int per = 512 * c.launch_share;
-  const int want = (ntickets + per - 1) / per;
-  return want < 1 ? 1 : (want > 148 * 8 ? 148 * 8 : want);
+static ChainView chain_view(Ctx& c, bool top_down) {
+  cudaMemsetAsync(c.ticket, 0, 2 * sizeof(unsigned), c.stream);
+  return ChainView{c.ch_ord, c.ch_tk[top_down ? 0 : 2], c.ch_tk[top_down ? 1 : 3], c.ch_totals, c.ticket, c.d_err};
 }
 
-static int chain_blocks(const Ctx& c, int ntickets) {
-  const int per = FSB_CHAIN_TICKETS_PER_BLOCK * c.launch_share;
-  const int want = (ntickets + per - 1) / per;
-  return want < 1 ? 1 : (want > 148 * 8 ? 148 * 8 : want);
+template <class Op>
+static void top_down(Ctx& c, const Op& op) {
+  const ChainView cv = chain_view(c, true);
+  k_top_down<Op><<<sweep_blocks(c), kSweepThreads, 0, c.stream>>>(cv, op);
+  k_top_down_leaves<Op><<<grid1d(c.nn), kBlock, 0, c.stream>>>(c.nn, c.rec, c.ndon, c.ch_head, op, c.d_err);
+  c.count_launch(2);
+}
+
+template <class Fin>
+static void bottom_up(Ctx& c, const Fin& fin, double* a) {
+  cudaMemsetAsync(a, 0xff, sizeof(double) * c.nn, c.stream);
+  const ChainView cv = chain_view(c, false);
+  k_bottom_up_leaves<Fin><<<grid1d(c.nn), kBlock, 0, c.stream>>>(c.nn, c.rec, c.ndon, c.ch_head, fin, a);
+  k_bottom_up<Fin><<<sweep_blocks(c), kSweepThreads, 0, c.stream>>>(cv, c.rec, c.ndon, c.don, fin, a);
+  c.count_launch(2);
 }
 
 void fill_chains(Ctx& c) {
-  next_epoch(c);
-  ChainView cv{c.ch_ord, c.ch_start, c.ch_tk_td, c.nchains, c.ntickets_td, c.nn};
   stage_begin(c, KT_FILL);
-  k_fill_chains<<<chain_blocks(c, cv.ntickets), 128, 0, c.stream>>>(cv, c.rec, c.ndon, c.h, c.hwater, c.lake_depth, c.ticket,
-                                                    c.done, c.epoch, c.d_err);
+  cudaMemsetAsync(c.hwater, 0xff, sizeof(double) * c.nn, c.stream);
+  top_down(c, FillOp{c.h, c.hwater, c.lake_depth});
   stage_end(c, KT_FILL);
-  c.count_launch();
 }
 
-void area_chains(Ctx& c) {
-  next_epoch(c);
-  ChainView cv{c.ch_ord, c.ch_start, c.ch_tk_bu, c.nchains, c.ntickets_bu, c.nn};
-  k_area_chains<<<chain_blocks_bu(c, cv.ntickets), 128, 0, c.stream>>>(cv, c.rec, c.ndon, c.don,
-                                                                 AreaFin{c.precip, c.dx * c.dy}, c.a, c.ticket,
-                                                                 c.done, c.epoch, c.d_err);
-  c.count_launch();
-}
+void area_chains(Ctx& c) { bottom_up(c, AreaFin{c.precip, c.dx * c.dy}, c.a); }
 
-void flux_chains(Ctx& c, double* flux) {
-  next_epoch(c);
-  ChainView cv{c.ch_ord, c.ch_start, c.ch_tk_bu, c.nchains, c.ntickets_bu, c.nn};
-  k_area_chains<<<chain_blocks_bu(c, cv.ntickets), 128, 0, c.stream>>>(cv, c.rec, c.ndon, c.don, FluxFin{c.erate}, flux,
-                                                                 c.ticket, c.done, c.epoch, c.d_err);
-  c.count_launch();
-}
+void flux_chains(Ctx& c, double* flux) { bottom_up(c, FluxFin{c.erate}, flux); }
 
 void chi_chains(Ctx& c, double a0, double mn, double* chi) {
-  next_epoch(c);
-  ChainView cv{c.ch_ord, c.ch_start, c.ch_tk_td, c.nchains, c.ntickets_td, c.nn};
-  k_chi_chains<<<chain_blocks(c, cv.ntickets), 128, 0, c.stream>>>(cv, c.rec, c.ndon, c.a, c.length, a0, mn, chi, c.ticket,
-                                                                c.done, c.epoch, c.d_err);
-  c.count_launch();
+  cudaMemsetAsync(chi, 0xff, sizeof(double) * c.nn, c.stream);
+  top_down(c, ChiOp{c.a, c.length, a0, mn, chi});
 }
 
-void spl_chains(Ctx& c, double* hnew) {
-  next_epoch(c);
-  ChainView cv{c.ch_ord, c.ch_start, c.ch_tk_td, c.nchains, c.ntickets_td, c.nn};
-  const int n1 = fabs(c.n - 1.0) < 2.2250738585072014e-308;
-  k_spl_chains<false><<<chain_blocks(c, cv.ntickets), 128, 0, c.stream>>>(
-      cv, c.rec, c.ndon, c.h, c.b, c.kf, c.a, c.length, c.kfsed, c.dt, c.m, c.n, 0.875 / c.n, n1, hnew, c.water,
-      GsIo{nullptr, nullptr, nullptr, nullptr}, c.ticket, c.done, c.epoch, c.d_err);
-  c.count_launch();
+template <int MODE, bool GS>
+static void spl_mode(Ctx& c, const double* fact, double* hnew, const double* elev, const double* hstart, int* sill,
+                     double* contrib) {
+  top_down(c, SplOp<MODE, GS>{c.h, fact, c.n, 0.875 / c.n, hnew, c.water, elev, hstart, sill, contrib, c.d_err});
 }
+
+template <bool GS>
+static void spl_sweep(Ctx& c, double* hnew, const double* elev, const double* hstart, int* sill, double* contrib) {
+  const int n1 = fabs(c.n - 1.0) < 2.2250738585072014e-308;
+  double* fact = reinterpret_cast<double*>(c.ch_val2);
+  k_spl_factor<<<grid1d(c.nn), kBlock, 0, c.stream>>>(c.nn, n1, c.rec, c.h, c.b, c.kf, c.a, c.length, c.kfsed, c.dt,
+                                                      c.m, c.n, fact);
+  c.count_launch();
+  cudaMemsetAsync(hnew, 0xff, sizeof(double) * c.nn, c.stream);
+  cudaMemsetAsync(c.water, 0xff, sizeof(double) * c.nn, c.stream);
+  if (GS) cudaMemsetAsync(sill, 0xff, sizeof(int) * c.nn, c.stream);
+  if (n1) spl_mode<0, GS>(c, fact, hnew, elev, hstart, sill, contrib);
+  else if (c.n == 1.5) spl_mode<1, GS>(c, fact, hnew, elev, hstart, sill, contrib);
+  else spl_mode<2, GS>(c, fact, hnew, elev, hstart, sill, contrib);
+}
+
+void spl_chains(Ctx& c, double* hnew) { spl_sweep<false>(c, hnew, nullptr, nullptr, nullptr, nullptr); }
 
 void spl_chains_gs(Ctx& c, const double* elev, const double* hstart, double* hnew, int* sill, double* contrib) {
-  next_epoch(c);
-  ChainView cv{c.ch_ord, c.ch_start, c.ch_tk_td, c.nchains, c.ntickets_td, c.nn};
-  const int n1 = fabs(c.n - 1.0) < 2.2250738585072014e-308;
-  k_spl_chains<true><<<chain_blocks(c, cv.ntickets), 128, 0, c.stream>>>(
-      cv, c.rec, c.ndon, c.h, c.b, c.kf, c.a, c.length, c.kfsed, c.dt, c.m, c.n, 0.875 / c.n, n1, hnew, c.water,
-      GsIo{elev, hstart, sill, contrib}, c.ticket, c.done, c.epoch, c.d_err);
-  c.count_launch();
+  spl_sweep<true>(c, hnew, elev, hstart, sill, contrib);
 }
 
 void gs_erosion_chains(Ctx& c, const double* hp, const int* sill, double* lsed, double* dh) {
-  next_epoch(c);
-  ChainView cv{c.ch_ord, c.ch_start, c.ch_tk_bu, c.nchains, c.ntickets_bu, c.nn};
-  k_area_chains<<<chain_blocks_bu(c, cv.ntickets), 128, 0, c.stream>>>(cv, c.rec, c.ndon, c.don, GsFin{c.h, hp, sill, lsed},
-                                                                 dh, c.ticket, c.done, c.epoch, c.d_err);
-  c.count_launch();
+  bottom_up(c, GsFin{c.h, hp, sill, lsed}, dh);
 }
 
 void lake_volume_chains(Ctx& c, const int* sill, const double* contrib, double* vol, double* up) {
-  next_epoch(c);
-  ChainView cv{c.ch_ord, c.ch_start, c.ch_tk_bu, c.nchains, c.ntickets_bu, c.nn};
-  k_area_chains<<<chain_blocks_bu(c, cv.ntickets), 128, 0, c.stream>>>(cv, c.rec, c.ndon, c.don, VolFin{sill, contrib, vol},
-                                                                 up, c.ticket, c.done, c.epoch, c.d_err);
-  c.count_launch();
+  bottom_up(c, VolFin{sill, contrib, vol}, up);
 }
 
 }  // namespace fsb

@@ -79,6 +79,14 @@ __device__ __forceinline__ double ld_relaxed_gpu(const double* p) {
 __device__ __forceinline__ void st_relaxed_gpu(double* p, double v) {
   asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
 }
+__device__ __forceinline__ void st_relaxed_gpu(int* p, int v) {
+  asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+// Sweeps publish values in arrays that start as all ones, so that a value says
+// itself that it has arrived; a NaN of that pattern travels as another NaN.
+__device__ __forceinline__ double publishable(double v) {
+  return __double_as_longlong(v) == -1ll ? __longlong_as_double(0x7ff8000000000000ll) : v;
+}
 __device__ __forceinline__ int ld_relaxed_gpu(const int* p) {
   int v;
   asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");

@@ -37,6 +37,10 @@ struct TileMap {
   size_t queue_entries() const { return ((size_t)nctas * ns) << (2 * lt); }
 };
 
+// heavy-path chains (fsb_chains.cu): nodes of a long one; ticket buckets (32
+// light depths x 32 length classes of the long chains, 32 depths of the others)
+constexpr int kLongChain = 16, kChainHist = 32 * 32 + 32;
+
 struct Ctx {
   // ---- configuration (setters of FastScape_ctx.f90) ----
   int nx = 0, ny = 0, nn = 0;
@@ -122,12 +126,10 @@ struct Ctx {
   unsigned long long *o_keys = nullptr, *o_keys2 = nullptr;
   int *o_vals = nullptr, *o_vals2 = nullptr, *o_pos = nullptr;
   // heavy-path chain schedule (fsb_chains.cu)
-  int *ch_heavy = nullptr, *ch_tmp = nullptr, *ch_tmp2 = nullptr, *ch_nxt = nullptr, *ch_nxt2 = nullptr;
-  unsigned long long *ch_val = nullptr, *ch_val2 = nullptr;
-  int *ch_ord = nullptr, *ch_pos = nullptr, *ch_ldep = nullptr, *ch_start = nullptr, *ch_cid = nullptr,
-      *ch_sid = nullptr, *ch_hist = nullptr, *ch_goff = nullptr, *ch_tk_td = nullptr, *ch_tk_bu = nullptr;
-  unsigned *ch_key = nullptr, *ch_skey = nullptr;
-  int nchains = 0, ntickets_td = 0, ntickets_bu = 0, nroots = 0;
+  unsigned long long *ch_val = nullptr, *ch_val2 = nullptr;  // nn+1 each; scratch between the schedule's steps
+  int *ch_ord = nullptr, *ch_flag = nullptr, *ch_start = nullptr, *ch_hist = nullptr, *ch_totals = nullptr;
+  unsigned char *ch_head = nullptr, *ch_depth = nullptr;
+  int4* ch_tk[4] = {};  // tickets: top-down long, short; bottom-up long, short chains
   bool chains_valid = false;  // the chain schedule matches the current forest
   // last-arriver sweeps (multiple flow)
   int *la_queue = nullptr, *la_cnt = nullptr, *cnt_acc = nullptr, *cnt_spl = nullptr;
@@ -145,8 +147,6 @@ struct Ctx {
   unsigned* la_ctl = nullptr;  // head, tail, done count
   int* s_scan2 = nullptr;
   // sweeps
-  unsigned *done = nullptr;  // epoch flags per node
-  unsigned epoch = 0;
   unsigned* ticket = nullptr;
   double* water = nullptr;
   double* hnew = nullptr;  // elevation written by the stream-power sweep
@@ -200,6 +200,7 @@ inline size_t rank_splitter_cap(size_t n) { return (n + kRankStride - 1) / kRank
 // primitives (fsb_prims.cu)
 void exclusive_scan_int(Ctx& c, const int* in, int* out, size_t n);
 void exclusive_scan_u32(Ctx& c, const unsigned* in, unsigned* out, size_t n);
+void exclusive_scan_u64(Ctx& c, const unsigned long long* in, unsigned long long* out, size_t n);
 void inclusive_scan_int(Ctx& c, const int* in, int* out, size_t n);
 void sort_pairs_u32(Ctx& c, const unsigned* kin, unsigned* kout, const int* vin, int* vout, size_t n, int end_bit);
 void sort_pairs_u64(Ctx& c, const unsigned long long* kin, unsigned long long* kout, const int* vin,

@@ -22,6 +22,12 @@ void exclusive_scan_u32(Ctx& c, const unsigned* in, unsigned* out, size_t n) {
   c.count_launch(2);
 }
 
+void exclusive_scan_u64(Ctx& c, const unsigned long long* in, unsigned long long* out, size_t n) {
+  size_t bytes = c.cub_tmp_bytes;
+  cub::DeviceScan::ExclusiveSum(c.cub_tmp, bytes, in, out, (int)n, c.stream);
+  c.count_launch(2);
+}
+
 void inclusive_scan_int(Ctx& c, const int* in, int* out, size_t n) {
   size_t bytes = c.cub_tmp_bytes;
   cub::DeviceScan::InclusiveSum(c.cub_tmp, bytes, in, out, (int)n, c.stream);
@@ -50,6 +56,8 @@ size_t cub_temp_bytes_needed(size_t nn, size_t nconn) {
   cub::DeviceScan::InclusiveSum(nullptr, b, (const int*)nullptr, (int*)nullptr, (int)ns);
   mx = std::max(mx, b);
   cub::DeviceScan::ExclusiveSum(nullptr, b, (const unsigned*)nullptr, (unsigned*)nullptr, (int)ns);
+  mx = std::max(mx, b);
+  cub::DeviceScan::ExclusiveSum(nullptr, b, (const unsigned long long*)nullptr, (unsigned long long*)nullptr, (int)ns);
   mx = std::max(mx, b);
   cub::DeviceRadixSort::SortPairs(nullptr, b, (const unsigned*)nullptr, (unsigned*)nullptr,
                                   (const int*)nullptr, (int*)nullptr, (int)std::max(nconn, nn), 0, 32);

@@ -150,19 +150,15 @@ __device__ __forceinline__ bool mail_read(const double2* p, double2& v) {
   v.y = ld_relaxed_gpu(d + 1);
   return __double_as_longlong(v.x) != -1ll && __double_as_longlong(v.y) != -1ll;
 }
-// a NaN whose bits are all ones travels as another NaN
-__device__ __forceinline__ double mail_word(double v) {
-  return __double_as_longlong(v) == -1ll ? __longlong_as_double(0x7ff8000000000000ll) : v;
-}
-__device__ __forceinline__ void mail_write(double* p, double v) { st_relaxed_gpu(p, mail_word(v)); }
+__device__ __forceinline__ void mail_write(double* p, double v) { st_relaxed_gpu(p, publishable(v)); }
 __device__ __forceinline__ void mail_write(float* p, float v) {
   const int b = __float_as_int(v);
-  asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(b == -1 ? 0x7fc00000 : b) : "memory");
+  st_relaxed_gpu(reinterpret_cast<int*>(p), b == -1 ? 0x7fc00000 : b);
 }
 __device__ __forceinline__ void mail_write(double2* p, double2 v) {
   double* d = reinterpret_cast<double*>(p);
-  st_relaxed_gpu(d, mail_word(v.x));
-  st_relaxed_gpu(d + 1, mail_word(v.y));
+  st_relaxed_gpu(d, publishable(v.x));
+  st_relaxed_gpu(d + 1, publishable(v.y));
 }
 
 // The eight neighbours in the order of the reference's loops (jj outer, ii
