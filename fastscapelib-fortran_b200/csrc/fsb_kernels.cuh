@@ -4,6 +4,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdint>
 #include <cstddef>
 #include <string>
@@ -92,10 +93,10 @@ struct Ctx {
   // ---- scratch ----
   int *s_flag = nullptr, *s_scan = nullptr, *s_roots = nullptr, *s_root_rank = nullptr;
   unsigned long long *s_list_a = nullptr, *s_list_b = nullptr;  // 2*nn each
-  // list ranking by sublist walks: predecessor flags (2*nn bytes), the
-  // splitter lists (ping-pong) and the count of list heads
+  // list ranking by sublist walks: predecessor flags (2*nn bytes), the shorter
+  // lists and the count of list heads
   unsigned char* s_rank_pred = nullptr;
-  unsigned long long *s_rank_sa = nullptr, *s_rank_sb = nullptr;
+  unsigned long long* s_rank_ws = nullptr;
   unsigned* s_rank_nheads = nullptr;
   // LocalMinima
   size_t conn_cap = 0;       // capacity of edge arrays
@@ -177,6 +178,36 @@ struct Ctx {
   std::string err;
 };
 
+// Dynamic shared memory beyond 48 KB.  cudaFuncSetAttribute holds up the other
+// threads' launches (24 grids on 16 streams: 120 ms with three calls per
+// instance, 92 without), so each kernel asks once per device; a
+// refused launch asks again (the device's context may have been made anew).
+template <auto Kernel>
+struct BigSmem {
+  static inline std::atomic<unsigned long long> devices{0};
+  static bool allow(int bytes, bool again = false) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (!again && (devices.load(std::memory_order_relaxed) & bit)) return true;
+    if (cudaFuncSetAttribute((const void*)Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    devices.fetch_or(bit);
+    return true;
+  }
+  // launches Kernel with up to `most` bytes; false when the device refuses it
+  static bool launch(unsigned blocks, unsigned threads, size_t bytes, int most, cudaStream_t st, void** args) {
+    for (int t = 0; t < 2; ++t) {
+      if (!allow(most, t == 1)) return false;
+      if (cudaLaunchKernel((const void*)Kernel, dim3(blocks), dim3(threads), args, bytes, st) == cudaSuccess) return true;
+      cudaGetLastError();
+    }
+    return false;
+  }
+};
+
 // per-stage / per-kernel CUDA events while profiling is on (fsb_api.cu)
 enum { KT_AREA_SWEEP = 10, KT_SPL_SWEEP = 11, KT_THOMAS_ROWS = 12, KT_THOMAS_COLS = 13, KT_FILL = 14 };
 void stage_begin(Ctx& c, int s);
@@ -191,11 +222,19 @@ void launch_find_receiver(Ctx& c, const double* h, int* rec, double* length);
 void launch_find_donors(Ctx& c, const int* rec, int* ndon, int* don);
 void build_stack(Ctx& c, const int* rec, int* ndon, int* don, int* stack, int* pos, int* size);
 unsigned long long* list_rank(Ctx& c, size_t n, unsigned long long* a, unsigned long long* b);
-// list ranking by sublist walks: a splitter every kRankStride entries plus each
-// list head (at most kRankMaxHeads heads)
-constexpr int kRankStride = 16;
-constexpr int kRankMaxHeads = 64;
-inline size_t rank_splitter_cap(size_t n) { return (n + kRankStride - 1) / kRankStride + kRankMaxHeads; }
+// list ranking by sublist walks: a splitter every 16 or 4 entries plus each
+// list head (at most kRankMaxHeads heads); a block ranks up to kRankBlock entries
+constexpr int kRankMaxHeads = 64, kRankBlock = 8192;
+// scratch entries below a list of n: per level its splitters and their walk's results
+inline size_t rank_scratch(size_t n) {
+  size_t total = 0;
+  while (n > (size_t)kRankBlock) {
+    const size_t stride = n > 4 * ((size_t)kRankBlock - kRankMaxHeads) ? 16 : 4;
+    n = (n + stride - 1) / stride + kRankMaxHeads;
+    total += 2 * n;
+  }
+  return total + 2 * kRankBlock;  // a shorter list may take the finer stride and one level more
+}
 
 // primitives (fsb_prims.cu)
 void exclusive_scan_int(Ctx& c, const int* in, int* out, size_t n);

@@ -40,11 +40,12 @@ enum {
 };
 constexpr int kNrCounters = 15;  // counters the NR sort reads back
 
-// Segments of 8..kNrMedium elements leave the level-synchronous partition and
-// are finished each by one warp in shared memory (k_nr_medium): the last
-// levels of the sort, which hold only such segments, would otherwise each
-// cost a round of grid-wide barriers.
+// Segments of 8..kNrBlock elements leave the level-synchronous partition and
+// are finished each by one block in shared memory (k_nr_block), where a
+// barrier costs 40 ns instead of the several us of a grid-wide one.  kNrMedium
+// is the longest segment nr_sort_local takes.
 constexpr int kNrMedium = 512;
+constexpr int kNrBlock = 8192;
 
 // Level bound of the emulation: every level shrinks every segment by at least
 // its pivot, so n + 8 levels always suffice.  A fixed bound would not do: the
@@ -222,7 +223,7 @@ __global__ void k_conn_gather(int n, const int* __restrict__ perm, const int* __
 // idx[1..n] holds 1-based edge ids, arr[1..n] the weights (arr = w - 1).
 __global__ void k_nr_init(int n, int* __restrict__ idx, int* __restrict__ segof, int* __restrict__ seg,
                           int* __restrict__ small, int* __restrict__ med, int* __restrict__ cnt) {
-  const bool level = n > kNrMedium;  // else the whole array is one medium or small segment
+  const bool level = n > kNrBlock;  // else the whole array is one block's or one small segment
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q <= n + 1; q += gridDim.x * blockDim.x) {
     if (q >= 1 && q <= n) idx[q] = q;
     segof[q] = (q >= 1 && q <= n && level) ? 0 : -1;
@@ -336,20 +337,20 @@ __device__ inline int nr_apply_one(int q, const int* segof, const int* seg,
 }
 
 // children segments [l, j-1] and [i, ir]: partitioned at the next level when
-// they hold more than kNrMedium elements (counted in cnt[out_slot]), finished
-// in shared memory when they hold 8..kNrMedium (cnt[C_NMED]), insertion-sorted
+// they hold more than `limit` elements (counted in cnt[out_slot]), finished
+// in shared memory when they hold 8..limit (cnt[C_NMED]), insertion-sorted
 // when fewer (M = 7)
 // The children's ids go to child[4s..4s+3] (i, left id, right id, j); child
 // may be meta itself (i and j are read before anything is written).
 __device__ inline void nr_newsegs_one(int s, int out_slot, const int* seg, const int* meta, int* child,
                                       int* seg2, int* small, int* med, int* cnt,
-                                      int small_cap, int med_cap) {
+                                      int small_cap, int med_cap, int limit = kNrMedium) {
   const int l = seg[2 * s], ir = seg[2 * s + 1];
   const int i = meta[4 * s + 1], j = meta[4 * s + 2];
   int ids[2] = {-1, -1};
   const int lo[2] = {l, i}, hi[2] = {j - 1, ir};
   for (int c = 0; c < 2; ++c) {
-    if (hi[c] - lo[c] >= 7 && hi[c] - lo[c] < kNrMedium) {
+    if (hi[c] - lo[c] >= 7 && hi[c] - lo[c] < limit) {
       const int id = atomicAdd(&cnt[C_NMED], 1);
       if (id < med_cap) { med[2 * id] = lo[c]; med[2 * id + 1] = hi[c]; }
       else atomicExch(&cnt[C_OVERFLOW], 1);
@@ -433,7 +434,7 @@ __global__ void k_nr_newsegs(int in_slot, int out_slot, const int* __restrict__ 
                              int* __restrict__ cnt, int small_cap, int med_cap) {
   const int nseg = cnt[in_slot];
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nseg; s += gridDim.x * blockDim.x)
-    nr_newsegs_one(s, out_slot, seg, meta, meta, seg2, small, med, cnt, small_cap, med_cap);
+    nr_newsegs_one(s, out_slot, seg, meta, meta, seg2, small, med, cnt, small_cap, med_cap, kNrBlock);
 }
 
 __global__ void k_nr_segof(int n, const int* __restrict__ seg, const int* __restrict__ meta,
@@ -566,7 +567,7 @@ __global__ void __launch_bounds__(kCoopThreads) k_nr_levels(NrCoop A) {
     for (int q = tid + 1; q <= n; q += nthreads)
       idx2[q] = nr_apply_one(q, A.segof, seg, A.meta, idx, A.lf, A.rf, A.ls, A.rs, A.lpos, A.rpos);
     for (int s = tid; s < nseg; s += nthreads)
-      nr_newsegs_one(s, out, seg, A.meta, A.child, seg2, A.small, A.med, A.cnt, A.small_cap, A.med_cap);
+      nr_newsegs_one(s, out, seg, A.meta, A.child, seg2, A.small, A.med, A.cnt, A.small_cap, A.med_cap, kNrBlock);
     grid.sync();
     // segment ids from the children, and the next level's medians on the
     // partitioned permutation (they touch neither segof nor child: one phase)
@@ -606,10 +607,10 @@ __global__ void k_nr_insertion(int nsmall, const int* __restrict__ small, const 
   }
 }
 
-// The whole NR quicksort of one segment of 8..kNrMedium elements, as the
+// The whole NR quicksort of one segment of up to kNrMedium elements, as the
 // reference runs it (LocalMinima.f90:953-1044: median of three, Hoare scans,
 // larger part stacked, straight insertion below M = 7), by one thread on the
-// segment's keys and ids in shared memory; positions are relative to the
+// segment's keys and ids; positions are relative to the
 // segment (the median index (l+ir)/2 keeps its value relative to l).
 // Segments are independent, so the order they are finished in does not
 // matter, and the insertion stops at the segment's start as k_nr_insertion's does.
@@ -670,29 +671,218 @@ __device__ bool nr_sort_local(double* key, int* id, int n) {
   return false;
 }
 
-constexpr int kNrMedWarps = 4;
-__global__ void __launch_bounds__(32 * kNrMedWarps) k_nr_medium(int nmed, const int* __restrict__ med,
-                                                               const double* __restrict__ arr, int* __restrict__ idx,
-                                                               int* __restrict__ cnt) {
-  __shared__ double key[kNrMedWarps][kNrMedium];
-  __shared__ int id[kNrMedWarps][kNrMedium];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int s = blockIdx.x * kNrMedWarps + w; s < nmed; s += gridDim.x * kNrMedWarps) {
-    const int l = med[2 * s], n = med[2 * s + 1] - l + 1;
-    if (n < 8 || n > kNrMedium) {  // never: nr_newsegs_one routes only such segments here
-      if (lane == 0) atomicExch(&cnt[C_OVERFLOW], 1);
+// One segment of 8..kNrBlock elements per block, keys and ids in shared memory.
+// A warp partitions a segment as the reference's two scans do, kNrRuns runs
+// of 32 positions from either end at a time: ballots list the stoppers of both
+// chunks, the t-th of the left is exchanged with the t-th of the right while
+// they have not met (the crossing rule of nr_cross_one), and only exchanged
+// elements are written.  It goes on with the larger part and queues the other
+// for the block's other warps; parts of up to kNrTail elements are sorted at the
+// end, one thread each (nr_sort_local).
+//
+// Measured (B200) on 101^2's 3,994 keys: 96 us, against 466 for grid-wide levels
+// down to 512 elements and a lane per segment below.  A level-synchronous form
+// in one block (flags, prefix sums, positions and the permutation of all
+// segments, five barriers a level) is as fast there and slower from 257^2 on
+// (the whole stage 1,037 us against 965): it is bound by the shared memory's
+// throughput, fifteen accesses per element and level where this one reads
+// each once.  One run of 32 instead of four at a time costs 130 us more.
+constexpr int kNrThreads = 512, kNrWarps = kNrThreads / 32, kNrRuns = 4, kNrTail = 16;
+constexpr int kNrQueue = kNrBlock / 8;  // parts of more than kNrTail elements that ever wait for a warp, and idle warps' claims
+struct NrBlockShared {
+  double key[kNrBlock];
+  int id[kNrBlock];                // 1-based edge ids
+  unsigned tail[kNrBlock / 2];     // parts of 2..kNrTail elements: start << 16 | end
+  unsigned queue[kNrQueue];        // parts for any warp: start << 16 | end, kNrEmpty until filled
+  unsigned short at[kNrWarps][2][32 * kNrRuns];  // a warp's stopper positions, left and right
+  int head, filled, open, ntail;
+};
+constexpr unsigned kNrEmpty = 0xffffffffu;
+static_assert(sizeof(NrBlockShared) <= 227 * 1024, "one block per SM");
+
+// Partitions positions l..ir (ir - l >= 7) and returns the parts' borders: [l, j-1] and [i, ir].
+__device__ __forceinline__ void nr_partition_warp(NrBlockShared& S, unsigned short (*at)[32 * kNrRuns], int l, int ir,
+                                                  int lane, int& i_out, int& j_out) {
+  constexpr unsigned kAll = 0xffffffffu;
+  double* key = S.key;
+  int* id = S.id;
+  if (lane == 0) {  // median of three (LocalMinima.f90:985-1006)
+    auto swap = [&](int x, int y) {
+      const double t = key[x]; key[x] = key[y]; key[y] = t;
+      const int u = id[x]; id[x] = id[y]; id[y] = u;
+    };
+    swap((l + ir) / 2, l + 1);  // as with the array's positions: both bounds shift by the same amount
+    if (key[l + 1] > key[ir]) swap(l + 1, ir);
+    if (key[l] > key[ir]) swap(l, ir);
+    if (key[l + 1] > key[l]) swap(l + 1, l);
+  }
+  __syncwarp();
+  const double a = key[l];
+  const unsigned lt = (1u << lane) - 1u;
+  int li = l + 2, ri = ir - 1;          // next positions to look at
+  int last_l = l, last_r = ir + 1;      // last exchanged pair (the scans' limits)
+  int nl = 0, ol = 0, nr = 0, orr = 0;  // stoppers listed and already matched, left and right
+  int next_l, next_r;
+  for (;;) {
+    while (ol == nl && li < last_r) {  // list the next left stoppers
+      nl = ol = 0;
+      bool f[kNrRuns];
+#pragma unroll
+      for (int r = 0; r < kNrRuns; ++r) {
+        const int q = li + 32 * r + lane;
+        f[r] = key[min(q, ir)] >= a && q < last_r;
+      }
+#pragma unroll
+      for (int r = 0; r < kNrRuns; ++r) {
+        const unsigned m = __ballot_sync(kAll, f[r]);
+        if (f[r]) at[0][nl + __popc(m & lt)] = (unsigned short)(li + 32 * r + lane);
+        nl += __popc(m);
+      }
+      li += 32 * kNrRuns;
+    }
+    while (orr == nr && ri > last_l) {
+      nr = orr = 0;
+      bool f[kNrRuns];
+#pragma unroll
+      for (int r = 0; r < kNrRuns; ++r) {
+        const int q = ri - 32 * r - lane;
+        f[r] = key[max(q, l)] <= a && q > last_l;
+      }
+#pragma unroll
+      for (int r = 0; r < kNrRuns; ++r) {
+        const unsigned m = __ballot_sync(kAll, f[r]);
+        if (f[r]) at[1][nr + __popc(m & lt)] = (unsigned short)(ri - 32 * r - lane);
+        nr += __popc(m);
+      }
+      ri -= 32 * kNrRuns;
+    }
+    __syncwarp();
+    next_l = ol < nl ? at[0][ol] : last_r;  // where the left scan stops next
+    next_r = orr < nr ? at[1][orr] : last_l;
+    if (next_l >= next_r) break;
+    // the t-th stoppers of both lists, as long as they have not met
+    const int m = min(nl - ol, nr - orr);
+    int cnt = 0;
+    for (int t0 = 0; t0 < m; t0 += 32) {
+      const int t = t0 + lane;
+      const int pl = t < m ? at[0][ol + t] : 0, pr = t < m ? at[1][orr + t] : 0;
+      const bool ex = t < m && pl < pr;
+      if (ex) {
+        const double kl = key[pl], kr = key[pr];
+        const int il = id[pl], jr = id[pr];
+        key[pl] = kr;
+        key[pr] = kl;
+        id[pl] = jr;
+        id[pr] = il;
+      }
+      const int c = __popc(__ballot_sync(kAll, ex));
+      cnt += c;
+      if (c < 32) break;
+    }
+    ol += cnt;
+    orr += cnt;
+    last_l = at[0][ol - 1];
+    last_r = at[1][orr - 1];
+    __syncwarp();
+  }
+  // the scans stop at the next stoppers or, at the latest, at the positions
+  // exchanged last; on one and the same position they pass each other
+  int i = min(next_l, last_r), j = max(next_r, last_l);
+  if (ol < nl && orr < nr && next_l == next_r) {
+    i = next_l + 1;
+    j = next_l - 1;
+  }
+  __syncwarp();
+  if (lane == 0) {
+    const int v = id[l];
+    key[l] = key[j];
+    id[l] = id[j];
+    key[j] = a;
+    id[j] = v;
+  }
+  __syncwarp();
+  i_out = i;
+  j_out = j;
+}
+
+__global__ void __launch_bounds__(kNrThreads) k_nr_block(const int* __restrict__ nmedp, const int* __restrict__ med,
+                                                         int med_cap, const double* __restrict__ arr,
+                                                         int* __restrict__ idx, int* __restrict__ cnt) {
+  extern __shared__ __align__(16) unsigned char nr_smem[];
+  NrBlockShared& S = *reinterpret_cast<NrBlockShared*>(nr_smem);
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int nmed = min(*nmedp, med_cap);
+  for (int m = blockIdx.x; m < nmed; m += gridDim.x) {
+    const int base = med[2 * m], n = med[2 * m + 1] - base + 1;
+    if (n < 8 || n > kNrBlock) {  // never: nr_newsegs_one routes only such segments here
+      if (tid == 0) atomicExch(&cnt[C_OVERFLOW], 1);
       continue;
     }
-    for (int p = lane; p < n; p += 32) {
-      const int v = idx[l + p];
-      id[w][p] = v;
-      key[w][p] = arr[v];
+    for (int p = tid; p < n; p += kNrThreads) {
+      const int e = idx[base + p];
+      S.id[p] = e;
+      S.key[p] = arr[e];
     }
-    __syncwarp();
-    if (lane == 0 && !nr_sort_local(key[w], id[w], n)) atomicExch(&cnt[C_OVERFLOW], 1);
-    __syncwarp();
-    for (int p = lane; p < n; p += 32) idx[l + p] = id[w][p];
-    __syncwarp();
+    for (int p = tid; p < kNrQueue; p += kNrThreads) S.queue[p] = p == 0 && n > kNrTail ? (unsigned)(n - 1) : kNrEmpty;
+    if (tid == 0) {
+      S.head = 0;
+      S.filled = 1;
+      S.open = n > kNrTail ? 1 : 0;  // parts queued or in work
+      S.ntail = n > kNrTail ? 0 : 1;
+      S.tail[0] = (unsigned)(n - 1);
+    }
+    __syncthreads();
+    // every warp claims a queue slot and waits until it is filled or all parts are done
+    for (;;) {
+      int slot = 0;
+      if (lane == 0) slot = atomicAdd(&S.head, 1);
+      slot = __shfl_sync(0xffffffffu, slot, 0);
+      unsigned part = kNrEmpty;
+      if (lane == 0 && slot < kNrQueue)
+        for (;;) {
+          part = *(volatile unsigned*)&S.queue[slot];
+          if (part != kNrEmpty || *(volatile int*)&S.open == 0) break;
+          __nanosleep(20);
+        }
+      part = __shfl_sync(0xffffffffu, part, 0);
+      if (part == kNrEmpty) break;
+      __threadfence_block();
+      int l = (int)(part >> 16), ir = (int)(part & 0xffffu);
+      while (ir - l >= kNrTail) {
+        int i, j;
+        nr_partition_warp(S, S.at[wid], l, ir, lane, i, j);
+        // the larger part stays with this warp, the other goes to the queue
+        int al = l, ae = j - 1, bl = i, be = ir;
+        if (ae - al < be - bl) {
+          al = i; ae = ir; bl = l; be = j - 1;
+        }
+        if (lane == 0) {
+          if (be - bl >= kNrTail) {
+            __threadfence_block();
+            atomicAdd(&S.open, 1);
+            const int f = atomicAdd(&S.filled, 1);
+            if (f < kNrQueue) *(volatile unsigned*)&S.queue[f] = (unsigned)bl << 16 | (unsigned)be;
+            else atomicExch(&cnt[C_OVERFLOW], 1);  // never: each queued part leaves a larger one behind
+          } else if (be > bl) {
+            S.tail[atomicAdd(&S.ntail, 1)] = (unsigned)bl << 16 | (unsigned)be;
+          }
+          if (ae - al < kNrTail && ae > al) S.tail[atomicAdd(&S.ntail, 1)] = (unsigned)al << 16 | (unsigned)ae;
+        }
+        l = al;
+        ir = ae;
+        __syncwarp();
+      }
+      __threadfence_block();
+      if (lane == 0) atomicSub(&S.open, 1);
+    }
+    __syncthreads();
+    for (int t = tid; t < S.ntail; t += kNrThreads) {
+      const int l = (int)(S.tail[t] >> 16), len = (int)(S.tail[t] & 0xffffu) - l + 1;
+      if (!nr_sort_local(S.key + l, S.id + l, len)) atomicExch(&cnt[C_OVERFLOW], 1);
+    }
+    __syncthreads();
+    for (int p = tid; p < n; p += kNrThreads) idx[base + p] = S.id[p];
+    __syncthreads();
   }
 }
 
@@ -854,6 +1044,64 @@ __global__ void __launch_bounds__(kCoopThreads) k_mst_coop(MstCoop A) {
     if (!flat) {
       if (tid == 0) A.cnt[C_OVERFLOW] = 1;
       break;
+    }
+  }
+}
+
+// The same rounds in one block, components in shared memory, for graphs of at
+// most kMstBlockRoots basins and kMstBlockEdges edges: a block barrier costs
+// 40 ns, a grid-wide one several us (101^2, 1,000 basins: 148 -> 29 us).
+constexpr int kMstBlockRoots = 8192, kMstBlockEdges = 32768, kMstThreads = 512;
+__global__ void __launch_bounds__(kMstThreads) k_mst_block(MstCoop A) {
+  extern __shared__ int mst_sh[];
+  int *comp = mst_sh, *mn = mst_sh + A.nb, *next = mst_sh + 2 * A.nb;
+  volatile int* vc = comp;
+  const int tid = threadIdx.x;
+  for (int c = tid; c < A.nb; c += kMstThreads) comp[c] = c;
+  for (int round = 0; round < 64; ++round) {
+    for (int c = tid; c < A.nb; c += kMstThreads) mn[c] = INT_MAX;
+    __syncthreads();
+#pragma unroll 4
+    for (int e = tid; e < A.ne; e += kMstThreads) {
+      const int cu = comp[A.b1[e] - 1], cv = comp[A.b2[e] - 1], r = A.rank[e];
+      if (cu == cv) continue;
+      atomicMin(&mn[cu], r);
+      atomicMin(&mn[cv], r);
+    }
+    __syncthreads();
+    bool changed = false;
+    for (int c = tid; c < A.nb; c += kMstThreads) {
+      next[c] = comp[c];
+      if (comp[c] != c) continue;
+      const int r = mn[c];
+      if (r == INT_MAX) continue;
+      const int e = A.idx1[r + 1] - 1;
+      const int cu = comp[A.b1[e] - 1], cv = comp[A.b2[e] - 1];
+      const int other = cu == c ? cv : cu;
+      A.inmst[e] = 1;
+      if (mn[other] == r && c < other) continue;  // mutual choice: the smaller id stays a root
+      next[c] = other;
+      changed = true;
+    }
+    if (!__syncthreads_or(changed)) return;
+    for (int c = tid; c < A.nb; c += kMstThreads) comp[c] = next[c];
+    __syncthreads();
+    // flatten in place: pointers only move towards their roots
+    bool flat = false;
+    for (int pass = 0; pass < 64 && !flat; ++pass) {
+      bool moved = false;
+      for (int c = tid; c < A.nb; c += kMstThreads) {
+        const int r = vc[c], rr = vc[r];
+        if (rr != r) {
+          vc[c] = rr;
+          moved = true;
+        }
+      }
+      flat = !__syncthreads_or(moved);
+    }
+    if (!flat) {
+      if (tid == 0) A.cnt[C_OVERFLOW] = 1;
+      return;
     }
   }
 }
@@ -1021,10 +1269,11 @@ static bool nr_indexx(Ctx& c, int n, const double* w) {
   const int small_cap = (int)(c.conn_cap / 2 + 8);
   k_nr_init<<<grid1d(n + 2), kBlock, 0, c.stream>>>(n, idx, c.nr_segof, seg, c.nr_small, c.nr_med, c.d_cnt);
   c.count_launch();
-  int nseg = 1;  // k_nr_init makes one segment of the whole array when n > kNrMedium
-  if (n <= kNrMedium) {
-    fetch_counters(c, kNrCounters);
-    nseg = c.h_cnt[C_NSEG];
+  int nseg = 1;  // k_nr_init makes one segment of the whole array when n > kNrBlock
+  if (n <= kNrBlock) {  // k_nr_init made one segment of it: what it counted is known
+    nseg = 0;
+    c.h_cnt[C_NMED] = n >= 8 ? 1 : 0;
+    c.h_cnt[C_NSMALL] = n >= 2 && n < 8 ? 1 : 0;
   }
   if (nseg > 0 && nr_levels_coop(c, n, arr, small_cap)) {
     if (c.h_cnt[C_OVERFLOW]) { c.err = "NR sort emulation: small-segment buffer overflow"; return false; }
@@ -1066,8 +1315,14 @@ static bool nr_indexx(Ctx& c, int n, const double* w) {
   }
   const int nmed = c.h_cnt[C_NMED];
   if (nmed > 0) {
-    const int blocks = std::min((nmed + kNrMedWarps - 1) / kNrMedWarps, 148 * 16);
-    k_nr_medium<<<blocks, 32 * kNrMedWarps, 0, c.stream>>>(nmed, c.nr_med, arr, idx, c.d_cnt);
+    const int* nmedp = c.d_cnt + C_NMED;
+    int cap = nr_med_cap(c);
+    void* args[] = {&nmedp, &c.nr_med, &cap, &arr, &idx, &c.d_cnt};
+    if (!BigSmem<k_nr_block>::launch(std::min(nmed, 148), kNrThreads, sizeof(NrBlockShared), (int)sizeof(NrBlockShared),
+                                     c.stream, args)) {
+      c.err = "NR sort emulation: a block's shared memory is not available";
+      return false;
+    }
     c.count_launch();
   }
   const int nsmall = c.h_cnt[C_NSMALL];
@@ -1075,16 +1330,12 @@ static bool nr_indexx(Ctx& c, int n, const double* w) {
     k_nr_insertion<<<grid1d(nsmall), kBlock, 0, c.stream>>>(nsmall, c.nr_small, arr, idx);
     c.count_launch();
   }
-  if (nmed > 0) {  // the medium kernel reports an impossible segment through the overflow flag
-    fetch_counters(c, kNrCounters);
-    if (c.h_cnt[C_OVERFLOW]) { c.err = "NR sort emulation: medium segment out of range"; return false; }
-  }
   if (idx != c.nr_idx)
     cudaMemcpyAsync(c.nr_idx, idx, sizeof(int) * (n + 2), cudaMemcpyDeviceToDevice, c.stream);
   return true;
 }
 
-// Borůvka in one cooperative launch; false when the device refuses it or the
+// Borůvka in one launch (a block's, or a cooperative one); false when the device refuses it or the
 // graph is large (the host-driven rounds run instead).  Measured on B200: the
 // cooperative form saves the rounds' read-backs (1025^2 grid, 3.7e5 edges:
 // LocalMinima 3.12 -> 2.71 ms), but its grid-wide barriers over many blocks
@@ -1093,6 +1344,15 @@ static bool nr_indexx(Ctx& c, int n, const double* w) {
 constexpr int kMstCoopMax = 1 << 20;
 
 static bool mst_coop(Ctx& c, int nroots, int ne) {
+  if (nroots <= kMstBlockRoots && ne <= kMstBlockEdges) {
+    MstCoop A{nroots, ne, c.nr_idx, c.e_b1, c.e_b2, c.e_rank, c.mst_comp, c.mst_min, c.mst_next, c.e_inmst, c.d_cnt};
+    void* args[] = {&A};
+    if (BigSmem<k_mst_block>::launch(1, kMstThreads, 3 * sizeof(int) * (size_t)nroots,
+                                     3 * (int)sizeof(int) * kMstBlockRoots, c.stream, args)) {
+      c.count_launch();
+      return true;
+    }
+  }
   if (std::max(ne, nroots) > kMstCoopMax) return false;
   int dev = 0, coop = 0, sms = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -1219,7 +1479,7 @@ bool local_minima(Ctx& c) {
   const int ntree = c.h_cnt[C_NTREE];
   c.tree_size = ntree;
   if (c.h_cnt[C_OVERFLOW]) {
-    c.err = "LocalMinima: the spanning tree's components did not flatten";
+    c.err = "LocalMinima: the edge sort met an impossible segment or the tree's components did not flatten";
     return false;
   }
   if (ntree != nroots - 1) {

@@ -971,21 +971,23 @@ template <class Op, int LT>
 bool region_fits(const TileMap& tm) {
   const int smem = region_smem(tm);
   if (smem > kMaxSmem) return false;
-  auto kern = k_region_sweep<Op, LT>;
   // the permitted maximum covers every plan, so instances with different
   // plans never undo each other's setting
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
+  using Big = BigSmem<k_region_sweep<Op, LT>>;
   int dev = 0, sms = 0, per_sm = 0, coop = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, (size_t)smem) != cudaSuccess) {
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) {
     cudaGetLastError();
     return false;
   }
+  for (int t = 0; t < 2 && per_sm == 0; ++t)
+    if (!Big::allow(kMaxSmem, t == 1) ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_region_sweep<Op, LT>, kThreads, (size_t)smem) !=
+            cudaSuccess) {
+      cudaGetLastError();
+      per_sm = 0;
+    }
   return per_sm * sms >= tm.nctas;
 }
 

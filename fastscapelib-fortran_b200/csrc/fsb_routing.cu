@@ -162,32 +162,18 @@ __global__ void k_euler_tour(int nn, const int* __restrict__ rec, const int* __r
   }
 }
 
-// One Wyllie pointer-jumping round: value += value(succ); succ = succ(succ).
-__global__ void k_list_rank_round(size_t n, const unsigned long long* __restrict__ in,
-                                  unsigned long long* __restrict__ out) {
-  const unsigned END = 0xffffffffu;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const unsigned long long cur = in[e];
-    const unsigned nx = (unsigned)(cur >> 32);
-    if (nx == END) {
-      out[e] = cur;
-    } else {
-      const unsigned long long nb = in[nx];
-      const unsigned v = (unsigned)cur + (unsigned)nb;
-      out[e] = (nb & 0xffffffff00000000ull) | (unsigned long long)v;
-    }
-  }
-}
-
 // ---- list ranking by sublist walks (long lists) --------------------------------
 // Entry e's result is the suffix sum of the weights from e to its list's end.
-// Splitters: every kRankStride-th entry and every head (an entry that is no
+// Splitters: every STRIDE-th entry and every head (an entry that is no
 // entry's successor).  Each splitter walks its sublist up to the next
 // splitter, writing for every entry (splitter id << 32 | prefix), the prefix
 // being the weights before the entry within the sublist, and records
-// (next splitter id << 32 | sublist total).  Pointer jumping over the
-// splitters then gives each its suffix sum V, and entry e's result is
-// V(its splitter) - its prefix.  O(n) work against Wyllie's O(n log n).
+// (next splitter id << 32 | sublist total).  The splitters' list is ranked in
+// the same way, down to a list that one block ranks in shared memory; entry
+// e's result is its splitter's suffix sum minus its prefix.  O(n) work.
+// Ranking by pointer jumping alone, or over the first splitters, took one
+// launch per doubling: 42 launches and 133 us of 101^2's step, now 9 and 81,
+// the basin tree's list among them.
 
 // flags every entry that is some entry's successor; leaves the unused head
 // slots of the splitter list inert (no successor, weight 0)
@@ -204,6 +190,7 @@ __global__ void k_rank_pred(size_t n, const unsigned long long* __restrict__ lst
 
 // one sublist walk from splitter entry e with splitter id `id`; every step is
 // one dependent load, and the walk ends within n steps
+template <int STRIDE>
 __device__ void rank_walk(size_t n, const unsigned long long* __restrict__ lst, unsigned long long* __restrict__ sub,
                           unsigned long long* __restrict__ spl, size_t e, unsigned id, int* err) {
   const unsigned END = 0xffffffffu;
@@ -219,8 +206,8 @@ __device__ void rank_walk(size_t n, const unsigned long long* __restrict__ lst, 
       atomicExch(err, DEV_STACK_ERROR);
       break;
     }
-    if (nx % kRankStride == 0) {
-      nid = nx / kRankStride;
+    if (nx % STRIDE == 0) {
+      nid = nx / STRIDE;
       break;
     }
     x = nx;
@@ -228,19 +215,25 @@ __device__ void rank_walk(size_t n, const unsigned long long* __restrict__ lst, 
   spl[id] = ((unsigned long long)nid << 32) | pre;
 }
 
-// thread t: the splitter at t*kRankStride, then any head among the next
-// kRankStride - 1 entries (one 16-byte load of their flags)
+// thread t: the splitter at t*STRIDE, then any head among the next STRIDE - 1
+// entries (one load of their flags)
+template <int STRIDE>
 __global__ void k_rank_walk(size_t n, size_t s0, const unsigned long long* __restrict__ lst,
                             const unsigned char* __restrict__ pred, unsigned long long* __restrict__ sub,
                             unsigned long long* __restrict__ spl, unsigned* nheads, int* err) {
-  static_assert(kRankStride == 16, "one uint4 of flags per splitter");
+  static_assert(STRIDE == 16 || STRIDE == 4, "one word of flags per splitter");
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < s0; t += (size_t)gridDim.x * blockDim.x) {
-    const size_t base = t * kRankStride;
-    rank_walk(n, lst, sub, spl, base, (unsigned)t, err);
-    const uint4 f4 = *reinterpret_cast<const uint4*>(pred + base);
-    const unsigned f[4] = {f4.x, f4.y, f4.z, f4.w};
+    const size_t base = t * STRIDE;
+    rank_walk<STRIDE>(n, lst, sub, spl, base, (unsigned)t, err);
+    unsigned f[STRIDE / 4];
+    if constexpr (STRIDE == 16) {
+      const uint4 f4 = *reinterpret_cast<const uint4*>(pred + base);
+      f[0] = f4.x; f[1] = f4.y; f[2] = f4.z; f[3] = f4.w;
+    } else {
+      f[0] = *reinterpret_cast<const unsigned*>(pred + base);
+    }
 #pragma unroll
-    for (int j = 1; j < kRankStride; ++j) {
+    for (int j = 1; j < STRIDE; ++j) {
       const size_t e = base + j;
       if (e >= n || ((f[j >> 2] >> (8 * (j & 3))) & 0xffu) != 0u) continue;
       const unsigned h = atomicAdd(nheads, 1u);
@@ -248,10 +241,47 @@ __global__ void k_rank_walk(size_t n, size_t s0, const unsigned long long* __res
         atomicExch(err, DEV_OVERFLOW);
         continue;
       }
-      rank_walk(n, lst, sub, spl, e, (unsigned)(s0 + h), err);
+      rank_walk<STRIDE>(n, lst, sub, spl, e, (unsigned)(s0 + h), err);
     }
   }
 }
+
+// Pointer jumping over a whole list in one block's shared memory.
+constexpr int kRankThreads = 512, kRankEach = kRankBlock / kRankThreads;
+__global__ void __launch_bounds__(kRankThreads, 2) k_rank_block(int n, unsigned long long* __restrict__ lst) {
+  extern __shared__ unsigned long long rank_sh[];
+  const unsigned END = 0xffffffffu;
+  const int tid = threadIdx.x;
+  for (int e = tid; e < n; e += kRankThreads) rank_sh[e] = lst[e];
+  __syncthreads();
+  for (int r = 1; r < 2 * n; r <<= 1) {  // after round i a value covers 2^i entries
+    unsigned long long v[kRankEach];
+    bool moved = false;
+#pragma unroll
+    for (int i = 0; i < kRankEach; ++i) {
+      const int e = tid + i * kRankThreads;
+      if (e >= n) break;
+      v[i] = rank_sh[e];
+      const unsigned nx = (unsigned)(v[i] >> 32);
+      if (nx == END || nx >= (unsigned)n) continue;
+      const unsigned long long nb = rank_sh[nx];
+      v[i] = (nb & 0xffffffff00000000ull) | (unsigned)((unsigned)v[i] + (unsigned)nb);
+      moved = true;
+    }
+    if (!__syncthreads_or(moved)) break;
+#pragma unroll
+    for (int i = 0; i < kRankEach; ++i) {
+      const int e = tid + i * kRankThreads;
+      if (e >= n) break;
+      rank_sh[e] = v[i];
+    }
+    __syncthreads();
+  }
+  for (int e = tid; e < n; e += kRankThreads) lst[e] = rank_sh[e];
+}
+
+// a device that refuses the block's shared memory: the step reports it
+__global__ void k_rank_refused(int* err) { *err = DEV_OVERFLOW; }
 
 __global__ void k_rank_final(size_t n, const unsigned long long* __restrict__ sub,
                              const unsigned long long* __restrict__ vs, unsigned long long* __restrict__ out) {
@@ -296,35 +326,38 @@ void launch_find_donors(Ctx& c, const int* rec, int* ndon, int* don) {
   c.count_launch();
 }
 
-// Wyllie list ranking over `n` packed entries, ping-ponging between a and b.
-// Returns the buffer that holds the result.
-static unsigned long long* wyllie(Ctx& c, size_t n, unsigned long long* a, unsigned long long* b) {
-  int rounds = 1;
-  while (((size_t)1 << rounds) < n) ++rounds;
-  for (int r = 0; r < rounds; ++r) {
-    k_list_rank_round<<<grid1d(n), kBlock, 0, c.stream>>>(n, a, b);
+// Ranks list a (n packed entries) in place; sub holds n entries, ws the scratch
+// of the shorter lists.
+static void rank_list(Ctx& c, size_t n, unsigned long long* a, unsigned long long* sub, unsigned long long* ws) {
+  if (n <= (size_t)kRankBlock) {
+    int len = (int)n;
+    void* args[] = {&len, &a};
+    if (!BigSmem<k_rank_block>::launch(1, kRankThreads, sizeof(unsigned long long) * n,
+                                       (int)sizeof(unsigned long long) * kRankBlock, c.stream, args))
+      k_rank_refused<<<1, 1, 0, c.stream>>>(c.d_err);
     c.count_launch();
-    std::swap(a, b);
+    return;
   }
-  return a;
+  // a splitter every 16 entries, or every 4 where that is enough: the longest
+  // sublist, about stride * ln(splitters) entries, is the walk's time
+  const bool coarse = n > 4 * ((size_t)kRankBlock - kRankMaxHeads);
+  const size_t stride = coarse ? 16 : 4, s0 = (n + stride - 1) / stride, n1 = s0 + kRankMaxHeads;
+  unsigned long long* spl = ws;
+  cudaMemsetAsync(c.s_rank_pred, 0, s0 * stride, c.stream);  // whole flag words past n too
+  cudaMemsetAsync(c.s_rank_nheads, 0, sizeof(unsigned), c.stream);
+  k_rank_pred<<<grid1d(n), kBlock, 0, c.stream>>>(n, a, c.s_rank_pred, spl, s0);
+  const unsigned blocks = (unsigned)((s0 + 127) / 128);
+  if (coarse) k_rank_walk<16><<<blocks, 128, 0, c.stream>>>(n, s0, a, c.s_rank_pred, sub, spl, c.s_rank_nheads, c.d_err);
+  else k_rank_walk<4><<<blocks, 128, 0, c.stream>>>(n, s0, a, c.s_rank_pred, sub, spl, c.s_rank_nheads, c.d_err);
+  rank_list(c, n1, spl, ws + n1, ws + 2 * n1);
+  k_rank_final<<<grid1d(n), kBlock, 0, c.stream>>>(n, sub, spl, a);
+  c.count_launch(3);
 }
 
-// Suffix sums of `n` packed entries (succ << 32 | weight) in the low words of
-// the returned buffer (a or b).  Lists of 2^16 entries or more are ranked by
-// sublist walks (n <= 2*nn: the scratch is sized for that), shorter ones by
-// Wyllie alone.
+// Suffix sums of `n` <= 2*nn packed entries (succ << 32 | weight) in the low
+// words of the returned buffer, a; b holds as many entries of scratch.
 unsigned long long* list_rank(Ctx& c, size_t n, unsigned long long* a, unsigned long long* b) {
-  if (n < ((size_t)1 << 16) || n > 2 * (size_t)c.nn) return wyllie(c, n, a, b);
-  const size_t s0 = (n + kRankStride - 1) / kRankStride;
-  cudaMemsetAsync(c.s_rank_pred, 0, s0 * kRankStride, c.stream);  // whole flag words past n too
-  cudaMemsetAsync(c.s_rank_nheads, 0, sizeof(unsigned), c.stream);
-  k_rank_pred<<<grid1d(n), kBlock, 0, c.stream>>>(n, a, c.s_rank_pred, c.s_rank_sa, s0);
-  k_rank_walk<<<(unsigned)((s0 + 127) / 128), 128, 0, c.stream>>>(n, s0, a, c.s_rank_pred, b, c.s_rank_sa,
-                                                                    c.s_rank_nheads, c.d_err);
-  c.count_launch(2);
-  const unsigned long long* v = wyllie(c, s0 + kRankMaxHeads, c.s_rank_sa, c.s_rank_sb);
-  k_rank_final<<<grid1d(n), kBlock, 0, c.stream>>>(n, b, v, a);
-  c.count_launch();
+  rank_list(c, n, a, b, c.s_rank_ws);
   return a;
 }
 
