@@ -279,7 +279,7 @@ struct Patience {
   int spins = 0, back = 32;
   __device__ bool over(int* err) {
     if (++spins > kSpinLimit) {
-      atomicExch(err, DEV_SPIN_LIMIT);
+      atomicCAS(err, 0, DEV_SPIN_LIMIT);  // an earlier error is the cause
       return true;
     }
     return (spins & 63) == 0 && *(volatile int*)err != 0;
@@ -395,7 +395,7 @@ __global__ void k_top_down_leaves(int nn, const int* __restrict__ rec, const int
     const int r = rec[k];
     typename Op::State st = op.root();
     if (r != k && !op.poll(r, st)) {
-      atomicExch(err, DEV_SPIN_LIMIT);  // never: the walkers have finished
+      atomicCAS(err, 0, DEV_SPIN_LIMIT);  // only after an error: the walkers have finished
       continue;
     }
     op.step(st, op.load(k), k, r == k, true);

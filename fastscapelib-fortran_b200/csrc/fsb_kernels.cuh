@@ -224,7 +224,7 @@ void build_stack(Ctx& c, const int* rec, int* ndon, int* don, int* stack, int* p
 unsigned long long* list_rank(Ctx& c, size_t n, unsigned long long* a, unsigned long long* b);
 // list ranking by sublist walks: a splitter every 16 or 4 entries plus each
 // list head (at most kRankMaxHeads heads); a block ranks up to kRankBlock entries
-constexpr int kRankMaxHeads = 64, kRankBlock = 8192;
+constexpr int kRankMaxHeads = 4, kRankBlock = 8192;
 // scratch entries below a list of n: per level its splitters and their walk's results
 inline size_t rank_scratch(size_t n) {
   size_t total = 0;

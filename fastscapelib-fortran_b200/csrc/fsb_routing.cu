@@ -175,17 +175,25 @@ __global__ void k_euler_tour(int nn, const int* __restrict__ rec, const int* __r
 // launch per doubling: 42 launches and 133 us of 101^2's step, now 9 and 81,
 // the basin tree's list among them.
 
-// flags every entry that is some entry's successor; leaves the unused head
-// slots of the splitter list inert (no successor, weight 0)
+// Head slots of a splitter list that no head took are inert: no list holds
+// them, and in the next list they must not pass for heads themselves (counted
+// as heads they fill that list's slots, one level after the other).
+constexpr unsigned kInert = 0xfffffffeu;
+
+// flags every entry that is some entry's successor, and the inert ones; the
+// next list's head slots start inert
 __global__ void k_rank_pred(size_t n, const unsigned long long* __restrict__ lst, unsigned char* __restrict__ pred,
-                            unsigned long long* __restrict__ spl, size_t s0) {
-  const unsigned END = 0xffffffffu;
+                            unsigned long long* __restrict__ sub, unsigned long long* __restrict__ spl, size_t s0) {
   const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   for (size_t e = tid; e < n; e += (size_t)gridDim.x * blockDim.x) {
     const unsigned nx = (unsigned)(lst[e] >> 32);
-    if (nx != END && nx < n) pred[nx] = 1;
+    if (nx < n) pred[nx] = 1;
+    if (nx == kInert) {
+      pred[e] = 1;
+      sub[e] = 0;  // not walked unless a splitter; k_rank_final reads it
+    }
   }
-  if (tid < (size_t)kRankMaxHeads) spl[s0 + tid] = (unsigned long long)END << 32;
+  if (tid < (size_t)kRankMaxHeads) spl[s0 + tid] = (unsigned long long)kInert << 32;
 }
 
 // one sublist walk from splitter entry e with splitter id `id`; every step is
@@ -202,6 +210,10 @@ __device__ void rank_walk(size_t n, const unsigned long long* __restrict__ lst, 
     pre += (unsigned)cur;
     const unsigned nx = (unsigned)(cur >> 32);
     if (nx == END) break;
+    if (nx == kInert) {
+      nid = kInert;
+      break;
+    }
     if (nx >= n || steps >= n) {  // not a list
       atomicExch(err, DEV_STACK_ERROR);
       break;
@@ -345,7 +357,7 @@ static void rank_list(Ctx& c, size_t n, unsigned long long* a, unsigned long lon
   unsigned long long* spl = ws;
   cudaMemsetAsync(c.s_rank_pred, 0, s0 * stride, c.stream);  // whole flag words past n too
   cudaMemsetAsync(c.s_rank_nheads, 0, sizeof(unsigned), c.stream);
-  k_rank_pred<<<grid1d(n), kBlock, 0, c.stream>>>(n, a, c.s_rank_pred, spl, s0);
+  k_rank_pred<<<grid1d(n), kBlock, 0, c.stream>>>(n, a, c.s_rank_pred, sub, spl, s0);
   const unsigned blocks = (unsigned)((s0 + 127) / 128);
   if (coarse) k_rank_walk<16><<<blocks, 128, 0, c.stream>>>(n, s0, a, c.s_rank_pred, sub, spl, c.s_rank_nheads, c.d_err);
   else k_rank_walk<4><<<blocks, 128, 0, c.stream>>>(n, s0, a, c.s_rank_pred, sub, spl, c.s_rank_nheads, c.d_err);
