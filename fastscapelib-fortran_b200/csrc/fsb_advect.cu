@@ -103,22 +103,23 @@ void advect(Ctx& c) {
   const int nx = c.nx, ny = c.ny, nn = c.nn;
   cudaStream_t st = c.stream;
   const double dx = c.xl / (nx - 1), dy = c.yl / (ny - 1);
-  double *A = c.dA, *B = c.dB, *C = c.dC, *G = c.dG, *T = c.dK;
+  double *A = c.dA, *B = c.dB, *C = c.dC, *G = c.dG;
+  double* T[3] = {c.dK, c.dF, c.dZ};
   double* fields[3] = {c.h, c.b, c.etot};
   const dim3 tb(kT, 8);
   // x-pass: one system per row j, element i at [i*ny + j]
   k_adv_xcoef<<<dim3((nx + kT - 1) / kT, (ny + kT - 1) / kT), tb, 0, st>>>(nx, ny, c.dt, dx, c.vx, A, B, C);
   c.count_launch();
-  for (double* f : fields) {
-    k_transpose<<<dim3((nx + kT - 1) / kT, (ny + kT - 1) / kT), tb, 0, st>>>(ny, nx, f, T);
-    thomas_lines(c, nx, ny, 0, ny, A, B, C, T, G);
-    k_transpose<<<dim3((ny + kT - 1) / kT, (nx + kT - 1) / kT), tb, 0, st>>>(nx, ny, T, f);
-    c.count_launch(2);
-  }
+  for (int f = 0; f < 3; ++f)
+    k_transpose<<<dim3((nx + kT - 1) / kT, (ny + kT - 1) / kT), tb, 0, st>>>(ny, nx, fields[f], T[f]);
+  thomas_lines(c, nx, ny, 0, ny, A, B, C, T, G);
+  for (int f = 0; f < 3; ++f)
+    k_transpose<<<dim3((ny + kT - 1) / kT, (nx + kT - 1) / kT), tb, 0, st>>>(nx, ny, T[f], fields[f]);
+  c.count_launch(6);
   // y-pass: one system per column i, element j at [j*nx + i], solved in place
   k_adv_ycoef<<<grid1d(nn), kBlock, 0, st>>>(nx, ny, c.dt, dy, c.vy, A, B, C);
   c.count_launch();
-  for (double* f : fields) thomas_lines(c, ny, nx, 0, nx, A, B, C, f, G);
+  thomas_lines(c, ny, nx, 0, nx, A, B, C, fields, G);
   k_min_b<<<grid1d(nn), kBlock, 0, st>>>(nn, c.h, c.b);
   c.count_launch();
 }

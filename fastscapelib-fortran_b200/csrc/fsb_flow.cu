@@ -1038,17 +1038,34 @@ __device__ inline Equation y_equation(const Bounds& bd, double dt2, double dx2, 
 }
 
 // x pass coefficients for rows j=1..ny-2, stored transposed: element i of
-// row j at [i*ny + j]
+// row j at [i*ny + j], through a tile in shared memory so that both the reads
+// and the writes are rows
 template <class T>
-__global__ void k_diff_xcoef(Bounds bd, double dt2, double dx2, double dy2, const double* __restrict__ K,
-                             const double* __restrict__ z, T* __restrict__ A, T* __restrict__ B,
-                             T* __restrict__ C, T* __restrict__ F) {
-  const int nx = bd.nx, ny = bd.ny;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y + 1;
-  if (i >= nx || j > ny - 2) return;
-  const Equation e = x_equation(bd, dt2, dx2, dy2, K, z, i, j);
-  store_equation(A, B, C, F, (size_t)i * ny + j, e.a, e.bb, e.c, e.f, e.zm, e.z0, e.zp);
+__global__ void __launch_bounds__(256) k_diff_xcoef(Bounds bd, double dt2, double dx2, double dy2,
+                                                    const double* __restrict__ K, const double* __restrict__ z,
+                                                    T* __restrict__ A, T* __restrict__ B, T* __restrict__ C,
+                                                    T* __restrict__ F) {
+  __shared__ T tile[4][32][33];
+  const int nx = bd.nx, ny = bd.ny, i0 = blockIdx.x * 32, j0 = blockIdx.y * 32 + 1;
+  for (int r = threadIdx.y; r < 32; r += blockDim.y) {
+    const int i = i0 + threadIdx.x, j = j0 + r;
+    if (i < nx && j <= ny - 2) {
+      const Equation e = x_equation(bd, dt2, dx2, dy2, K, z, i, j);
+      store_equation(tile[0][r], tile[1][r], tile[2][r], tile[3][r], threadIdx.x, e.a, e.bb, e.c, e.f, e.zm, e.z0,
+                     e.zp);
+    }
+  }
+  __syncthreads();
+  for (int r = threadIdx.y; r < 32; r += blockDim.y) {
+    const int i = i0 + r, j = j0 + threadIdx.x;
+    if (i < nx && j <= ny - 2) {
+      const size_t o = (size_t)i * ny + j;
+      A[o] = tile[0][threadIdx.x][r];
+      B[o] = tile[1][threadIdx.x][r];
+      C[o] = tile[2][threadIdx.x][r];
+      F[o] = tile[3][threadIdx.x][r];
+    }
+  }
 }
 
 // y pass coefficients for columns i=1..nx-2 (natural layout [j*nx + i])
@@ -1065,125 +1082,238 @@ __global__ void k_diff_ycoef(Bounds bd, double dt2, double dx2, double dy2, cons
 }
 
 // tridag (Diffusion.f90:164-202) for independent systems s in [s0, s1):
-// element t of system s at [t*L + s]; the solution overwrites F.  A block
-// of 32 threads solves 32 systems, one each (the recurrence is sequential,
-// and its arithmetic is the reference's).  Coefficients move through shared
-// memory in chunks of kTC steps, double-buffered: the next chunk's copies
-// are in flight while the recurrence runs through the current one, so it
-// waits on its divisions, not on DRAM.  Every lane touches only its own
-// column of the buffers.
-constexpr int kTC = 16;
+// element t of system s at [t*L + s]; the solution overwrites F.  NR right-hand
+// sides share one matrix.  A block solves 32 systems, one per lane, with the
+// reference's arithmetic, whose two recurrences are its time: a division, a
+// product and a difference per equation for the pivots, and the same again for
+// the right-hand side.  They depend on each other one way only, so different
+// warps run them: while one computes the pivots of chunk q, another eliminates
+// chunk q-1 (one warp per right-hand side), others copy chunk q+2 in and write
+// chunk q-2 back, with a block barrier between chunks.  The
+// back substitution is staged likewise.
+//
+// Measured (B200), 2,047 systems of 2,049 equations: 682 us with one warp
+// per 32 systems doing all of it, 275 now.  Of 217 us in the elimination the
+// divisions' chain is about 140 (130 cycles an equation) and the copies alone
+// 132; equations loaded straight into the chains' registers take 450 us in
+// all, the loads' waits then lying on the chains.  Three right-hand sides in one
+// launch (advection of 513x511): 1,344 -> 445 us for both directions.
+constexpr int kTC = 8, kTAhead = 2, kTSlots = kTAhead + 3;  // equations per chunk, chunks copied ahead
+
+// step(r) for the first tn of K rows, with row(r) (its loads) issued kTPre rows
+// earlier; a whole chunk carries no tests
+constexpr int kTPre = 4;
+template <int K, class Row, class Step>
+__device__ __forceinline__ void in_chunk(int tn, Row row, Step step) {
+  if (tn == K) {
+#pragma unroll
+    for (int r = 0; r < kTPre; ++r) row(r);
+#pragma unroll
+    for (int r = 0; r < K; ++r) {
+      if (r + kTPre < K) row(r + kTPre);
+      step(r);
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < K; ++r)
+      if (r < tn) { row(r); step(r); }
+  }
+}
+
+template <class T, int NR>
+struct ThomasArgs {
+  const T *A, *B, *C;
+  T* F[NR];
+  T* G;
+  int N, L, s0, s1;
+  int* err;
+};
+template <class T, int NR>
+constexpr int thomas_smem() { return (3 + NR) * kTSlots * kTC * 32 * (int)sizeof(T); }
+
 __device__ inline void cp_async_elem(double* smem, const double* gmem) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
 
 __device__ inline void cp_async_elem(float* smem, const float* gmem) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
-__device__ inline void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+__device__ inline void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 
 template <int N>
 __device__ inline void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-template <class T>
-__global__ void __launch_bounds__(32) k_thomas(int N, int L, int s0, int s1, const T* __restrict__ A,
-                                               const T* __restrict__ B, const T* __restrict__ C,
-                                               T* __restrict__ F, T* __restrict__ G,
-                                               int* __restrict__ err) {
-  __shared__ T sa[2][kTC][33], sb[2][kTC][33], sc[2][kTC][33], sf[2][kTC][33];
-  const int lane = threadIdx.x;
-  const int s = s0 + blockIdx.x * 32 + lane;
-  const bool act = s < s1;
-  // forward elimination
-  auto load_fwd = [&](int buf, int t0) {
-    const int tn = min(kTC, N - t0);
-    if (act)
-      for (int r = 0; r < tn; ++r) {
-        const size_t o = (size_t)(t0 + r) * L + s;
-        cp_async_elem(&sa[buf][r][lane], &A[o]);
-        cp_async_elem(&sb[buf][r][lane], &B[o]);
-        cp_async_elem(&sf[buf][r][lane], &F[o]);
-        if (t0 + r > 0) cp_async_elem(&sc[buf][r][lane], &C[o - L]);
+template <class T, int NR>
+__global__ void __launch_bounds__(32 * (NR + 4)) k_thomas(ThomasArgs<T, NR> P) {
+  extern __shared__ __align__(16) unsigned char thomas_smem_raw[];
+  T* const sm = reinterpret_cast<T*>(thomas_smem_raw);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int N = P.N;
+  const size_t L = P.L;
+  const int sys = P.s0 + blockIdx.x * 32 + lane;
+  const bool act = sys < P.s1;
+  const bool loader = warp > NR + 1, storer = warp == NR + 1;
+  const int half = warp - (NR + 2);  // of the loaders
+  const int rhs = warp - 1;  // of warps 1..NR
+
+  // row r of array v (0: a, 1: b, later the pivot, 2: c, later g, 3..: f, later
+  // u) of the slot that chunk q has
+  auto at = [&](int q, int v, int r) { return sm + (((q % kTSlots) * (3 + NR) + v) * kTC + r) * 32 + lane; };
+  const int nq = (N + kTC - 1) / kTC;
+  // one warp copies a and c, the other b and f
+  auto load = [&](int q) {
+    if (act && q < nq) {
+      const int t0 = q * kTC, tn = min(kTC, N - t0);
+      const size_t o = t0 * L + sys;
+      const T* x = (half ? P.B : P.A) + o;
+      T* const to = at(q, half, 0);
+#pragma unroll
+      for (int r = 0; r < kTC; ++r)
+        if (r < tn) cp_async_elem(to + r * 32, x + r * L);
+      if (half) {
+#pragma unroll
+        for (int v = 0; v < NR; ++v)
+#pragma unroll
+          for (int r = 0; r < kTC; ++r)
+            if (r < tn) cp_async_elem(at(q, 3 + v, 0) + r * 32, P.F[v] + o + r * L);
+      } else {
+        const T* y = P.C + o - L;
+#pragma unroll
+        for (int r = 0; r < kTC; ++r)
+          if (r < tn && t0 + r > 0) cp_async_elem(at(q, 2, 0) + r * 32, y + r * L);
       }
+    }
     cp_async_commit();
   };
-  T bet = 0, up = 0;
+  if (loader) {
+    for (int q = 0; q < kTAhead; ++q) load(q);
+    cp_async_wait<kTAhead - 1>();
+  }
+  __syncthreads();
+  T bet = 1, u = 0;
   bool bad = false;
-  load_fwd(0, 0);
-  for (int t0 = 0, k = 0; t0 < N; t0 += kTC, ++k) {
-    const int buf = k & 1;
-    const int tn = min(kTC, N - t0);
-    if (t0 + kTC < N) {
-      load_fwd(buf ^ 1, t0 + kTC);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncwarp();
-    if (act && !bad) {
-      for (int r = 0; r < tn; ++r) {
-        const int t = t0 + r;
-        if (t == 0) {
-          bet = sb[buf][0][lane];
-          if (bet == 0.0) { bad = true; break; }
-          up = sf[buf][0][lane] / bet;
-          sf[buf][0][lane] = up;
-          sc[buf][0][lane] = 0.0;
-        } else {
-          const T g = sc[buf][r][lane] / bet;
-          sc[buf][r][lane] = g;
-          bet = sb[buf][r][lane] - sa[buf][r][lane] * g;
-          if (bet == 0.0) { bad = true; break; }
-          up = (sf[buf][r][lane] - sa[buf][r][lane] * up) / bet;
-          sf[buf][r][lane] = up;
-        }
+  for (int q = 0; q < nq + 2; ++q) {
+    if (loader) {
+      load(q + kTAhead);
+      cp_async_wait<kTAhead - 1>();
+    } else if (storer) {
+      if (act && q >= 2) {
+        const int t0 = (q - 2) * kTC, tn = min(kTC, N - t0);
+        const size_t o = t0 * L + sys;
+#pragma unroll
+        for (int r = 0; r < kTC; ++r)
+          if (r < tn) P.G[o + r * L] = *at(q - 2, 2, r);
+#pragma unroll
+        for (int v = 0; v < NR; ++v)
+#pragma unroll
+          for (int r = 0; r < kTC; ++r)
+            if (r < tn) P.F[v][o + r * L] = *at(q - 2, 3 + v, r);
       }
-    }
-    if (act)
-      for (int r = 0; r < tn; ++r) {
-        const size_t o = (size_t)(t0 + r) * L + s;
-        F[o] = sf[buf][r][lane];
-        G[o] = sc[buf][r][lane];
+    } else if (warp == 0) {
+      if (act && q < nq) {
+        // the rows' loads are issued kTPre rows ahead, in the gaps of the chain
+        T a[kTC], b[kTC], c[kTC];
+        auto row = [&](int r) { a[r] = *at(q, 0, r); b[r] = *at(q, 1, r); c[r] = *at(q, 2, r); };
+        in_chunk<kTC>(min(kTC, N - q * kTC), row, [&](int r) {
+          T g = 0;
+          if (r == 0 && q == 0) {
+            bet = b[0];
+          } else {
+            g = c[r] / bet;
+            bet = b[r] - a[r] * g;
+          }
+          bad |= bet == T(0);
+          *at(q, 2, r) = g;
+          *at(q, 1, r) = bet;
+        });
       }
-    __syncwarp();
+    } else if (act && !bad && q >= 1 && q - 1 < nq) {
+      T a[kTC], b[kTC], f[kTC];
+      auto row = [&](int r) { a[r] = *at(q - 1, 0, r); b[r] = *at(q - 1, 1, r); f[r] = *at(q - 1, 3 + rhs, r); };
+      in_chunk<kTC>(min(kTC, N - (q - 1) * kTC), row, [&](int r) {
+        bad |= b[r] == T(0);
+        u = r == 0 && q == 1 ? f[0] / b[0] : (f[r] - a[r] * u) / b[r];
+        if (!bad) *at(q - 1, 3 + rhs, r) = u;
+      });
+    }
+    __syncthreads();  // the last one also orders the stores before the loads below
   }
-  if (bad) { atomicExch(err, DEV_TRIDAG_ZERO); return; }
-  // back substitution u(t) = u(t) - gam(t+1)*u(t+1), chunked from the end;
-  // this lane's forward stores are visible to its own later loads
-  auto load_bwd = [&](int buf, int t1) {
-    const int tlo = max(0, t1 - kTC);
-    if (act)
-      for (int r = 0; r < t1 - tlo; ++r) {
-        const size_t o = (size_t)(tlo + r) * L + s;
-        cp_async_elem(&sf[buf][r][lane], &F[o]);
-        cp_async_elem(&sc[buf][r][lane], &G[o + L]);
+  if (warp == 0 && bad) atomicExch(P.err, DEV_TRIDAG_ZERO);
+
+  // back substitution u(t) = u(t) - gam(t+1)*u(t+1), in chunks from the end;
+  // a system with a zero pivot stays as it is
+  constexpr int kTB = kTC * (3 + NR) / (1 + NR);
+  auto back = [&](int q, int v, int r) { return sm + (((q % kTSlots) * (1 + NR) + v) * kTB + r) * 32 + lane; };
+  const int nb = (N - 1 + kTB - 1) / kTB;
+  auto load_back = [&](int q) {  // one loader copies u, the other g
+    if (act && q < nb) {
+      const int t1 = N - 1 - q * kTB, tn = min(kTB, t1);
+      const size_t o = (size_t)(t1 - 1) * L + sys;
+      if (half) {
+#pragma unroll
+        for (int v = 0; v < NR; ++v)
+#pragma unroll
+          for (int r = 0; r < kTB; ++r)
+            if (r < tn) cp_async_elem(back(q, 1 + v, r), P.F[v] + o - r * L);
+      } else {
+#pragma unroll
+        for (int r = 0; r < kTB; ++r)
+          if (r < tn) cp_async_elem(back(q, 0, r), P.G + o + L - r * L);
       }
+    }
     cp_async_commit();
   };
-  if (act) up = F[(size_t)(N - 1) * L + s];
-  if (N > 1) load_bwd(0, N - 1);
-  for (int t1 = N - 1, k = 0; t1 > 0; t1 -= kTC, ++k) {
-    const int buf = k & 1;
-    const int tlo = max(0, t1 - kTC);
-    const int tn = t1 - tlo;
-    if (tlo > 0) {
-      load_bwd(buf ^ 1, tlo);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncwarp();
-    if (act)
-      for (int r = tn - 1; r >= 0; --r) {
-        up = sf[buf][r][lane] - sc[buf][r][lane] * up;
-        sf[buf][r][lane] = up;
-      }
-    if (act)
-      for (int r = 0; r < tn; ++r) F[(size_t)(tlo + r) * L + s] = sf[buf][r][lane];
-    __syncwarp();
+  if (loader) {
+    for (int q = 0; q < kTAhead; ++q) load_back(q);
+    cp_async_wait<kTAhead - 1>();
   }
+  __syncthreads();
+  for (int q = 0; q < nb + 1; ++q) {
+    if (loader) {
+      load_back(q + kTAhead);
+      cp_async_wait<kTAhead - 1>();
+    } else if (storer) {
+      if (act && q >= 1) {
+        const int t1 = N - 1 - (q - 1) * kTB, tn = min(kTB, t1);
+        const size_t o = (size_t)(t1 - 1) * L + sys;
+#pragma unroll
+        for (int v = 0; v < NR; ++v)
+#pragma unroll
+          for (int r = 0; r < kTB; ++r)
+            if (r < tn) P.F[v][o - r * L] = *back(q - 1, 1 + v, r);
+      }
+    } else if (warp > 0 && act && !bad && q < nb) {
+      T g[kTB], f[kTB];
+      auto row = [&](int r) { g[r] = *back(q, 0, r); f[r] = *back(q, 1 + rhs, r); };
+      in_chunk<kTB>(min(kTB, N - 1 - q * kTB), row, [&](int r) {
+        u = f[r] - g[r] * u;
+        *back(q, 1 + rhs, r) = u;
+      });
+    }
+    __syncthreads();
+  }
+}
+
+template <class T, int NR>
+static void launch_thomas(ThomasArgs<T, NR> P, cudaStream_t st);
+// one right-hand side
+template <class T>
+static void thomas1(int N, int L, int s0, int s1, const T* A, const T* B, const T* C, T* F, T* G, int* err,
+                    cudaStream_t st) {
+  launch_thomas(ThomasArgs<T, 1>{A, B, C, {F}, G, N, L, s0, s1, err}, st);
+}
+template <class T, int NR>
+static void launch_thomas(ThomasArgs<T, NR> P, cudaStream_t st) {
+  if (P.s1 <= P.s0) return;
+  void* args[] = {&P};
+  constexpr int smem = thomas_smem<T, NR>();
+  const unsigned blocks = (P.s1 - P.s0 + 31) / 32, threads = 32 * (NR + 4);
+  if (smem <= 48 * 1024)
+    cudaLaunchKernel((const void*)k_thomas<T, NR>, dim3(blocks), dim3(threads), args, (size_t)smem, st);
+  else if (!BigSmem<k_thomas<T, NR>>::launch(blocks, threads, (size_t)smem, smem, st, args))
+    for (int v = 0; v < NR; ++v) thomas1(P.N, P.L, P.s0, P.s1, P.A, P.B, P.C, P.F[v], P.G, P.err, st);
 }
 
 // zint = x-pass result on rows 1..ny-2, h elsewhere (natural layout); in the
@@ -1395,10 +1525,9 @@ void stream_power(Ctx& c) {
   c.count_launch();
 }
 
-void thomas_lines(Ctx& c, int N, int L, int s0, int s1, const double* A, const double* B, const double* C, double* F,
-                  double* G) {
-  if (s1 <= s0) return;
-  k_thomas<double><<<(s1 - s0 + 31) / 32, 32, 0, c.stream>>>(N, L, s0, s1, A, B, C, F, G, c.d_err);
+void thomas_lines(Ctx& c, int N, int L, int s0, int s1, const double* A, const double* B, const double* C,
+                  double* const* F, double* G) {
+  launch_thomas(ThomasArgs<double, 3>{A, B, C, {F[0], F[1], F[2]}, G, N, L, s0, s1, c.d_err}, c.stream);
   c.count_launch();
 }
 
@@ -1413,17 +1542,17 @@ static void diffusion_mixed(Ctx& c) {
         *C = reinterpret_cast<float*>(c.dC), *F = reinterpret_cast<float*>(c.dF),
         *G = reinterpret_cast<float*>(c.dG);
   k_diff_kdint<<<grid1d(nn), kBlock, 0, c.stream>>>(nn, c.kdsed, c.kd, c.h, c.b, K);
-  dim3 gx((nx + 127) / 128, ny - 2);
-  k_diff_xcoef<float><<<gx, 128, 0, c.stream>>>(c.bd, dt2, dx2, dy2, K, c.h, A, B, C, F);
+  dim3 gx((nx + 31) / 32, (ny - 2 + 31) / 32);
+  k_diff_xcoef<float><<<gx, dim3(32, 8), 0, c.stream>>>(c.bd, dt2, dx2, dy2, K, c.h, A, B, C, F);
   stage_begin(c, KT_THOMAS_ROWS);
-  k_thomas<float><<<(ny - 2 + 31) / 32, 32, 0, c.stream>>>(nx, ny, 1, ny - 1, A, B, C, F, G, c.d_err);
+  thomas1<float>(nx, ny, 1, ny - 1, A, B, C, F, G, c.d_err, c.stream);
   stage_end(c, KT_THOMAS_ROWS);
   dim3 g2((nx + 31) / 32, (ny + 31) / 32);
   k_diff_xgather<float><<<g2, dim3(32, 8), 0, c.stream>>>(c.bd, F, c.h, Z);
   dim3 gy((nx + 127) / 128, ny);
   k_diff_ycoef<float><<<gy, 128, 0, c.stream>>>(c.bd, dt2, dx2, dy2, K, Z, A, B, C, F);
   stage_begin(c, KT_THOMAS_COLS);
-  k_thomas<float><<<(nx - 2 + 31) / 32, 32, 0, c.stream>>>(ny, nx, 1, nx - 1, A, B, C, F, G, c.d_err);
+  thomas1<float>(ny, nx, 1, nx - 1, A, B, C, F, G, c.d_err, c.stream);
   stage_end(c, KT_THOMAS_COLS);
   k_diff_finish_m<<<grid1d(nn), kBlock, 0, c.stream>>>(c.bd, c.dt, F, Z, c.h, c.b, c.etot, c.erate);
   c.count_launch(7);
@@ -1440,11 +1569,11 @@ void diffusion(Ctx& c) {
   k_diff_kdint<<<grid1d(nn), kBlock, 0, c.stream>>>(nn, c.kdsed, c.kd, c.h, c.b, K);
   c.count_launch();
   {
-    dim3 g((nx + 127) / 128, ny - 2);
-    k_diff_xcoef<double><<<g, 128, 0, c.stream>>>(c.bd, dt2, dx2, dy2, K, c.h, A, B, C, F);
+    dim3 g((nx + 31) / 32, (ny - 2 + 31) / 32);
+    k_diff_xcoef<double><<<g, dim3(32, 8), 0, c.stream>>>(c.bd, dt2, dx2, dy2, K, c.h, A, B, C, F);
     // systems are rows j=1..ny-2 with element i at [i*ny + j]
     stage_begin(c, KT_THOMAS_ROWS);
-    k_thomas<double><<<(ny - 2 + 31) / 32, 32, 0, c.stream>>>(nx, ny, 1, ny - 1, A, B, C, F, G, c.d_err);
+    thomas1<double>(nx, ny, 1, ny - 1, A, B, C, F, G, c.d_err, c.stream);
     stage_end(c, KT_THOMAS_ROWS);
     dim3 g2((nx + 31) / 32, (ny + 31) / 32);
     k_diff_xgather<double><<<g2, dim3(32, 8), 0, c.stream>>>(c.bd, F, c.h, Z);
@@ -1454,7 +1583,7 @@ void diffusion(Ctx& c) {
     dim3 g((nx + 127) / 128, ny);
     k_diff_ycoef<double><<<g, 128, 0, c.stream>>>(c.bd, dt2, dx2, dy2, K, Z, A, B, C, F);
     stage_begin(c, KT_THOMAS_COLS);
-    k_thomas<double><<<(nx - 2 + 31) / 32, 32, 0, c.stream>>>(ny, nx, 1, nx - 1, A, B, C, F, G, c.d_err);
+    thomas1<double>(ny, nx, 1, nx - 1, A, B, C, F, G, c.d_err, c.stream);
     stage_end(c, KT_THOMAS_COLS);
     c.count_launch(2);
   }
@@ -1477,14 +1606,14 @@ void diffusion_raw(const Bounds& bd, double dx, double dy, double dt, double kds
   double* G = F + nn;
   double* Z = G + nn;
   k_diff_kdint<<<grid1d(nn), kBlock, 0, st>>>(nn, kdsed, kd, h, b, K);
-  dim3 gx((nx + 127) / 128, ny - 2);
-  k_diff_xcoef<double><<<gx, 128, 0, st>>>(bd, dt2, dx2, dy2, K, h, A, B, C, F);
-  k_thomas<double><<<(ny - 2 + 31) / 32, 32, 0, st>>>(nx, ny, 1, ny - 1, A, B, C, F, G, err);
+  dim3 gx((nx + 31) / 32, (ny - 2 + 31) / 32);
+  k_diff_xcoef<double><<<gx, dim3(32, 8), 0, st>>>(bd, dt2, dx2, dy2, K, h, A, B, C, F);
+  thomas1<double>(nx, ny, 1, ny - 1, A, B, C, F, G, err, st);
   dim3 gt((nx + 31) / 32, (ny + 31) / 32);
   k_diff_xgather<double><<<gt, dim3(32, 8), 0, st>>>(bd, F, h, Z);
   dim3 gy((nx + 127) / 128, ny);
   k_diff_ycoef<double><<<gy, 128, 0, st>>>(bd, dt2, dx2, dy2, K, Z, A, B, C, F);
-  k_thomas<double><<<(nx - 2 + 31) / 32, 32, 0, st>>>(ny, nx, 1, nx - 1, A, B, C, F, G, err);
+  thomas1<double>(ny, nx, 1, nx - 1, A, B, C, F, G, err, st);
   k_diff_finish<<<grid1d(nn), kBlock, 0, st>>>(bd, dt, F, h, b, etot, erate);
 }
 

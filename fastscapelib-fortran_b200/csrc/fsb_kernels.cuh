@@ -265,8 +265,8 @@ void flux_mfd(Ctx& c, double* flux);                  // compute_fluxes' flux, m
 TileMap plan_tiles(int nx, int ny, int lt, int sms);
 bool region_accumulate(Ctx& c);
 bool region_stream_power(Ctx& c);
-void thomas_lines(Ctx& c, int N, int L, int s0, int s1, const double* A, const double* B, const double* C, double* F,
-                  double* G);
+void thomas_lines(Ctx& c, int N, int L, int s0, int s1, const double* A, const double* B, const double* C,
+                  double* const* F, double* G);
 void advect(Ctx& c);  // fsb_advect.cu
 int write_vtk(Ctx& c, const double* f_dev, double vex, const char* dir);  // fsb_vtk.cu
 // the stream power law with the sediment term g > 0 (fsb_sediment.cu)
