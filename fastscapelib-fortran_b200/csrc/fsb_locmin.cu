@@ -34,18 +34,24 @@ namespace {
 enum {
   C_NBASINS = 0, C_NLOCMIN = 1, C_BASIN0 = 2, C_NEDGE = 3, C_NSEG = 4, C_NSMALL = 5,
   C_CHANGED = 6, C_NTREE = 7, C_NLOCMIN_AFTER = 8, C_OVERFLOW = 9, C_NSEG2 = 11,
-  C_NRIDX = 12, C_NRLEVELS = 13, C_NMED = 14,
+  C_NRIDX = 12, C_NRLEVELS = 13, C_NMED = 14, C_NRHEAD = 15, C_NROPEN = 16,
   C_MST_CHANGED = 24, C_MST_FLAT = 25,  // 25..27: the cooperative MST's rotating flags
   C_MST_DONE = 28                        // host-driven MST: a round changed nothing
 };
 constexpr int kNrCounters = 15;  // counters the NR sort reads back
 
-// Segments of 8..kNrBlock elements leave the level-synchronous partition and
-// are finished each by one block in shared memory (k_nr_block), where a
-// barrier costs 40 ns instead of the several us of a grid-wide one.  kNrMedium
-// is the longest segment nr_sort_local takes.
+// The sort's segments by length: above kNrSplit they are partitioned level by
+// level over the whole grid, up to kNrSplit by one block in global memory (the
+// parts of one segment by as many blocks), up to kNrBlock in a block's shared
+// memory (both k_nr_block).  kNrMedium is the longest part nr_sort_local takes.
+// A grid-wide level costs 80-110 us whatever its segments are, most of it
+// barriers; a block partitions 91,445 elements in 50 us and 4,000 in 8, and
+// the parts go on at once.  With kNrSplit 2^17 or 2^19 the stage of 2049^2
+// takes 120 or 530 us more; with kNrBlock 1,024 or 4,096 that of 2049^2 330
+// more or as long, that of 101^2 6 less or 45 more.
 constexpr int kNrMedium = 512;
-constexpr int kNrBlock = 8192;
+constexpr int kNrBlock = 2048;
+constexpr int kNrSplit = 1 << 18;
 
 // Level bound of the emulation: every level shrinks every segment by at least
 // its pivot, so n + 8 levels always suffice.  A fixed bound would not do: the
@@ -221,20 +227,33 @@ __global__ void k_conn_gather(int n, const int* __restrict__ perm, const int* __
 
 // ---- loc_min_3_indexx emulation (1-based positions l..ir) -----------------
 // idx[1..n] holds 1-based edge ids, arr[1..n] the weights (arr = w - 1).
-__global__ void k_nr_init(int n, int* __restrict__ idx, int* __restrict__ segof, int* __restrict__ seg,
-                          int* __restrict__ small, int* __restrict__ med, int* __restrict__ cnt) {
-  const bool level = n > kNrBlock;  // else the whole array is one block's or one small segment
+// key (the weights in the segments' order) is what the blocks' partitions
+// move along with idx
+__global__ void k_nr_init(int n, const double* __restrict__ arr, int* __restrict__ idx, double* __restrict__ key,
+                          int* __restrict__ segof, int* __restrict__ seg, int* __restrict__ small,
+                          int* __restrict__ med, int* __restrict__ cnt) {
+  const bool level = n > kNrSplit;  // else the whole array is one block's or one small segment
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q <= n + 1; q += gridDim.x * blockDim.x) {
-    if (q >= 1 && q <= n) idx[q] = q;
-    segof[q] = (q >= 1 && q <= n && level) ? 0 : -1;
+    if (q >= 1 && q <= n) {
+      idx[q] = q;
+      if (!level) key[q] = arr[q];
+    }
+    if (level) segof[q] = q >= 1 && q <= n ? 0 : -1;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     cnt[C_NSEG] = 0;
     cnt[C_NMED] = 0;
+    cnt[C_NRHEAD] = 0;
+    cnt[C_NROPEN] = 1;  // segments queued or in work
     if (level) { seg[0] = 1; seg[1] = n; cnt[C_NSEG] = 1; }
     else if (n - 1 >= 7) { med[0] = 1; med[1] = n; cnt[C_NMED] = 1; }
     else if (n >= 2) { small[0] = 1; small[1] = n; cnt[C_NSMALL] = 1; }
   }
+}
+__global__ void k_nr_keys(int n, const double* __restrict__ arr, const int* __restrict__ idx,
+                          double* __restrict__ key, int* __restrict__ cnt) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) cnt[C_NROPEN] = cnt[C_NMED];
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x + 1; q <= n; q += gridDim.x * blockDim.x) key[q] = arr[idx[q]];
 }
 
 __device__ inline void iswap(int* v, int a, int b) { const int t = v[a]; v[a] = v[b]; v[b] = t; }
@@ -434,7 +453,7 @@ __global__ void k_nr_newsegs(int in_slot, int out_slot, const int* __restrict__ 
                              int* __restrict__ cnt, int small_cap, int med_cap) {
   const int nseg = cnt[in_slot];
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nseg; s += gridDim.x * blockDim.x)
-    nr_newsegs_one(s, out_slot, seg, meta, meta, seg2, small, med, cnt, small_cap, med_cap, kNrBlock);
+    nr_newsegs_one(s, out_slot, seg, meta, meta, seg2, small, med, cnt, small_cap, med_cap, kNrSplit);
 }
 
 __global__ void k_nr_segof(int n, const int* __restrict__ seg, const int* __restrict__ meta,
@@ -567,7 +586,7 @@ __global__ void __launch_bounds__(kCoopThreads) k_nr_levels(NrCoop A) {
     for (int q = tid + 1; q <= n; q += nthreads)
       idx2[q] = nr_apply_one(q, A.segof, seg, A.meta, idx, A.lf, A.rf, A.ls, A.rs, A.lpos, A.rpos);
     for (int s = tid; s < nseg; s += nthreads)
-      nr_newsegs_one(s, out, seg, A.meta, A.child, seg2, A.small, A.med, A.cnt, A.small_cap, A.med_cap, kNrBlock);
+      nr_newsegs_one(s, out, seg, A.meta, A.child, seg2, A.small, A.med, A.cnt, A.small_cap, A.med_cap, kNrSplit);
     grid.sync();
     // segment ids from the children, and the next level's medians on the
     // partitioned permutation (they touch neither segof nor child: one phase)
@@ -671,34 +690,48 @@ __device__ bool nr_sort_local(double* key, int* id, int n) {
   return false;
 }
 
-// One segment of 8..kNrBlock elements per block, keys and ids in shared memory.
-// A warp partitions a segment as the reference's two scans do, kNrRuns runs
+// Segments of 8..kNrSplit elements, taken by blocks from a queue.  A block
+// partitions a segment above kNrBlock as a whole (nr_partition_block), goes on
+// with the larger part and queues the other.  Up to kNrBlock elements are sorted
+// in shared memory: a warp partitions a segment as the reference's two scans do, kNrRuns runs
 // of 32 positions from either end at a time: ballots list the stoppers of both
 // chunks, the t-th of the left is exchanged with the t-th of the right while
 // they have not met (the crossing rule of nr_cross_one), and only exchanged
 // elements are written.  It goes on with the larger part and queues the other
 // for the block's other warps; parts of up to kNrTail elements are sorted at the
-// end, one thread each (nr_sort_local).
+// end by eight lanes each.
 //
-// Measured (B200) on 101^2's 3,994 keys: 96 us, against 466 for grid-wide levels
-// down to 512 elements and a lane per segment below.  A level-synchronous form
-// in one block (flags, prefix sums, positions and the permutation of all
-// segments, five barriers a level) is as fast there and slower from 257^2 on
-// (the whole stage 1,037 us against 965): it is bound by the shared memory's
-// throughput, fifteen accesses per element and level where this one reads
-// each once.  One run of 32 instead of four at a time costs 130 us more.
-constexpr int kNrThreads = 512, kNrWarps = kNrThreads / 32, kNrRuns = 4, kNrTail = 16;
-constexpr int kNrQueue = kNrBlock / 8;  // parts of more than kNrTail elements that ever wait for a warp, and idle warps' claims
+// Measured (B200): 101^2's 4,076 keys 466 us with grid-wide levels down to 512
+// elements and a lane per segment below, 96 in one block, 83 now; 513x511's
+// 91,445 keys 570 with grid-wide levels down to 8,192 elements, 290 now, bound
+// by the chain of partitions of the largest parts (the weights arrive partly
+// ordered: 91,445 -> 89,919 -> 77,236 -> 56,739 ...).  A level-synchronous
+// form in one block is bound by the shared memory's throughput, fifteen accesses
+// per element and level where this one reads each once; one run of 32 positions
+// at a time instead of four costs 101^2 130 us more.
+constexpr int kNrThreads = 512, kNrWarps = kNrThreads / 32, kNrRuns = 4, kNrTail = 7;
+constexpr int kNrQueue = kNrBlock / 8;  // every queued part holds 8 elements of its own
+// positions nr_partition_block lists at a time from either end
+constexpr int kNrEach = 12, kNrSide = kNrEach * kNrThreads;
 struct NrBlockShared {
-  double key[kNrBlock];
-  int id[kNrBlock];                // 1-based edge ids
-  unsigned tail[kNrBlock / 2];     // parts of 2..kNrTail elements: start << 16 | end
-  unsigned queue[kNrQueue];        // parts for any warp: start << 16 | end, kNrEmpty until filled
-  unsigned short at[kNrWarps][2][32 * kNrRuns];  // a warp's stopper positions, left and right
+  union {
+    struct {
+      double key[kNrBlock];
+      int id[kNrBlock];              // 1-based edge ids
+      unsigned tail[kNrBlock / 2];   // parts of 2..kNrTail elements: start << 16 | end
+      unsigned queue[kNrQueue];      // parts for any warp: start << 16 | end, kNrEmpty until filled
+      unsigned short at[kNrWarps][2][32 * kNrRuns];  // a warp's stopper positions, left and right
+    };
+    struct {
+      unsigned short side[2][kNrSide];    // a block's stopper offsets, left and right
+      int runs[kNrEach * kNrWarps + 1];   // stoppers before each warp's run
+    };
+  };
   int head, filled, open, ntail;
+  unsigned long long seg;  // the block's segment: first position, last position << 32
 };
 constexpr unsigned kNrEmpty = 0xffffffffu;
-static_assert(sizeof(NrBlockShared) <= 227 * 1024, "one block per SM");
+static_assert(sizeof(NrBlockShared) <= 48 * 1024, "no opt-in needed");
 
 // Partitions positions l..ir (ir - l >= 7) and returns the parts' borders: [l, j-1] and [i, ir].
 __device__ __forceinline__ void nr_partition_warp(NrBlockShared& S, unsigned short (*at)[32 * kNrRuns], int l, int ir,
@@ -805,45 +838,267 @@ __device__ __forceinline__ void nr_partition_warp(NrBlockShared& S, unsigned sho
   j_out = j;
 }
 
-__global__ void __launch_bounds__(kNrThreads) k_nr_block(const int* __restrict__ nmedp, const int* __restrict__ med,
-                                                         int med_cap, const double* __restrict__ arr,
-                                                         int* __restrict__ idx, int* __restrict__ cnt) {
+// The same by a block, keys and ids in global memory (positions are 1-based).
+// Another block may have written them, so they are read past the L1 cache.
+__device__ __forceinline__ void nr_partition_block(NrBlockShared& S, double* key, int* id, int l, int ir, int& i_out,
+                                                   int& j_out) {
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  unsigned short *const at_l = S.side[0], *const at_r = S.side[1];  // offsets from the listed ends
+  int* const runs = S.runs;
+  if (tid == 0) {
+    auto swap = [&](int x, int y) {
+      const double t = __ldcg(&key[x]), u = __ldcg(&key[y]);
+      const int v = __ldcg(&id[x]), w = __ldcg(&id[y]);
+      key[x] = u; key[y] = t;
+      id[x] = w; id[y] = v;
+    };
+    swap((l + ir) / 2, l + 1);
+    if (__ldcg(&key[l + 1]) > __ldcg(&key[ir])) swap(l + 1, ir);
+    if (__ldcg(&key[l]) > __ldcg(&key[ir])) swap(l, ir);
+    if (__ldcg(&key[l + 1]) > __ldcg(&key[l])) swap(l + 1, l);
+  }
+  __syncthreads();
+  const double a = __ldcg(&key[l]);
+  const unsigned lt = (1u << lane) - 1u;
+  double k[kNrEach];  // the keys of the next listing, if pre says so already loaded
+  int pre = 0;        // 1: the left side's, 2: the right side's
+  auto load = [&](int base, int dir) {
+#pragma unroll
+    for (int r = 0; r < kNrEach; ++r) k[r] = __ldcg(&key[min(max(base + dir * (r * kNrThreads + tid), l), ir)]);
+  };
+  // lists the stoppers among positions base + dir * (0 .. kNrSide - 1); returns their number
+  auto list = [&](int base, int dir, unsigned short* at, auto stops) {
+    bool f[kNrEach];
+    unsigned m[kNrEach];
+#pragma unroll
+    for (int r = 0; r < kNrEach; ++r) {
+      const int q = base + dir * (r * kNrThreads + tid);
+      f[r] = q >= l && q <= ir && stops(q, k[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < kNrEach; ++r) {
+      m[r] = __ballot_sync(0xffffffffu, f[r]);
+      if (lane == 0) runs[r * kNrWarps + wid] = __popc(m[r]);
+    }
+    __syncthreads();
+    if (wid == 0) {  // exclusive prefix over the runs
+      constexpr int kTot = kNrEach * kNrWarps, kPer = (kTot + 31) / 32;
+      int v[kPer], sum = 0;
+#pragma unroll
+      for (int t = 0; t < kPer; ++t) {
+        const int o = lane * kPer + t;
+        v[t] = o < kTot ? runs[o] : 0;
+        sum += v[t];
+      }
+      int x = sum;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      int before = x - sum;
+#pragma unroll
+      for (int t = 0; t < kPer; ++t) {
+        const int o = lane * kPer + t;
+        if (o < kTot) runs[o] = before;
+        before += v[t];
+      }
+      if (lane == 31) runs[kTot] = before;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kNrEach; ++r)
+      if (f[r]) at[runs[r * kNrWarps + wid] + __popc(m[r] & lt)] = (unsigned short)(r * kNrThreads + tid);
+    const int n = runs[kNrEach * kNrWarps];
+    __syncthreads();
+    return n;
+  };
+  int li = l + 2, ri = ir - 1, lb = li, rb = ri;  // next positions to look at; ends of the listed ones
+  int last_l = l, last_r = ir + 1;
+  int nl = 0, ol = 0, nr = 0, orr = 0;
+  int next_l, next_r;
+  for (;;) {
+    while (ol == nl && li < last_r) {
+      lb = li;
+      const int lim = last_r;
+      // keys loaded ahead hold unless the right side has listed some of them since
+      if (pre != 1 || li + kNrSide - 1 > ri) load(li, 1);
+      pre = 0;
+      nl = list(lb, 1, at_l, [&](int q, double v) { return v >= a && q < lim; });
+      ol = 0;
+      li += kNrSide;
+    }
+    while (orr == nr && ri > last_l) {
+      rb = ri;
+      const int lim = last_l;
+      if (pre != 2 || ri - kNrSide + 1 < li) load(ri, -1);
+      pre = 0;
+      nr = list(rb, -1, at_r, [&](int q, double v) { return v <= a && q > lim; });
+      orr = 0;
+      ri -= kNrSide;
+    }
+    next_l = ol < nl ? lb + at_l[ol] : last_r;
+    next_r = orr < nr ? rb - at_r[orr] : last_l;
+    if (next_l >= next_r) break;
+    const int m = min(nl - ol, nr - orr);
+    int cnt = 0;
+    if (nl - ol <= nr - orr && li < last_r) {  // the left side is listed next
+      load(li, 1);
+      pre = 1;
+    } else if (ri > last_l) {
+      load(ri, -1);
+      pre = 2;
+    }
+    constexpr int kPairs = 6;  // exchanges in flight per thread
+    for (int t0 = 0; t0 < m; t0 += kPairs * kNrThreads) {
+      int pl[kPairs], pr[kPairs], vl[kPairs], vr[kPairs];
+      double kl[kPairs], kr[kPairs];
+      bool ex[kPairs];
+#pragma unroll
+      for (int e = 0; e < kPairs; ++e) {
+        const int t = t0 + e * kNrThreads + tid;
+        pl[e] = t < m ? lb + at_l[ol + t] : 0;
+        pr[e] = t < m ? rb - at_r[orr + t] : 0;
+        ex[e] = pl[e] < pr[e];
+        if (ex[e]) {
+          kl[e] = __ldcg(&key[pl[e]]);
+          kr[e] = __ldcg(&key[pr[e]]);
+          vl[e] = __ldcg(&id[pl[e]]);
+          vr[e] = __ldcg(&id[pr[e]]);
+        }
+      }
+      int c = 0;
+#pragma unroll
+      for (int e = 0; e < kPairs; ++e) {
+        if (ex[e]) {
+          key[pl[e]] = kr[e];
+          key[pr[e]] = kl[e];
+          id[pl[e]] = vr[e];
+          id[pr[e]] = vl[e];
+        }
+        c += __syncthreads_count(ex[e]);
+      }
+      cnt += c;
+      if (c < kPairs * kNrThreads) break;
+    }
+    ol += cnt;
+    orr += cnt;
+    last_l = lb + at_l[ol - 1];
+    last_r = rb - at_r[orr - 1];
+    __syncthreads();  // the lists are read before they are written anew
+  }
+  int i = min(next_l, last_r), j = max(next_r, last_l);
+  if (ol < nl && orr < nr && next_l == next_r) {
+    i = next_l + 1;
+    j = next_l - 1;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    const int v = __ldcg(&id[l]);
+    key[l] = __ldcg(&key[j]);
+    id[l] = __ldcg(&id[j]);
+    key[j] = a;
+    id[j] = v;
+  }
+  __syncthreads();
+  i_out = i;
+  j_out = j;
+}
+
+// Takes the next filled slot of a queue; -1 when every part is done.  A slot
+// is taken only once it is filled, so a waiter may leave at any time.
+__device__ __forceinline__ int nr_take(int* head, int* filled, int* open, int cap, int rest_ns) {
+  for (int spins = 0; spins < kSpinLimit; ++spins) {
+    const int h = *(volatile int*)head;
+    if (h < min(*(volatile int*)filled, cap)) {
+      if (atomicCAS(head, h, h + 1) == h) return h;
+      continue;
+    }
+    if (*(volatile int*)open <= 0) break;
+    __nanosleep(rest_ns);
+  }
+  return -1;
+}
+// the slot's part: written right after the slot was counted
+template <class P>
+__device__ __forceinline__ P nr_read_slot(const P* slot, P empty, int* overflow) {
+  for (int spins = 0; spins < kSpinLimit; ++spins) {
+    const P v = *(const volatile P*)slot;
+    if (v != empty) return v;
+  }
+  atomicExch(overflow, 1);
+  return empty;
+}
+
+__global__ void __launch_bounds__(kNrThreads) k_nr_block(unsigned long long* __restrict__ med, int med_cap,
+                                                            double* key, int* idx, int* cnt) {
   extern __shared__ __align__(16) unsigned char nr_smem[];
   NrBlockShared& S = *reinterpret_cast<NrBlockShared*>(nr_smem);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int nmed = min(*nmedp, med_cap);
-  for (int m = blockIdx.x; m < nmed; m += gridDim.x) {
-    const int base = med[2 * m], n = med[2 * m + 1] - base + 1;
-    if (n < 8 || n > kNrBlock) {  // never: nr_newsegs_one routes only such segments here
-      if (tid == 0) atomicExch(&cnt[C_OVERFLOW], 1);
-      continue;
+  for (;;) {
+    if (tid == 0) {
+      S.seg = 0;
+      const int slot = nr_take(&cnt[C_NRHEAD], &cnt[C_NMED], &cnt[C_NROPEN], med_cap, 200);
+      if (slot >= 0) S.seg = nr_read_slot(&med[slot], 0ull, &cnt[C_OVERFLOW]);
+      __threadfence();
     }
+    __syncthreads();
+    int base = (int)(unsigned)S.seg, last = (int)(S.seg >> 32);  // first and last position, low word first
+    __syncthreads();
+    if (base == 0) break;
+    while (last - base >= kNrBlock) {
+      int i, j;
+      nr_partition_block(S, key, idx, base, last, i, j);
+      int al = base, ae = j - 1, bl = i, be = last;
+      if (ae - al < be - bl) {
+        al = i; ae = last; bl = base; be = j - 1;
+      }
+      if (tid == 0) {
+        if (be - bl >= 7) {
+          __threadfence();
+          atomicAdd(&cnt[C_NROPEN], 1);
+          const int f = atomicAdd(&cnt[C_NMED], 1);
+          if (f < med_cap) *(volatile unsigned long long*)&med[f] = (unsigned long long)be << 32 | (unsigned)bl;
+          else atomicExch(&cnt[C_OVERFLOW], 1);  // never: every queued part holds 8 elements of its own
+        } else {
+          for (int q = bl + 1; q <= be; ++q) {  // straight insertion (LocalMinima.f90:967-976)
+            const double a = __ldcg(&key[q]);
+            const int v = __ldcg(&idx[q]);
+            int p = q - 1;
+            for (; p >= bl; --p) {
+              const double b = __ldcg(&key[p]);
+              if (b <= a) break;
+              key[p + 1] = b;
+              idx[p + 1] = __ldcg(&idx[p]);
+            }
+            key[p + 1] = a;
+            idx[p + 1] = v;
+          }
+        }
+      }
+      base = al;
+      last = ae;
+      __syncthreads();
+    }
+    const int n = last - base + 1;
     for (int p = tid; p < n; p += kNrThreads) {
-      const int e = idx[base + p];
-      S.id[p] = e;
-      S.key[p] = arr[e];
+      S.id[p] = __ldcg(&idx[base + p]);
+      S.key[p] = __ldcg(&key[base + p]);
     }
     for (int p = tid; p < kNrQueue; p += kNrThreads) S.queue[p] = p == 0 && n > kNrTail ? (unsigned)(n - 1) : kNrEmpty;
     if (tid == 0) {
       S.head = 0;
-      S.filled = 1;
+      S.filled = n > kNrTail ? 1 : 0;
       S.open = n > kNrTail ? 1 : 0;  // parts queued or in work
       S.ntail = n > kNrTail ? 0 : 1;
       S.tail[0] = (unsigned)(n - 1);
     }
     __syncthreads();
-    // every warp claims a queue slot and waits until it is filled or all parts are done
     for (;;) {
-      int slot = 0;
-      if (lane == 0) slot = atomicAdd(&S.head, 1);
-      slot = __shfl_sync(0xffffffffu, slot, 0);
       unsigned part = kNrEmpty;
-      if (lane == 0 && slot < kNrQueue)
-        for (;;) {
-          part = *(volatile unsigned*)&S.queue[slot];
-          if (part != kNrEmpty || *(volatile int*)&S.open == 0) break;
-          __nanosleep(20);
-        }
+      if (lane == 0) {
+        const int slot = nr_take(&S.head, &S.filled, &S.open, kNrQueue, 20);
+        if (slot >= 0) part = nr_read_slot(&S.queue[slot], kNrEmpty, &cnt[C_OVERFLOW]);
+      }
       part = __shfl_sync(0xffffffffu, part, 0);
       if (part == kNrEmpty) break;
       __threadfence_block();
@@ -876,13 +1131,33 @@ __global__ void __launch_bounds__(kNrThreads) k_nr_block(const int* __restrict__
       if (lane == 0) atomicSub(&S.open, 1);
     }
     __syncthreads();
-    for (int t = tid; t < S.ntail; t += kNrThreads) {
-      const int l = (int)(S.tail[t] >> 16), len = (int)(S.tail[t] & 0xffffu) - l + 1;
-      if (!nr_sort_local(S.key + l, S.id + l, len)) atomicExch(&cnt[C_OVERFLOW], 1);
+    // parts of up to seven elements: straight insertion is a stable sort, so an
+    // element's place is the number of those that belong before it; eight
+    // lanes per part
+    for (int t0 = wid * 4; t0 < S.ntail; t0 += kNrWarps * 4) {
+      const int t = t0 + (lane >> 3), e = lane & 7;
+      const unsigned part = t < S.ntail ? S.tail[t] : 0u;
+      const int l = (int)(part >> 16), len = t < S.ntail ? (int)(part & 0xffffu) - l + 1 : 0;
+      const bool in = e < len;
+      const double v = in ? S.key[l + e] : 0.0;
+      const int id = in ? S.id[l + e] : 0;
+      int before = 0;
+#pragma unroll
+      for (int o = 0; o < 7; ++o) {
+        const double w = __shfl_sync(0xffffffffu, v, o, 8);
+        before += o < len && (w < v || (w == v && o < e));
+      }
+      const unsigned odd = __ballot_sync(0xffffffffu, v != v);  // a NaN has no place by counting
+      if ((odd >> (lane & 24)) & 0xffu) {
+        if (e == 0 && !nr_sort_local(S.key + l, S.id + l, len)) atomicExch(&cnt[C_OVERFLOW], 1);
+      } else if (in) {
+        S.id[l + before] = id;
+      }
     }
     __syncthreads();
     for (int p = tid; p < n; p += kNrThreads) idx[base + p] = S.id[p];
     __syncthreads();
+    if (tid == 0) atomicSub(&cnt[C_NROPEN], 1);
   }
 }
 
@@ -1267,10 +1542,13 @@ static bool nr_indexx(Ctx& c, int n, const double* w) {
   int* seg = c.nr_seg;
   int* seg2 = c.nr_seg2;
   const int small_cap = (int)(c.conn_cap / 2 + 8);
-  k_nr_init<<<grid1d(n + 2), kBlock, 0, c.stream>>>(n, idx, c.nr_segof, seg, c.nr_small, c.nr_med, c.d_cnt);
+  double* key = c.r_w - 1;  // 1-based; the edges' unsorted weights are not needed any more
+  const int med_cap = nr_med_cap(c);
+  cudaMemsetAsync(c.nr_med, 0, 2 * sizeof(int) * (size_t)std::min(n / 8 + 8, med_cap), c.stream);  // empty slots
+  k_nr_init<<<grid1d(n + 2), kBlock, 0, c.stream>>>(n, arr, idx, key, c.nr_segof, seg, c.nr_small, c.nr_med, c.d_cnt);
   c.count_launch();
-  int nseg = 1;  // k_nr_init makes one segment of the whole array when n > kNrBlock
-  if (n <= kNrBlock) {  // k_nr_init made one segment of it: what it counted is known
+  int nseg = 1;  // k_nr_init makes one segment of the whole array when n > kNrSplit
+  if (n <= kNrSplit) {  // k_nr_init made one segment of it: what it counted is known
     nseg = 0;
     c.h_cnt[C_NMED] = n >= 8 ? 1 : 0;
     c.h_cnt[C_NSMALL] = n >= 2 && n < 8 ? 1 : 0;
@@ -1313,16 +1591,15 @@ static bool nr_indexx(Ctx& c, int n, const double* w) {
     nseg = c.h_cnt[in];
     if (c.h_cnt[C_OVERFLOW]) { c.err = "NR sort emulation: small-segment buffer overflow"; return false; }
   }
-  const int nmed = c.h_cnt[C_NMED];
-  if (nmed > 0) {
-    const int* nmedp = c.d_cnt + C_NMED;
-    int cap = nr_med_cap(c);
-    void* args[] = {&nmedp, &c.nr_med, &cap, &arr, &idx, &c.d_cnt};
-    if (!BigSmem<k_nr_block>::launch(std::min(nmed, 148), kNrThreads, sizeof(NrBlockShared), (int)sizeof(NrBlockShared),
-                                     c.stream, args)) {
-      c.err = "NR sort emulation: a block's shared memory is not available";
-      return false;
+  if (c.h_cnt[C_NMED] > 0) {
+    if (n > kNrSplit) {
+      k_nr_keys<<<grid1d(n), kBlock, 0, c.stream>>>(n, arr, idx, key, c.d_cnt);
+      c.count_launch();
     }
+    // half of kNrBlock elements per block, at most what is resident at once
+    const int blocks = std::max(1, std::min(n / (kNrBlock / 2 * c.launch_share), 148));
+    k_nr_block<<<blocks, kNrThreads, sizeof(NrBlockShared), c.stream>>>(
+        reinterpret_cast<unsigned long long*>(c.nr_med), med_cap, key, idx, c.d_cnt);
     c.count_launch();
   }
   const int nsmall = c.h_cnt[C_NSMALL];

@@ -39,3 +39,9 @@ def test_sort_permutation(side, levels):
         assert np.array_equal(dg[k], do[k]), k
     assert np.array_equal(g.copy_int("rec"), O.copy_int("rec"))
     g.destroy()
+
+
+@pytest.mark.parametrize("side", [200, 560, 900])  # edges: below and above one block's partition
+@pytest.mark.parametrize("levels", [0, 40])
+def test_sort_permutation_of_block_partitions(side, levels):
+    test_sort_permutation(side, levels)
