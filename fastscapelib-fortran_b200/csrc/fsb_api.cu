@@ -123,9 +123,12 @@ size_t layout(fsb::Ctx& c, char* base) {
   c.s_flag = L.take<int>(N + 1); c.s_scan = L.take<int>(N + 1); c.s_roots = L.take<int>(N);
   c.s_root_rank = L.take<int>(N);
   c.s_list_a = L.take<unsigned long long>(2 * N); c.s_list_b = L.take<unsigned long long>(2 * N);
-  c.s_rank_ws = L.take<unsigned long long>(fsb::rank_scratch(2 * N));
+  const size_t paths = fsb::tour_elements(c.nx, c.ny);
+  c.s_tour = L.take<unsigned long long>(paths); c.s_tour_sub = L.take<unsigned long long>(paths);
+  c.s_tour_weight = L.take<unsigned>(paths);
+  c.s_rank_ws = L.take<unsigned long long>(fsb::rank_scratch(std::max(2 * N, paths)));
   c.s_rank_nheads = L.take<unsigned>(1);
-  c.s_rank_pred = L.take<unsigned char>(2 * N + 16);  // whole 16-byte flag groups
+  c.s_rank_pred = L.take<unsigned char>(std::max(2 * N, paths) + 16);  // whole 16-byte flag groups
   c.ht_key = L.take<unsigned long long>(hcap); c.ht_wmin = L.take<unsigned long long>(hcap);
   c.ht_first = L.take<unsigned>(hcap); c.ht_best = L.take<unsigned>(hcap);
   c.e_b1 = L.take<int>(E); c.e_b2 = L.take<int>(E); c.e_n1 = L.take<int>(E); c.e_n2 = L.take<int>(E);

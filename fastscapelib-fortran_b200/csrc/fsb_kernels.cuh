@@ -95,6 +95,8 @@ struct Ctx {
   unsigned long long *s_list_a = nullptr, *s_list_b = nullptr;  // 2*nn each
   // list ranking by sublist walks: predecessor flags (2*nn bytes), the shorter
   // lists and the count of list heads
+  unsigned long long *s_tour = nullptr, *s_tour_sub = nullptr;  // the tour's paths (tour_elements) and their walks
+  unsigned* s_tour_weight = nullptr;
   unsigned char* s_rank_pred = nullptr;
   unsigned long long* s_rank_ws = nullptr;
   unsigned* s_rank_nheads = nullptr;
@@ -225,6 +227,11 @@ unsigned long long* list_rank(Ctx& c, size_t n, unsigned long long* a, unsigned 
 // list ranking by sublist walks: a splitter every 16 or 4 entries plus each
 // list head (at most kRankMaxHeads heads); a block ranks up to kRankBlock entries
 constexpr int kRankMaxHeads = 4, kRankBlock = 8192;
+// tiles of the Euler tour and list elements per tile (fsb_routing.cu)
+constexpr int kTourTileX = 64, kTourTileY = 32, kTourSlots = 768;
+inline size_t tour_elements(int nx, int ny) {
+  return (size_t)((nx + kTourTileX - 1) / kTourTileX) * ((ny + kTourTileY - 1) / kTourTileY) * kTourSlots;
+}
 // scratch entries below a list of n: per level its splitters and their walk's results
 inline size_t rank_scratch(size_t n) {
   size_t total = 0;
