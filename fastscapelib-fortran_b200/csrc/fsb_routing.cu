@@ -80,7 +80,28 @@ __global__ void k_find_donors(Bounds bd, const int* __restrict__ rec, int* __res
   const int nx = bd.nx, ny = bd.ny;
   const int nn = nx * ny;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
-    const int i = k % nx, j = k / nx;
+    const int j = k / nx, i = k - j * nx;
+    if (i > 0 && i < nx - 1 && j > 0 && j < ny - 1) {  // the neighbours in ascending order
+      const int q[8] = {k - nx - 1, k - nx, k - nx + 1, k - 1, k + 1, k + nx - 1, k + nx, k + nx + 1};
+      int r[8], d[8], n = 0;
+#pragma unroll
+      for (int t = 0; t < 8; ++t) r[t] = rec[q[t]];
+#pragma unroll
+      for (int t = 0; t < 8; ++t) d[t] = -1;
+#pragma unroll
+      for (int t = 0; t < 8; ++t)
+        if (r[t] == k) {
+#pragma unroll
+          for (int u = 0; u <= t; ++u)
+            if (u == n) d[u] = q[t];
+          ++n;
+        }
+      ndon[k] = n;
+      int4* row = reinterpret_cast<int4*>(don + (size_t)k * 8);
+      row[0] = make_int4(d[0], d[1], d[2], d[3]);
+      row[1] = make_int4(d[4], d[5], d[6], d[7]);
+      continue;
+    }
     int cand[8];
     int nc = 0;
     // Distinct neighbours in the wrapped 3x3 block (rows/columns that fall off
