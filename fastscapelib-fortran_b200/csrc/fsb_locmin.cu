@@ -35,8 +35,7 @@ enum {
   C_NBASINS = 0, C_NLOCMIN = 1, C_BASIN0 = 2, C_NEDGE = 3, C_NSEG = 4, C_NSMALL = 5,
   C_CHANGED = 6, C_NTREE = 7, C_NLOCMIN_AFTER = 8, C_OVERFLOW = 9, C_NSEG2 = 11,
   C_NRIDX = 12, C_NRLEVELS = 13, C_NMED = 14, C_NRHEAD = 15, C_NROPEN = 16,
-  C_MST_CHANGED = 24, C_MST_FLAT = 25,  // 25..27: the cooperative MST's rotating flags
-  C_MST_DONE = 28                        // host-driven MST: a round changed nothing
+  C_MST_DONE = 28  // host-driven MST: a round changed nothing
 };
 constexpr int kNrCounters = 15;  // counters the NR sort reads back
 
@@ -91,19 +90,48 @@ __global__ void k_basins(int nn, const int* __restrict__ stack, const int* __res
 // active roots (local minima) and basin0 = first basin whose root is on a fixed boundary
 // the root count comes from cnt[C_NBASINS] (set on the device), so that one
 // read-back brings the basins, the pits and basin0 together
-__global__ void k_roots_scan(Bounds bd, const int* __restrict__ roots, int* cnt) {
+__global__ void k_roots_scan(Bounds bd, const int* __restrict__ roots, unsigned char* __restrict__ open, int* cnt) {
   const int nroots = cnt[C_NBASINS];
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nroots; r += gridDim.x * blockDim.x) {
     const int k = roots[r];
-    if (is_bc_node(bd, k % bd.nx, k / bd.nx)) atomicMin(&cnt[C_BASIN0], r + 1);
+    const bool bc = is_bc_node(bd, k % bd.nx, k / bd.nx);
+    open[r] = bc;
+    if (bc) atomicMin(&cnt[C_BASIN0], r + 1);
     else atomicAdd(&cnt[C_NLOCMIN], 1);
   }
 }
 
 // ---- connect_basins ------------------------------------------------------
+// Open addressing.  A pair (b, nb) has its place in the kPairSlots slots of basin
+// b, in order, so that the pairs of neighbouring basins share cache lines (basin
+// ids follow their roots' rows), and when they are taken (basins with many
+// neighbours) in the first free slot from a mixed position on.  A basin's slots
+// are read at once.  Nothing is ever removed: a slot seen taken stays so.
+// Measured (B200, 2049^2, 1.5e6 pairs): both passes and the list 709 us with
+// mixed positions only in twice the slots, 500 now (list 240 -> 45).
+constexpr int kPairSlots = 8;
+__device__ __forceinline__ size_t ht_own(size_t cap, unsigned long long key) {
+  return ((size_t)(key >> 32) * kPairSlots) & (cap - 1);
+}
+// the position of the key or of the first free slot among the basin's slots, or kPairSlots
+__device__ __forceinline__ int ht_look(const unsigned long long* own, unsigned long long key) {
+  int at = kPairSlots;
+#pragma unroll
+  for (int t = 0; t < kPairSlots; t += 2) {
+    const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(own + t);  // a stale free slot only costs a try
+    if (at == kPairSlots && (k.x == key || k.x == ~0ull)) at = t;
+    if (at == kPairSlots && (k.y == key || k.y == ~0ull)) at = t + 1;
+  }
+  return at;
+}
 __device__ inline unsigned ht_insert(unsigned long long* keys, size_t cap, unsigned long long key) {
+  const size_t own = ht_own(cap, key);
+  for (int t = ht_look(keys + own, key); t < kPairSlots; ++t) {
+    const unsigned long long old = atomicCAS(&keys[own + t], ~0ull, key);
+    if (old == ~0ull || old == key) return (unsigned)(own + t);
+  }
   size_t s = mix64(key) & (cap - 1);
-  const size_t limit = cap < 4096 ? cap : 4096;  // load stays below 1/2: long probes mean overflow
+  const size_t limit = cap < 4096 ? cap : 4096;  // load stays below 3/4: long probes mean overflow
   for (size_t probe = 0; probe < limit; ++probe) {
     const unsigned long long old = atomicCAS(&keys[s], ~0ull, key);
     if (old == ~0ull || old == key) return (unsigned)s;
@@ -113,6 +141,9 @@ __device__ inline unsigned ht_insert(unsigned long long* keys, size_t cap, unsig
 }
 
 __device__ inline unsigned ht_find(const unsigned long long* keys, size_t cap, unsigned long long key) {
+  const size_t own = ht_own(cap, key);
+  const int t = ht_look(keys + own, key);
+  if (t < kPairSlots) return keys[own + t] == key ? (unsigned)(own + t) : 0xffffffffu;
   size_t s = mix64(key) & (cap - 1);
   const size_t limit = cap < 4096 ? cap : 4096;
   for (size_t probe = 0; probe < limit; ++probe) {
@@ -126,18 +157,19 @@ __device__ inline unsigned ht_find(const unsigned long long* keys, size_t cap, u
 
 // pass 0: insert pairs, min weight, first discovery; pass 1: earliest
 // discovery among the minimum-weight candidates of each pair.
+// open[b - 1]: basin b ends at a fixed boundary, kept per basin instead of told
+// from the root with two divisions per neighbour (2049^2: 510 -> 450 us both).
 template <int PASS>
-__global__ void k_conn_pass(Bounds bd, const int* __restrict__ basins, const int* __restrict__ roots,
+__global__ void k_conn_pass(Bounds bd, const int* __restrict__ basins, const unsigned char* __restrict__ open,
                             const int* __restrict__ pos, const double* __restrict__ h,
-                            unsigned long long* __restrict__ ht_key, unsigned long long* __restrict__ ht_wmin,
-                            unsigned* __restrict__ ht_first, unsigned* __restrict__ ht_best, size_t cap,
+                            unsigned long long* ht_key, unsigned long long* ht_wmin,
+                            unsigned* ht_first, unsigned* ht_best, size_t cap,
                             int* __restrict__ cnt) {
   const int nx = bd.nx, ny = bd.ny, nn = nx * ny;
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < nn; p += gridDim.x * blockDim.x) {
     const int b = basins[p];
-    const int outlet = roots[b - 1];
-    if (is_bc_node(bd, outlet % nx, outlet / nx)) continue;  // inactive basin: not scanned
-    const int i = p % nx, j = p / nx;
+    if (open[b - 1]) continue;  // inactive basin: not scanned
+    const int j = p / nx, i = p - j * nx;
     const double hp = h[p];
     const unsigned disc0 = (unsigned)pos[p] * 8u;
     for (int k = 0; k < 8; ++k) {
@@ -145,20 +177,23 @@ __global__ void k_conn_pass(Bounds bd, const int* __restrict__ basins, const int
       if (ki < 0 || ki >= nx || kj < 0 || kj >= ny) continue;
       const int q = ki + kj * nx;
       const int nb = basins[q];
-      const int nbo = roots[nb - 1];
-      if (b >= nb && !is_bc_node(bd, nbo % nx, nbo / nx)) continue;
+      if (nb == b) continue;
+      if (b > nb && !open[nb - 1]) continue;
       const double w = fmax(hp, h[q]);
       const unsigned long long key = ((unsigned long long)b << 32) | (unsigned)nb;
       const unsigned disc = disc0 + (unsigned)k;
       if (PASS == 0) {
         const unsigned s = ht_insert(ht_key, cap, key);
         if (s == 0xffffffffu) { atomicExch(&cnt[C_OVERFLOW], 1); continue; }
-        atomicMin(&ht_wmin[s], ordered_u64(w));
-        atomicMin(&ht_first[s], disc);
+        // the minima only fall, so a stale value in the L1 cache can only call for
+        // an atomic that was not needed
+        const unsigned long long o = ordered_u64(w);
+        if (o < ht_wmin[s]) atomicMin(&ht_wmin[s], o);
+        if (disc < ht_first[s]) atomicMin(&ht_first[s], disc);
       } else {
         const unsigned s = ht_find(ht_key, cap, key);
         if (s == 0xffffffffu) continue;
-        if (ordered_u64(w) == ht_wmin[s]) atomicMin(&ht_best[s], disc);
+        if (ordered_u64(w) == ht_wmin[s] && disc < ht_best[s]) atomicMin(&ht_best[s], disc);
       }
     }
   }
@@ -170,11 +205,43 @@ __global__ void k_conn_compact(Bounds bd, size_t cap, const unsigned long long* 
                                unsigned* __restrict__ r_key, int* __restrict__ r_b1, int* __restrict__ r_b2,
                                int* __restrict__ r_n1, int* __restrict__ r_n2, double* __restrict__ r_w,
                                int* __restrict__ cnt) {
-  const int nx = bd.nx;
-  for (size_t s = blockIdx.x * (size_t)blockDim.x + threadIdx.x; s < cap; s += (size_t)gridDim.x * blockDim.x) {
-    const unsigned long long key = ht_key[s];
+  // a block counts the pairs of kEach slots per thread before it asks for their places
+  constexpr int kEach = 4;
+  __shared__ int warps[kBlock / 32], base;
+  const int nx = bd.nx, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  unsigned long long keys[kEach];
+  const size_t s0 = (size_t)blockIdx.x * kBlock * kEach + threadIdx.x;
+  int mine = 0;
+#pragma unroll
+  for (int t = 0; t < kEach; ++t) {
+    const size_t s = s0 + (size_t)t * kBlock;
+    keys[t] = s < cap ? ht_key[s] : ~0ull;
+    mine += keys[t] != ~0ull;
+  }
+  int x = mine;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) warps[wid] = x;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int sum = 0;
+    for (int w = 0; w < kBlock / 32; ++w) {
+      const int v = warps[w];
+      warps[w] = sum;
+      sum += v;
+    }
+    base = sum ? atomicAdd(&cnt[C_NEDGE], sum) : 0;
+  }
+  __syncthreads();
+  int at = base + warps[wid] + x - mine;
+#pragma unroll
+  for (int t = 0; t < kEach; ++t) {
+    const unsigned long long key = keys[t];
     if (key == ~0ull) continue;
-    const int idx = atomicAdd(&cnt[C_NEDGE], 1);
+    const size_t s = s0 + (size_t)t * kBlock;
+    const int idx = at++;
     if ((size_t)idx >= conn_cap) { atomicExch(&cnt[C_OVERFLOW], 1); continue; }
     const unsigned best = ht_best[s];
     if (best == 0xffffffffu) { atomicExch(&cnt[C_OVERFLOW], 1); continue; }
@@ -1171,19 +1238,19 @@ __global__ void k_mst_init(int nb, int* __restrict__ comp) {
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) comp[b] = b;
 }
 
-// Host-driven Borůvka rounds (graphs above kMstCoopMax edges).  Rounds are
-// launched in batches without a read-back in between: once a round's hooking
-// changes nothing, k_mst_check sets C_MST_DONE and every later kernel of the
-// batch returns at once.
-__global__ void k_mst_reset(int nb, int* __restrict__ mn, const int* __restrict__ done) {
-  if (*done) return;
+// Host-driven Borůvka rounds (where a cooperative launch is refused), three
+// kernels each, launched in batches without a read-back in between: once a round's
+// hooking changes nothing, k_mst_compress sets C_MST_DONE and every later kernel
+// of the batch returns at once.
+__global__ void k_mst_reset(int nb, int* __restrict__ mn) {
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) mn[b] = INT_MAX;
 }
 
 __global__ void k_mst_minedge(int ne, const int* __restrict__ b1, const int* __restrict__ b2,
                               const int* __restrict__ rank, const int* __restrict__ comp, int* __restrict__ mn,
-                              const int* __restrict__ done) {
-  if (*done) return;
+                              int* __restrict__ cnt) {
+  if (cnt[C_MST_DONE]) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) cnt[C_CHANGED] = 0;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += gridDim.x * blockDim.x) {
     const int cu = comp[b1[e] - 1], cv = comp[b2[e] - 1];
     if (cu == cv) continue;
@@ -1196,6 +1263,7 @@ __global__ void k_mst_hook(int nb, const int* __restrict__ idx1, const int* __re
                            const int* __restrict__ b2, const int* __restrict__ comp, const int* __restrict__ mn,
                            int* __restrict__ next, int* __restrict__ inmst, int* __restrict__ cnt) {
   if (cnt[C_MST_DONE]) return;
+  bool changed = false;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nb; c += gridDim.x * blockDim.x) {
     next[c] = comp[c];
     if (comp[c] != c) continue;
@@ -1207,53 +1275,43 @@ __global__ void k_mst_hook(int nb, const int* __restrict__ idx1, const int* __re
     inmst[e] = 1;
     if (mn[other] == r && c < other) continue;  // mutual choice: the smaller id stays a root
     next[c] = other;
-    cnt[C_CHANGED] = 1;
+    changed = true;
   }
+  // one store per block: one per thread to the same word was most of the time
+  // (2049^2's first round 123 us)
+  if (__syncthreads_or(changed) && threadIdx.x == 0) cnt[C_CHANGED] = 1;
 }
 
-// one thread: a round whose hooking changed nothing ends the MST
-__global__ void k_mst_check(int* cnt) {
+// The root of c in the hook forest.  Every thread moves its pointer to its
+// grandparent until it reaches a root; other threads' updates only move
+// pointers towards the roots (which never change here), so the walk is
+// bounded by the number of components.
+__device__ __forceinline__ int mst_root(volatile int* next, int c, int nb, int* cnt) {
+  int r = next[c];
+  for (int it = 0; it <= nb; ++it) {
+    const int rr = next[r];
+    if (rr == r) return r;
+    next[c] = rr;
+    r = rr;
+  }
+  atomicExch(&cnt[C_OVERFLOW], 1);
+  return r;
+}
+
+__global__ void k_mst_compress(int nb, int* next, int* __restrict__ comp, int* __restrict__ mn, int* cnt) {
   if (cnt[C_MST_DONE]) return;
-  if (!cnt[C_CHANGED]) cnt[C_MST_DONE] = 1;
-  cnt[C_CHANGED] = 0;
-}
-
-__global__ void k_mst_apply(int nb, const int* __restrict__ next, int* __restrict__ comp,
-                            const int* __restrict__ done) {
-  if (*done) return;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nb; c += gridDim.x * blockDim.x) comp[c] = next[c];
-}
-
-// Flattens the hook forest in one launch: each thread moves its pointer to
-// its grandparent until it reaches a root.  Other threads' updates only move
-// pointers towards the roots (which never change here), so every thread ends
-// at its root; the loop is bounded by the number of components.
-__global__ void k_mst_flatten(int nb, int* comp, int* cnt) {
-  if (*(volatile int*)&cnt[C_MST_DONE]) return;
-  volatile int* vc = comp;
+  if (!cnt[C_CHANGED]) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) cnt[C_MST_DONE] = 1;
+    return;
+  }
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nb; c += gridDim.x * blockDim.x) {
-    int it = 0;
-    for (;; ++it) {
-      const int r = vc[c];
-      const int rr = vc[r];
-      if (rr == r) break;
-      if (it > nb) {  // not a forest
-        atomicExch(&cnt[C_OVERFLOW], 1);
-        break;
-      }
-      vc[c] = rr;
-    }
+    comp[c] = mst_root(next, c, nb, cnt);
+    mn[c] = INT_MAX;
   }
 }
 
-// All Borůvka rounds in one cooperative launch (the kernels above, as phases
-// separated by grid-wide barriers), so that no round waits for the host.
-// Flattening jumps in place: comp[c] <- comp[comp[c]] only ever moves a
-// pointer towards its root, so concurrent updates leave the same roots.  A
-// pass's "not flat" flag is one of three slots used in turn: the slot a pass
-// sets was cleared two barriers earlier, after every thread had read it.
-// Rounds and passes are bounded (64 each, as the host loop); a flatten that
-// does not end sets the overflow counter.
+// Borůvka in one cooperative launch: minimum edges, hooking, compression, a
+// grid-wide barrier after each.  Rounds are bounded (64, as the host loop).
 struct MstCoop {
   int nb, ne;
   const int *idx1, *b1, *b2, *rank;
@@ -1265,68 +1323,50 @@ __global__ void __launch_bounds__(kCoopThreads) k_mst_coop(MstCoop A) {
   cg::grid_group grid = cg::this_grid();
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int nthreads = gridDim.x * blockDim.x;
-  volatile int* comp = A.comp;
-  for (int c = tid; c < A.nb; c += nthreads) comp[c] = c;
+  for (int c = tid; c < A.nb; c += nthreads) {
+    A.comp[c] = c;
+    A.mn[c] = INT_MAX;
+  }
+  grid.sync();
   for (int round = 0; round < 64; ++round) {
-    for (int c = tid; c < A.nb; c += nthreads) A.mn[c] = INT_MAX;
-    if (tid == 0) {
-      A.cnt[C_MST_CHANGED] = 0;
-      A.cnt[C_MST_FLAT] = 0;
-    }
-    grid.sync();
+    if (tid == 0) A.cnt[C_CHANGED] = 0;
     for (int e = tid; e < A.ne; e += nthreads) {
-      const int cu = comp[A.b1[e] - 1], cv = comp[A.b2[e] - 1];
+      const int cu = __ldcg(&A.comp[A.b1[e] - 1]), cv = __ldcg(&A.comp[A.b2[e] - 1]);
       if (cu == cv) continue;
       atomicMin(&A.mn[cu], A.rank[e]);
       atomicMin(&A.mn[cv], A.rank[e]);
     }
     grid.sync();
+    bool changed = false;
     for (int c = tid; c < A.nb; c += nthreads) {
-      A.next[c] = comp[c];
-      if (comp[c] != c) continue;
+      const int own = __ldcg(&A.comp[c]);
+      A.next[c] = own;
+      if (own != c) continue;
       const int r = __ldcg(&A.mn[c]);
       if (r == INT_MAX) continue;
       const int e = A.idx1[r + 1] - 1;
-      const int cu = comp[A.b1[e] - 1], cv = comp[A.b2[e] - 1];
+      const int cu = __ldcg(&A.comp[A.b1[e] - 1]), cv = __ldcg(&A.comp[A.b2[e] - 1]);
       const int other = cu == c ? cv : cu;
       A.inmst[e] = 1;
       if (__ldcg(&A.mn[other]) == r && c < other) continue;  // mutual choice: the smaller id stays a root
       A.next[c] = other;
-      A.cnt[C_MST_CHANGED] = 1;
+      changed = true;
+    }
+    if (__syncthreads_or(changed) && threadIdx.x == 0) A.cnt[C_CHANGED] = 1;
+    grid.sync();
+    if (__ldcg(&A.cnt[C_CHANGED]) == 0) break;  // read by every thread after the barrier
+    for (int c = tid; c < A.nb; c += nthreads) {
+      A.comp[c] = mst_root(A.next, c, A.nb, A.cnt);
+      A.mn[c] = INT_MAX;
     }
     grid.sync();
-    if (__ldcg(&A.cnt[C_MST_CHANGED]) == 0) break;  // read by every thread after the barrier
-    for (int c = tid; c < A.nb; c += nthreads) comp[c] = __ldcg(&A.next[c]);
-    grid.sync();
-    bool flat = false;
-    for (int pass = 0; pass < 64; ++pass) {
-      volatile int* fl = A.cnt + C_MST_FLAT + pass % 3;
-      if (tid == 0) A.cnt[C_MST_FLAT + (pass + 1) % 3] = 0;
-      for (int c = tid; c < A.nb; c += nthreads) {
-        const int r = comp[c];
-        const int rr = comp[r];
-        if (rr != r) {
-          comp[c] = rr;
-          *fl = 1;
-        }
-      }
-      grid.sync();
-      if (*fl == 0) {
-        flat = true;
-        break;
-      }
-    }
-    if (!flat) {
-      if (tid == 0) A.cnt[C_OVERFLOW] = 1;
-      break;
-    }
   }
 }
 
 // The same rounds in one block, components in shared memory, for graphs of at
 // most kMstBlockRoots basins and kMstBlockEdges edges: a block barrier costs
 // 40 ns, a grid-wide one several us (101^2, 1,000 basins: 148 -> 29 us).
-constexpr int kMstBlockRoots = 8192, kMstBlockEdges = 32768, kMstThreads = 512;
+constexpr int kMstBlockRoots = 2048, kMstBlockEdges = 8192, kMstThreads = 512;
 __global__ void __launch_bounds__(kMstThreads) k_mst_block(MstCoop A) {
   extern __shared__ int mst_sh[];
   int *comp = mst_sh, *mn = mst_sh + A.nb, *next = mst_sh + 2 * A.nb;
@@ -1612,25 +1652,17 @@ static bool nr_indexx(Ctx& c, int n, const double* w) {
   return true;
 }
 
-// Borůvka in one launch (a block's, or a cooperative one); false when the device refuses it or the
-// graph is large (the host-driven rounds run instead).  Measured on B200: the
-// cooperative form saves the rounds' read-backs (1025^2 grid, 3.7e5 edges:
-// LocalMinima 3.12 -> 2.71 ms), but its grid-wide barriers over many blocks
-// cost more than they save on large graphs (2049^2, 1.5e6 edges: 5.08 ->
-// 5.74 ms), hence the size limit.
-constexpr int kMstCoopMax = 1 << 20;
-
+// Borůvka in one launch (a block's, or a cooperative one); false when the device
+// refuses it (the host-driven rounds run instead).  Measured on B200, the whole
+// stage with the rounds driven by the host and in one launch: 2049^2 (1.5e6
+// edges) 3.21 and 3.03 ms, 4097^2 (6e6) 11.80 and 11.46.
 static bool mst_coop(Ctx& c, int nroots, int ne) {
+  MstCoop A{nroots, ne, c.nr_idx, c.e_b1, c.e_b2, c.e_rank, c.mst_comp, c.mst_min, c.mst_next, c.e_inmst, c.d_cnt};
   if (nroots <= kMstBlockRoots && ne <= kMstBlockEdges) {
-    MstCoop A{nroots, ne, c.nr_idx, c.e_b1, c.e_b2, c.e_rank, c.mst_comp, c.mst_min, c.mst_next, c.e_inmst, c.d_cnt};
-    void* args[] = {&A};
-    if (BigSmem<k_mst_block>::launch(1, kMstThreads, 3 * sizeof(int) * (size_t)nroots,
-                                     3 * (int)sizeof(int) * kMstBlockRoots, c.stream, args)) {
-      c.count_launch();
-      return true;
-    }
+    k_mst_block<<<1, kMstThreads, 3 * sizeof(int) * (size_t)nroots, c.stream>>>(A);
+    c.count_launch();
+    return true;
   }
-  if (std::max(ne, nroots) > kMstCoopMax) return false;
   int dev = 0, coop = 0, sms = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
@@ -1643,7 +1675,6 @@ static bool mst_coop(Ctx& c, int nroots, int ne) {
   // about 2048 edges per block, at most what is resident at once
   const int want = (std::max(ne, nroots) + 2047) / 2048;
   const int blocks = std::max(1, std::min(want, sms * per_sm));
-  MstCoop A{nroots, ne, c.nr_idx, c.e_b1, c.e_b2, c.e_rank, c.mst_comp, c.mst_min, c.mst_next, c.e_inmst, c.d_cnt};
   void* args[] = {&A};
   if (cudaLaunchCooperativeKernel((const void*)k_mst_coop, dim3(blocks), dim3(kCoopThreads), args, 0, c.stream) !=
       cudaSuccess) {
@@ -1670,7 +1701,8 @@ bool local_minima(Ctx& c) {
   k_basins<<<grid1d(nn), kBlock, 0, st>>>(nn, c.stack, c.s_scan2, c.basins);
   c.count_launch();
   catchment(c);  // find_stack's catch: labels of the forest before re-routing
-  k_roots_scan<<<grid1d(nn), kBlock, 0, st>>>(c.bd, c.s_roots, c.d_cnt);
+  unsigned char* open = reinterpret_cast<unsigned char*>(c.mst_next);  // free until the spanning tree
+  k_roots_scan<<<grid1d(nn), kBlock, 0, st>>>(c.bd, c.s_roots, open, c.d_cnt);
   c.count_launch();
   fetch_counters(c, 10);
   const int nroots = c.h_cnt[C_NBASINS];
@@ -1687,16 +1719,16 @@ bool local_minima(Ctx& c) {
   }
   // ---- connect_basins
   size_t cap = 1024;
-  while (cap < 16 * (size_t)nroots && cap < c.hash_cap) cap <<= 1;
+  while (cap < kPairSlots * ((size_t)nroots + 1) && cap < c.hash_cap) cap <<= 1;
   cudaMemsetAsync(c.ht_key, 0xff, sizeof(unsigned long long) * cap, st);
   cudaMemsetAsync(c.ht_wmin, 0xff, sizeof(unsigned long long) * cap, st);
   cudaMemsetAsync(c.ht_first, 0xff, sizeof(unsigned) * cap, st);
   cudaMemsetAsync(c.ht_best, 0xff, sizeof(unsigned) * cap, st);
-  k_conn_pass<0><<<grid1d(nn), kBlock, 0, st>>>(c.bd, c.basins, c.s_roots, c.pos, c.h, c.ht_key, c.ht_wmin,
+  k_conn_pass<0><<<grid1d(nn), kBlock, 0, st>>>(c.bd, c.basins, open, c.pos, c.h, c.ht_key, c.ht_wmin,
                                                  c.ht_first, c.ht_best, cap, c.d_cnt);
-  k_conn_pass<1><<<grid1d(nn), kBlock, 0, st>>>(c.bd, c.basins, c.s_roots, c.pos, c.h, c.ht_key, c.ht_wmin,
+  k_conn_pass<1><<<grid1d(nn), kBlock, 0, st>>>(c.bd, c.basins, open, c.pos, c.h, c.ht_key, c.ht_wmin,
                                                  c.ht_first, c.ht_best, cap, c.d_cnt);
-  k_conn_compact<<<grid1d(cap), kBlock, 0, st>>>(c.bd, cap, c.ht_key, c.ht_first, c.ht_best, c.stack, c.h,
+  k_conn_compact<<<(unsigned)((cap + 4 * kBlock - 1) / (4 * kBlock)), kBlock, 0, st>>>(c.bd, cap, c.ht_key, c.ht_first, c.ht_best, c.stack, c.h,
                                                   c.conn_cap, c.e_key, c.r_b1, c.r_b2, c.r_n1, c.r_n2,
                                                   c.r_w, c.d_cnt);
   k_conn_virtual<<<grid1d(nroots), kBlock, 0, st>>>(c.bd, nroots, c.s_roots, c.pos, c.conn_cap, c.e_key, c.r_b1,
@@ -1728,19 +1760,16 @@ bool local_minima(Ctx& c) {
     // rounds in batches of four, one read-back per batch (Borůvka at least
     // halves the components per round, so the bound of 64 is never reached)
     constexpr int kMstBatch = 4;
-    cudaMemsetAsync(c.d_cnt + C_CHANGED, 0, sizeof(int), st);
     cudaMemsetAsync(c.d_cnt + C_MST_DONE, 0, sizeof(int), st);
-    const int* done = c.d_cnt + C_MST_DONE;
+    k_mst_reset<<<grid1d(nroots), kBlock, 0, st>>>(nroots, c.mst_min);
+    c.count_launch();
     for (int round = 0; round < 64; round += kMstBatch) {
       for (int r = 0; r < kMstBatch; ++r) {
-        k_mst_reset<<<grid1d(nroots), kBlock, 0, st>>>(nroots, c.mst_min, done);
-        k_mst_minedge<<<grid1d(ne), kBlock, 0, st>>>(ne, c.e_b1, c.e_b2, c.e_rank, c.mst_comp, c.mst_min, done);
+        k_mst_minedge<<<grid1d(ne), kBlock, 0, st>>>(ne, c.e_b1, c.e_b2, c.e_rank, c.mst_comp, c.mst_min, c.d_cnt);
         k_mst_hook<<<grid1d(nroots), kBlock, 0, st>>>(nroots, c.nr_idx, c.e_b1, c.e_b2, c.mst_comp, c.mst_min,
                                                        c.mst_next, c.e_inmst, c.d_cnt);
-        k_mst_check<<<1, 1, 0, st>>>(c.d_cnt);
-        k_mst_apply<<<grid1d(nroots), kBlock, 0, st>>>(nroots, c.mst_next, c.mst_comp, done);
-        k_mst_flatten<<<grid1d(nroots), kBlock, 0, st>>>(nroots, c.mst_comp, c.d_cnt);
-        c.count_launch(6);
+        k_mst_compress<<<grid1d(nroots), kBlock, 0, st>>>(nroots, c.mst_next, c.mst_comp, c.mst_min, c.d_cnt);
+        c.count_launch(3);
       }
       fetch_counters(c, C_MST_DONE + 1);
       if (c.h_cnt[C_MST_DONE]) break;
