@@ -450,7 +450,7 @@ struct AccMfdOp {
 // hw[k] = (h, water); h keeps ht.  k's dependents are the donors that read it.
 // With GS (g > 0, StreamPowerLaw.f90:89-177 in a Gauss-Seidel iteration) the
 // surface comes from `elev`, Newton starts from the current iterate `hstart`,
-// and sill / contrib record the lake bookkeeping (as in k_spl_chains).
+// and sill / contrib record the lake bookkeeping (as in the single-flow solve).
 template <bool GS>
 struct SplMfdOp {
   const SplLine* line;

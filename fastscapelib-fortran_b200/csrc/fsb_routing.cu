@@ -14,7 +14,7 @@
 // reference's recursion it is built from the Euler tour of the forest: every
 // node k contributes an enter event E(k)=2k and an exit event X(k)=2k+1, the
 // tour successor of each event is local information (first donor, next
-// sibling, parent, next root), and list ranking by pointer jumping counts the
+// sibling, parent, next root), and list ranking (in tiles first) counts the
 // enter events from each event to the end of the tour.  That count gives the
 // preorder position and the subtree size of every node exactly.
 #include "fsb_kernels.cuh"
