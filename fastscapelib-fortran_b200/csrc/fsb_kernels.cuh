@@ -93,10 +93,10 @@ struct Ctx {
   // ---- scratch ----
   int *s_flag = nullptr, *s_scan = nullptr, *s_roots = nullptr, *s_root_rank = nullptr;
   unsigned long long *s_list_a = nullptr, *s_list_b = nullptr;  // 2*nn each
-  // list ranking by sublist walks: predecessor flags (2*nn bytes), the shorter
-  // lists and the count of list heads
-  unsigned long long *s_tour = nullptr, *s_tour_sub = nullptr;  // the tour's paths (tour_elements) and their walks
+  // the Euler tour's paths through the tiles (tour_elements of them): list, walks, weights
+  unsigned long long *s_tour = nullptr, *s_tour_sub = nullptr;
   unsigned* s_tour_weight = nullptr;
+  // list ranking by sublist walks: predecessor flags, the shorter lists and the count of list heads
   unsigned char* s_rank_pred = nullptr;
   unsigned long long* s_rank_ws = nullptr;
   unsigned* s_rank_nheads = nullptr;
@@ -118,7 +118,7 @@ struct Ctx {
       *nr_rs = nullptr, *nr_lpos = nullptr, *nr_rpos = nullptr, *nr_segof = nullptr;
   int *nr_seg = nullptr, *nr_seg2 = nullptr;  // segments: pairs (l, ir), 1-based
   int *nr_small = nullptr;                    // small segments (l, ir)
-  int *nr_med = nullptr;                      // segments of 8..512 elements (l, ir), finished in shared memory
+  int *nr_med = nullptr;                      // queue of the segments (l, ir) that blocks take
   double* nr_piv = nullptr;
   int* nr_segmeta = nullptr;  // per segment: pv, i, j, T
   int* nr_child = nullptr;    // per level segment: i, left id, right id, j (cooperative levels)
