@@ -14,8 +14,9 @@
 // parallel.  The sorted permutation itself is reproduced exactly: quicksort
 // segments are independent once created, and one Hoare partition of a
 // segment is determined by the positions of the left-scan stoppers
-// (arr >= pivot) and right-scan stoppers (arr <= pivot) of the segment, which
-// prefix sums give in parallel (see k_nr_cross for the crossing rule).  The
+// (arr not below the pivot: the negated test, which a NaN passes as it ends the
+// scan) and right-scan stoppers (arr not above it) of the segment, which
+// prefix sums give in parallel (see nr_cross_one for the crossing rule).  The
 // conn list is built in the reference's discovery order: edge (b,nb) sits at
 // the first (stack position, neighbour slot) where it is met and keeps the
 // earliest minimum-weight pass.  Receiver corrections touch disjoint child
@@ -344,8 +345,11 @@ __device__ inline void nr_median_one(int s, const int* seg, const double* __rest
   meta[4 * s] = idx[l];
 }
 
-// stopper flags of position q: the left scan stops where arr >= a (positions
-// l+2..ir), the right scan where arr <= a (positions l+1..ir-1)
+// stopper flags of position q: the left scan goes on while arr < a (positions
+// l+2..ir), the right scan while arr > a (positions l+1..ir-1).  A NaN stops
+// both, and a NaN pivot stops them everywhere, as in the sequential scans; the
+// median of three leaves a stopper at ir and at l+1 whatever the three are, so
+// that neither list is empty.
 __device__ inline void nr_flags_one(int q, const int* segof, const int* seg,
                                     const double* piv, const double* __restrict__ arr,
                                     const int* idx, int& a, int& b) {
@@ -356,8 +360,8 @@ __device__ inline void nr_flags_one(int q, const int* segof, const int* seg,
     const int l = seg[2 * s], ir = seg[2 * s + 1];
     const double pv = piv[s];
     const double v = arr[idx[q]];
-    a = (q >= l + 2 && q <= ir && v >= pv) ? 1 : 0;
-    b = (q >= l + 1 && q <= ir - 1 && v <= pv) ? 1 : 0;
+    a = (q >= l + 2 && q <= ir && !(v < pv)) ? 1 : 0;
+    b = (q >= l + 1 && q <= ir - 1 && !(v > pv)) ? 1 : 0;
   }
 }
 
@@ -675,7 +679,8 @@ __global__ void __launch_bounds__(kCoopThreads) k_nr_levels(NrCoop A) {
 
 // straight insertion of a small segment (LocalMinima.f90:967-976); the
 // reference's inner loop runs down to 1 but stops at position l-1 at the
-// latest because everything left of a segment is <= everything in it.
+// latest because everything left of a segment is <= everything in it (a NaN
+// there would not stop it; this one ends at the segment's start all the same).
 __global__ void k_nr_insertion(int nsmall, const int* __restrict__ small, const double* __restrict__ arr,
                                int* __restrict__ idx) {
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nsmall; s += gridDim.x * blockDim.x) {
@@ -830,7 +835,7 @@ __device__ __forceinline__ void nr_partition_warp(NrBlockShared& S, unsigned sho
 #pragma unroll
       for (int r = 0; r < kNrRuns; ++r) {
         const int q = li + 32 * r + lane;
-        f[r] = key[min(q, ir)] >= a && q < last_r;
+        f[r] = !(key[min(q, ir)] < a) && q < last_r;  // a NaN stops both scans
       }
 #pragma unroll
       for (int r = 0; r < kNrRuns; ++r) {
@@ -846,7 +851,7 @@ __device__ __forceinline__ void nr_partition_warp(NrBlockShared& S, unsigned sho
 #pragma unroll
       for (int r = 0; r < kNrRuns; ++r) {
         const int q = ri - 32 * r - lane;
-        f[r] = key[max(q, l)] <= a && q > last_l;
+        f[r] = !(key[max(q, l)] > a) && q > last_l;
       }
 #pragma unroll
       for (int r = 0; r < kNrRuns; ++r) {
@@ -990,7 +995,7 @@ __device__ __forceinline__ void nr_partition_block(NrBlockShared& S, double* key
       // keys loaded ahead hold unless the right side has listed some of them since
       if (pre != 1 || li + kNrSide - 1 > ri) load(li, 1);
       pre = 0;
-      nl = list(lb, 1, at_l, [&](int q, double v) { return v >= a && q < lim; });
+      nl = list(lb, 1, at_l, [&](int q, double v) { return !(v < a) && q < lim; });
       ol = 0;
       li += kNrSide;
     }
@@ -999,7 +1004,7 @@ __device__ __forceinline__ void nr_partition_block(NrBlockShared& S, double* key
       const int lim = last_l;
       if (pre != 2 || ri - kNrSide + 1 < li) load(ri, -1);
       pre = 0;
-      nr = list(rb, -1, at_r, [&](int q, double v) { return v <= a && q > lim; });
+      nr = list(rb, -1, at_r, [&](int q, double v) { return !(v > a) && q > lim; });
       orr = 0;
       ri -= kNrSide;
     }
@@ -1156,7 +1161,7 @@ __global__ void __launch_bounds__(kNrThreads) k_nr_block(unsigned long long* __r
       S.head = 0;
       S.filled = n > kNrTail ? 1 : 0;
       S.open = n > kNrTail ? 1 : 0;  // parts queued or in work
-      S.ntail = n > kNrTail ? 0 : 1;
+      S.ntail = n > 1 && n <= kNrTail ? 1 : 0;
       S.tail[0] = (unsigned)(n - 1);
     }
     __syncthreads();
