@@ -191,11 +191,13 @@ __device__ __forceinline__ unsigned edges_of(int di, int dj) {
   return (di < 0 ? kWest : di > 0 ? kEast : 0u) | (dj < 0 ? kSouth : dj > 0 ? kNorth : 0u);
 }
 template <class T>
-struct __align__(32) RecordT {
+struct RecordFields {
   unsigned codes, meta;
   double base;
   T c[8];
 };
+template <class T>
+struct __align__(32) RecordT : RecordFields<T> {};
 static_assert(sizeof(RecordT<double>) == 96 && sizeof(RecordT<float>) == 64, "whole 32-byte sectors");
 
 // ---- record builders --------------------------------------------------------
@@ -240,9 +242,14 @@ __device__ __forceinline__ unsigned tile_edges(const Bounds& bd, int ts, int i, 
 // whole lines; built in place, word by word, k_acc_records took 328 us and
 // k_spl_records 580 of 2049^2, now 236 and 462.
 constexpr int kRecPitch = 104;  // bytes per record there: an odd number of double words
+// node: its place among the block's 256.  The staged form carries the fields'
+// own alignment only: at this pitch the compiler must not take the 16-byte
+// header for one store.
 template <class T>
-__device__ __forceinline__ RecordT<T>* staged_record(unsigned char* sm) {
-  return reinterpret_cast<RecordT<T>*>(sm + (threadIdx.y * 32 + threadIdx.x) * kRecPitch);
+__device__ __forceinline__ RecordFields<T>* staged_record(unsigned char* sm, int node) {
+  using Staged = RecordFields<T>;
+  static_assert(kRecPitch % alignof(Staged) == 0 && sizeof(RecordT<T>) <= kRecPitch, "every staged record is aligned");
+  return reinterpret_cast<Staged*>(sm + node * kRecPitch);
 }
 template <class T>
 __device__ __forceinline__ void store_records(const Bounds& bd, const unsigned char* sm, RecordT<T>* __restrict__ rec) {
@@ -269,7 +276,7 @@ __global__ void __launch_bounds__(256) k_acc_records(Bounds bd, int ts, double d
     const unsigned edges = tile_edges(bd, ts, i, j);
     unsigned codes = 0, far = 0;
     int n = 0;
-    RecordT<T>* r = staged_record<T>(sm);
+    RecordFields<T>* r = staged_record<T>(sm, threadIdx.y * 32 + threadIdx.x);
   #pragma unroll
     for (int t = 0; t < 8; ++t) {
       int d;
@@ -332,7 +339,7 @@ __global__ void __launch_bounds__(256) k_spl_records(
     const int r = recv[k];
     const unsigned edges = tile_edges(bd, ts, i, j);
     unsigned codes = 0, waits = 0, far = 0, rcode = 0, lengths = 0;
-    RecordT<T>* out = staged_record<T>(sm);
+    RecordFields<T>* out = staged_record<T>(sm, me);
     if (r != k) {
       factor[me] = ((kfsed > 0.0 && (htk - b[k]) > 1.0) ? kfsed : kf[k]) * dt;
       const double ak = a[k];
@@ -410,7 +417,7 @@ __global__ void __launch_bounds__(256) k_spl_records(
   __syncwarp();
   for (int e = threadIdx.x; e < total; e += 32) {
     const int slot = slots[threadIdx.y][e] & 7, node = threadIdx.y * 32 + (slots[threadIdx.y][e] >> 3);
-    T* const c = &reinterpret_cast<RecordT<T>*>(sm + node * kRecPitch)->c[slot];
+    T* const c = &staged_record<T>(sm, node)->c[slot];
     const int len = (lens[node] >> (2 * slot)) & 3;
     const double kk = factor[node], l = __ldg(&ltab[len]);
     const T ln = __ldg(&lpow[len]), aw = *c;
