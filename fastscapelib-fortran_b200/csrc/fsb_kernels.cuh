@@ -141,7 +141,6 @@ struct Ctx {
   double* slots = nullptr;   // kSlotStride input slots per node of the multiple-flow sweeps
   // region-owned sweeps (fsb_region.cu)
   TileMap tplan[kTilePlans];  // per tile side
-  bool region_enabled = true;  // use them when the plan and a cooperative launch allow
   signed char region_ok[8] = {};  // per sweep op: 0 unchecked, 1 usable, -1 not
   unsigned short* rl_wmeta = nullptr;  // per node: inputs to wait for | dependents' directions << 8
   unsigned* rl_flags = nullptr;        // rim_words per tile

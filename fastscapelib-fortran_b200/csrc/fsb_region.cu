@@ -1051,7 +1051,7 @@ bool region_fits(const TileMap& tm) {
 // whether the sweep of Op can run on the plan (checked once per instance)
 template <class Op, int LT>
 bool region_usable(Ctx& c, const TileMap& tm) {
-  if (!c.region_enabled || tm.ntx == 0) return false;
+  if (tm.ntx == 0) return false;
   signed char& st = c.region_ok[Op::kId];
   if (st == 0) st = region_fits<Op, LT>(tm) ? 1 : -1;
   return st > 0;
@@ -1077,13 +1077,13 @@ bool launch_region(Ctx& c, const TileMap& plan, Op op) {
   stage_begin(c, timer);
   const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_region_sweep<Op, LT>, dim3(tm.nctas), dim3(kThreads),
                                                     args, (size_t)region_smem(tm), c.stream);
-  stage_end(c, timer);
-  c.count_launch();
   if (e != cudaSuccess) {  // e.g. the GPU is shared and the CTAs no longer fit
     cudaGetLastError();
     c.region_ok[Op::kId] = -1;
     return false;
   }
+  stage_end(c, timer);  // the timers count sweeps that ran here
+  c.count_launch();
   return true;
 }
 
