@@ -983,7 +983,19 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int c = R::index((X & (kTS - 1)) - di, (Y & (kTS - 1)) - dj, ow, oh);
         const size_t tile = (size_t)oy * tm.ntx + ox;
         mail_write(mbox + tile * R::kCells + c, out);
-        atomicOr(&flags[tile * R::kWords + (c >> 5)], 1u << (c & 31));
+        // Around a cyclic side that one tile spans the node is this CTA's own: its
+        // counter is at hand, and warp 0 need not hear of it (area of 3 x 3736 nodes,
+        // flow along it: 6.4 -> 4.1 ms, of 60000 x 20 264 -> 165)
+        if (ox == ti.x0 >> LT && oy == ti.y0 >> LT) {
+          const int l = (id >> (2 * LT) << (2 * LT)) | ((Y & (kTS - 1)) << LT) | (X & (kTS - 1));
+          __threadfence_block();  // the cell before the counter
+          if (release(l)) {
+            __threadfence_block();
+            push(atomicAdd(&qtail, 1), X + Y * tm.nx, l);
+          }
+        } else {
+          atomicOr(&flags[tile * R::kWords + (c >> 5)], 1u << (c & 31));
+        }
       }
       done += on && sl == 0;
       k = nk;

@@ -1,6 +1,7 @@
-"""The region sweeps (csrc/fsb_region.cu) against the queue engine of fsb_flow.cu.
-The sweeps' timers count launches, so that a step that fell back to the queue
-engine would show.
+"""The region sweeps (csrc/fsb_region.cu) on strips: cyclic sides that one tile
+spans, whose nodes release each other without the mailbox.  The sweeps' timers count launches,
+so that a step that fell back to the queue engine of fsb_flow.cu would show.
+Against the oracle as in test_region_sweeps.py.
 
 Both engines do a node's arithmetic in the same order: with g > 0 below the
 smallest normal number the step takes one Gauss-Seidel iteration, which is the
@@ -8,7 +9,9 @@ g = 0 solve on the queue engine (and no deposition), and must give its bits."""
 import numpy as np
 import pytest
 
+import oracle as O
 from fastscapelib_fortran import workloads as W
+from test_region_sweeps import _rel
 
 pytestmark = pytest.mark.gpu
 
@@ -33,6 +36,30 @@ def _field(x, name, nn):
     out = np.empty(nn)
     x.copy(name, out)
     return out
+
+
+def _tilted(wl):
+    j, i = np.divmod(np.arange(wl.nn), wl.nx)
+    wl.h0 = wl.h0 + 0.3 * (j if wl.ny > wl.nx else i)  # flow along the strip
+    return wl
+
+
+STRIPS = [(3, 700, 1010), (700, 4, 101), (20, 300, 1000), (300, 31, 1), (32, 300, 1010)]
+
+
+@pytest.mark.parametrize("nx,ny,bc", STRIPS)
+@pytest.mark.parametrize("n", [1.0, 1.5, 1.27])
+def test_strips_match_oracle(nx, ny, bc, n):
+    wl = _tilted(W.mfd(nx, ny, seed=nx * 1000 + ny, n=n, bc=bc))
+    wl.apply(O)
+    O.fastscape_execute_step()
+    x = _gpu(wl)
+    st = x.stage_times()
+    assert st["k_area_sweep"][1] == 1 and st["k_spl_sweep"][1] == 1
+    assert np.array_equal(x.copy_int("rec"), O.copy_int("rec"))
+    for f in ("drainage_area", "h", "total_erosion"):
+        assert _rel(_field(x, f, wl.nn), O.copy_double(f)) <= 1e-9, f
+    x.destroy()
 
 
 @pytest.mark.parametrize("nx,ny,bc", [(3, 3, 1010), (33, 64, 1010), (130, 96, 101), (64, 300, 1111), (20, 300, 1000),
