@@ -1141,10 +1141,10 @@ bool stream_power_t(Ctx& c) {
   return true;
 }
 
-template <class T>
+template <class T, int LT>
 bool stream_power_n(Ctx& c) {
-  if (fabs(c.n - 1.0) < DBL_MIN) return stream_power_t<T, 0, 5>(c);
-  return c.n == 1.5 ? stream_power_t<T, 1, 5>(c) : stream_power_t<T, 2, 5>(c);
+  if (fabs(c.n - 1.0) < DBL_MIN) return stream_power_t<T, 0, LT>(c);
+  return c.n == 1.5 ? stream_power_t<T, 1, LT>(c) : stream_power_t<T, 2, LT>(c);
 }
 
 }  // namespace
@@ -1170,11 +1170,26 @@ TileMap plan_tiles(int nx, int ny, int lt, int sms) {
 // nodes, all sources at once, are spread anyway.  B200, side 32 / 64: area
 // 257^2 0.48 / 0.53 ms, 1025x769 3.05 / 2.88, 2049^2 6.4 / 5.8; stream power
 // (n = 1.5) 0.69 / 0.84, 3.98 / 4.27, 6.9 / 7.3, 4097^2 18.0 / 18.0.
+// A strip that one larger tile spans and a smaller one does not takes the larger:
+// its flow runs along it, and every row of nodes would wait for a crossing
+// (4000x33, a cone: area 11.3 / 5.5 ms, stream power 15.7 / 10.8; 256x50, a ramp:
+// 1.07 / 0.68 and 1.32 / 1.01).  Short ones have more to lose without a slope
+// (128x64, a relief: 0.18 / 0.24 and 0.31 / 0.50).
+static bool larger_tiles(const Ctx& c, bool area) {
+  constexpr int kSmall = 1 << kLogTileMin;
+  const int across = std::min(c.nx, c.ny), along = std::max(c.nx, c.ny);
+  if (across > kSmall && across <= 2 * kSmall && along >= 8 * kSmall) return true;
+  return area && c.nn > 1 << 18;
+}
+
 bool region_accumulate(Ctx& c) {
-  if (c.nn <= 1 << 18) return c.mixed ? accumulate_t<float, 5>(c) : accumulate_t<double, 5>(c);
+  if (!larger_tiles(c, true)) return c.mixed ? accumulate_t<float, 5>(c) : accumulate_t<double, 5>(c);
   return c.mixed ? accumulate_t<float, 6>(c) : accumulate_t<double, 6>(c);
 }
 
-bool region_stream_power(Ctx& c) { return c.mixed ? stream_power_n<float>(c) : stream_power_n<double>(c); }
+bool region_stream_power(Ctx& c) {
+  if (!larger_tiles(c, false)) return c.mixed ? stream_power_n<float, 5>(c) : stream_power_n<double, 5>(c);
+  return c.mixed ? stream_power_n<float, 6>(c) : stream_power_n<double, 6>(c);
+}
 
 }  // namespace fsb

@@ -1,5 +1,6 @@
 """The region sweeps (csrc/fsb_region.cu) on strips: cyclic sides that one tile
-spans, whose nodes release each other without the mailbox.  The sweeps' timers count launches,
+spans, whose nodes release each other without the mailbox, and the borders of
+the rule that gives strips the larger tiles.  The sweeps' timers count launches,
 so that a step that fell back to the queue engine of fsb_flow.cu would show.
 Against the oracle as in test_region_sweeps.py.
 
@@ -44,7 +45,8 @@ def _tilted(wl):
     return wl
 
 
-STRIPS = [(3, 700, 1010), (700, 4, 101), (20, 300, 1000), (300, 31, 1), (32, 300, 1010)]
+STRIPS = [(3, 700, 1010), (700, 4, 101), (20, 300, 1000), (300, 31, 1), (32, 300, 1010), (33, 256, 1010), (33, 255, 1111),
+          (256, 64, 101), (64, 300, 1111), (65, 300, 1010), (300, 64, 1)]
 
 
 @pytest.mark.parametrize("nx,ny,bc", STRIPS)
