@@ -123,7 +123,7 @@ size_t layout(fsb::Ctx& c, char* base) {
   c.s_flag = L.take<int>(N + 1); c.s_scan = L.take<int>(N + 1); c.s_roots = L.take<int>(N);
   c.s_root_rank = L.take<int>(N);
   c.s_list_a = L.take<unsigned long long>(2 * N); c.s_list_b = L.take<unsigned long long>(2 * N);
-  const size_t paths = fsb::tour_elements(c.nx, c.ny);
+  const size_t paths = fsb::TourTiles(c.nx, c.ny).elements();
   c.s_tour = L.take<unsigned long long>(paths); c.s_tour_sub = L.take<unsigned long long>(paths);
   c.s_tour_weight = L.take<unsigned>(paths);
   c.s_rank_ws = L.take<unsigned long long>(fsb::rank_scratch(std::max(2 * N, paths)));

@@ -93,7 +93,7 @@ struct Ctx {
   // ---- scratch ----
   int *s_flag = nullptr, *s_scan = nullptr, *s_roots = nullptr, *s_root_rank = nullptr;
   unsigned long long *s_list_a = nullptr, *s_list_b = nullptr;  // 2*nn each
-  // the Euler tour's paths through the tiles (tour_elements of them): list, walks, weights
+  // the Euler tour's paths through the tiles (TourTiles::elements of them): list, walks, weights
   unsigned long long *s_tour = nullptr, *s_tour_sub = nullptr;
   unsigned* s_tour_weight = nullptr;
   // list ranking by sublist walks: predecessor flags, the shorter lists and the count of list heads
@@ -226,11 +226,25 @@ unsigned long long* list_rank(Ctx& c, size_t n, unsigned long long* a, unsigned 
 // list ranking by sublist walks: a splitter every 16 or 4 entries plus each
 // list head (at most kRankMaxHeads heads); a block ranks up to kRankBlock entries
 constexpr int kRankMaxHeads = 4, kRankBlock = 8192;
-// tiles of the Euler tour and list elements per tile (fsb_routing.cu)
-constexpr int kTourTileX = 64, kTourTileY = 32, kTourSlots = 768;
-inline size_t tour_elements(int nx, int ny) {
-  return (size_t)((nx + kTourTileX - 1) / kTourTileX) * ((ny + kTourTileY - 1) / kTourTileY) * kTourSlots;
-}
+// Tiles of the Euler tour (fsb_routing.cu): 2048 nodes, 64 x 32, or as wide (high)
+// as a narrower grid's power of two and so much higher (wider), and list elements
+// per tile: paths leave a tile from the two outermost rows and columns beyond
+// which the grid goes on, or from the last root of a row.
+constexpr int kTourNodes = 2048;
+struct TourTiles {
+  int lx = 6, ly = 5;  // log2 of the sides
+  int tiles_x, tiles_y, slots;
+  TourTiles(int nx, int ny) {
+    while (lx > 2 && nx <= 1 << (lx - 1)) --lx, ++ly;
+    if (lx == 6)
+      while (ly > 2 && ny <= 1 << (ly - 1)) --ly, ++lx;
+    tiles_x = ((nx - 1) >> lx) + 1;
+    tiles_y = ((ny - 1) >> ly) + 1;
+    const int inner = ((1 << lx) - (tiles_x > 1 ? 4 : 0)) * ((1 << ly) - (tiles_y > 1 ? 4 : 0));
+    slots = 2 * (kTourNodes - inner) + (1 << ly);
+  }
+  size_t elements() const { return (size_t)tiles_x * tiles_y * slots; }
+};
 // scratch entries below a list of n: per level its splitters and their walk's results
 inline size_t rank_scratch(size_t n) {
   size_t total = 0;

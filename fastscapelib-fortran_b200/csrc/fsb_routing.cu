@@ -319,22 +319,23 @@ __global__ void k_rank_final(size_t n, const unsigned long long* __restrict__ su
 // leaves (weight 0): 2k is followed by the first donor's entry or by 2k+1, 2k+1
 // by the next donor of k's receiver, by the receiver's exit, or for a root by
 // the next root.  Suffix sums of the weights give the stack's positions.
-// Successors are nearly always neighbours, so a block takes a tile of
-// kTourX x kTourY nodes and jumps pointers in shared memory: every entry learns
-// the last entry of its path inside the tile and the weight up to there.  Only
-// the paths go to the list ranking, one element each.  A path can leave a tile
-// from its two outermost rings of nodes (donors and receivers are one node
-// away, siblings two) or from the last root of a row, hence kTourSlots.
+// Successors are nearly always neighbours, so a block takes a tile of 2048 nodes
+// and jumps pointers in shared memory: every entry learns the last entry of its
+// path inside the tile and the weight up to there.  Only the paths go to the list
+// ranking, one element each.  A path can leave a tile from its two outermost rings
+// of nodes (donors and receivers are one node away, siblings two) or from the last
+// root of a row, hence TourTiles::slots.
 //
 // Measured (B200): walking all 2 nn entries in random order took 595 us twice
 // per step of 2049^2, the tiles and their paths' ranking 190.  The stack of
 // 1023x767 329 -> 151 us, of 101^2 68 -> 62; the stack after LocalMinima gains
-// more, its walks being longer.
-constexpr int kTourX = 64, kTourY = 32, kTourNodes = kTourX * kTourY, kTourThreads = 512;
-static_assert(kTourSlots >= 2 * (kTourNodes - (kTourX - 4) * (kTourY - 4)) + kTourY, "every path has a slot");
-static_assert(kTourX == kTourTileX && kTourY == kTourTileY, "the arena's tiles");
+// more, its walks being longer.  Strips' tiles follow their shorter side: tiles of
+// 64 x 32 gave a strip under 12 nodes wide a longer list than the 2 nn entries (3 x
+// 60000: stack 126 us with those, 165 so, 80 with tiles of 4 x 512).
+constexpr int kTourThreads = 512;
 
-__global__ void __launch_bounds__(kTourThreads) k_tour_tiles(int nx, int ny, const int* __restrict__ rec,
+__global__ void __launch_bounds__(kTourThreads) k_tour_tiles(int nx, int ny, TourTiles tt,
+                                                             const int* __restrict__ rec,
                                                              const int* __restrict__ ndon,
                                                              const int* __restrict__ don,
                                                              const int* __restrict__ roots,
@@ -350,8 +351,8 @@ __global__ void __launch_bounds__(kTourThreads) k_tour_tiles(int nx, int ny, con
   __shared__ unsigned char inner[2 * kTourNodes];  // has a predecessor in the tile
   __shared__ int count;
   const int tid = threadIdx.x;
-  const int x0 = blockIdx.x * kTourX, y0 = blockIdx.y * kTourY;
-  const unsigned tile = blockIdx.y * gridDim.x + blockIdx.x, first = tile * kTourSlots;
+  const int tx = 1 << tt.lx, ty = 1 << tt.ly, x0 = blockIdx.x << tt.lx, y0 = blockIdx.y << tt.ly;
+  const unsigned tile = blockIdx.y * gridDim.x + blockIdx.x, first = tile * tt.slots;
   const int R = *nroots;
   if (tid == 0) count = 0;
   for (int e = tid; e < 2 * kTourNodes / 4; e += kTourThreads) reinterpret_cast<unsigned*>(inner)[e] = 0u;
@@ -360,7 +361,7 @@ __global__ void __launch_bounds__(kTourThreads) k_tour_tiles(int nx, int ny, con
   int node[kEach];
 #pragma unroll
   for (int n = 0; n < kEach; ++n) {
-    const int ln = tid + n * kTourThreads, x = x0 + ln % kTourX, y = y0 + ln / kTourX;
+    const int ln = tid + n * kTourThreads, x = x0 + (ln & (tx - 1)), y = y0 + (ln >> tt.lx);
     valid[n] = x < nx && y < ny;
     const int k = x + y * nx;
     node[n] = k;
@@ -391,8 +392,8 @@ __global__ void __launch_bounds__(kTourThreads) k_tour_tiles(int nx, int ny, con
       unsigned to = (unsigned)e;  // the path's last entry points to itself
       if (valid[n] && next[2 * n + b] != END) {
         const int q = (int)(next[2 * n + b] >> 1), qy = q / nx, lx = q - qy * nx - x0, ly = qy - y0;
-        if (lx >= 0 && lx < kTourX && ly >= 0 && ly < kTourY) {
-          to = 2u * (unsigned)(ly * kTourX + lx) + (next[2 * n + b] & 1u);
+        if (lx >= 0 && lx < tx && ly >= 0 && ly < ty) {
+          to = 2u * (unsigned)((ly << tt.lx) + lx) + (next[2 * n + b] & 1u);
           inner[to] = 1;
         }
       }
@@ -422,7 +423,7 @@ __global__ void __launch_bounds__(kTourThreads) k_tour_tiles(int nx, int ny, con
       const unsigned e = 2u * (tid + n * kTourThreads) + b;
       if (valid[n] && path[e] >> 16 == e) {
         const int s = atomicAdd(&count, 1);
-        if (s < kTourSlots) {
+        if (s < tt.slots) {
           slot[e] = (unsigned short)s;
           list[2 * (size_t)(first + s) + 1] = next[2 * n + b];
         } else {
@@ -431,7 +432,7 @@ __global__ void __launch_bounds__(kTourThreads) k_tour_tiles(int nx, int ny, con
       }
     }
   __syncthreads();
-  for (int s = count + tid; s < kTourSlots; s += kTourThreads) {
+  for (int s = count + tid; s < tt.slots; s += kTourThreads) {
     list[2 * (size_t)(first + s)] = 0u;
     list[2 * (size_t)(first + s) + 1] = kInert;
   }
@@ -465,14 +466,14 @@ __global__ void k_tour_link(int nn, size_t n, const unsigned* __restrict__ head_
 }
 
 // preorder position and subtree size from the ranks of the enter/exit entries
-__global__ void k_stack_from_tiles(int nx, int ny, const unsigned* __restrict__ info,
+__global__ void k_stack_from_tiles(int nx, int ny, TourTiles tt, const unsigned* __restrict__ info,
                                    const unsigned long long* __restrict__ ranks, const unsigned* __restrict__ weight,
                                    int* __restrict__ pos, int* __restrict__ size, int* __restrict__ stack,
                                    int* __restrict__ err) {
-  const int nn = nx * ny, tiles_x = (nx + kTourX - 1) / kTourX;
+  const int nn = nx * ny;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
     const int y = k / nx, x = k - y * nx;
-    const size_t first = (size_t)((y / kTourY) * tiles_x + x / kTourX) * kTourSlots;
+    const size_t first = (size_t)((y >> tt.ly) * tt.tiles_x + (x >> tt.lx)) * tt.slots;
     const uint2 w = reinterpret_cast<const uint2*>(info)[k];
     const size_t se = first + (w.x >> 16), sx = first + (w.y >> 16);
     // from the path's first entry, less what lies before this one
@@ -551,15 +552,16 @@ void build_stack(Ctx& c, const int* rec, int* ndon, int* don, int* stack, int* p
   exclusive_scan_int(c, c.s_flag, c.s_scan, nn + 1);  // s_scan[nn] = number of roots
   k_root_list<<<grid1d(nn), kBlock, 0, c.stream>>>(nn, rec, c.s_scan, c.s_roots, c.s_root_rank);
   c.count_launch();
-  const dim3 tiles((c.nx + kTourX - 1) / kTourX, (c.ny + kTourY - 1) / kTourY);
-  const size_t n = tour_elements(c.nx, c.ny);
+  const TourTiles tt(c.nx, c.ny);
+  const dim3 tiles(tt.tiles_x, tt.tiles_y);
+  const size_t n = tt.elements();
   unsigned* head_slot = reinterpret_cast<unsigned*>(c.s_list_a);
   unsigned* info = head_slot + 2 * (size_t)nn;
-  k_tour_tiles<<<tiles, kTourThreads, 0, c.stream>>>(c.nx, c.ny, rec, ndon, don, c.s_roots, c.s_root_rank, c.s_scan + nn,
+  k_tour_tiles<<<tiles, kTourThreads, 0, c.stream>>>(c.nx, c.ny, tt, rec, ndon, don, c.s_roots, c.s_root_rank, c.s_scan + nn,
                                                      head_slot, info, reinterpret_cast<unsigned*>(c.s_tour), c.d_err);
   k_tour_link<<<grid1d(n), kBlock, 0, c.stream>>>(nn, n, head_slot, c.s_tour, c.s_tour_weight);
   rank_list<false>(c, n, c.s_tour, c.s_tour_sub, c.s_rank_ws);
-  k_stack_from_tiles<<<grid1d(nn), kBlock, 0, c.stream>>>(c.nx, c.ny, info, c.s_tour, c.s_tour_weight, pos, size, stack,
+  k_stack_from_tiles<<<grid1d(nn), kBlock, 0, c.stream>>>(c.nx, c.ny, tt, info, c.s_tour, c.s_tour_weight, pos, size, stack,
                                                           c.d_err);
   c.count_launch(3);
 }
