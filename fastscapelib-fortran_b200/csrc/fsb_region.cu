@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   unsigned char* rim = smem + tm.ns * kNodes;                                        // tm.ns * R::kCells
   unsigned* seen = reinterpret_cast<unsigned*>(rim + tm.ns * R::kCells);            // tm.ns * R::kWords
   TileInfo* tab = reinterpret_cast<TileInfo*>(seen + tm.ns * R::kWords);  // tm.ns
-  long long* q = queue + (size_t)blockIdx.x * tm.ns * kNodes;
+  long long* q = queue + blockIdx.x * tm.cta_nodes();
   const unsigned long long t0 = global_ns();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int kWarps = kThreads / 32;
