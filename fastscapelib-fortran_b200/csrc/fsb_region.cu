@@ -21,7 +21,8 @@
 // says whether it has arrived, so no fence beyond CTA scope runs during a
 // sweep (a fence at GPU scope would empty the SM's L1).  The arithmetic of a
 // node, including the order of its sums, is that of the queue engine in
-// fsb_flow.cu, so both engines give bit-identical results.
+// fsb_flow.cu, so both engines give bit-identical results in FP64 (the mixed form's
+// FP32 sweeps are this engine's alone).
 //
 // What bounds them (2049^2, B200, a trace of every node's start and end
 // followed back from the last one): the path is about 6,000 hops, 90 % of
@@ -1182,14 +1183,22 @@ static bool larger_tiles(const Ctx& c, bool area) {
   return area && c.nn > 1 << 18;
 }
 
+// The mixed form's sweeps run in FP32 on up to 296 blocks of 256 x 128 nodes (9.7e6)
+// and in FP64 beyond: the rounding of the areas grows with the number of nodes
+// that drain through one, and elevations with them (relative error of h after a
+// step of 3001^2: 4.5e-7; of 4097^2 2.3e-5 with FP32 sweeps, 2.3e-7 without).
+static bool fp32_sweeps(const Ctx& c) { return c.mixed && ((c.nx + 255) / 256) * ((c.ny + 127) / 128) <= 296; }
+
 bool region_accumulate(Ctx& c) {
-  if (!larger_tiles(c, true)) return c.mixed ? accumulate_t<float, 5>(c) : accumulate_t<double, 5>(c);
-  return c.mixed ? accumulate_t<float, 6>(c) : accumulate_t<double, 6>(c);
+  const bool f32 = fp32_sweeps(c);
+  if (!larger_tiles(c, true)) return f32 ? accumulate_t<float, 5>(c) : accumulate_t<double, 5>(c);
+  return f32 ? accumulate_t<float, 6>(c) : accumulate_t<double, 6>(c);
 }
 
 bool region_stream_power(Ctx& c) {
-  if (!larger_tiles(c, false)) return c.mixed ? stream_power_n<float, 5>(c) : stream_power_n<double, 5>(c);
-  return c.mixed ? stream_power_n<float, 6>(c) : stream_power_n<double, 6>(c);
+  const bool f32 = fp32_sweeps(c);
+  if (!larger_tiles(c, false)) return f32 ? stream_power_n<float, 5>(c) : stream_power_n<double, 5>(c);
+  return f32 ? stream_power_n<float, 6>(c) : stream_power_n<double, 6>(c);
 }
 
 }  // namespace fsb
