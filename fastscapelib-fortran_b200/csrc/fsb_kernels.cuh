@@ -34,13 +34,9 @@ struct TileMap {
   int nx = 0, ny = 0, lt = 0;
   int ntx = 0, nty = 0;  // ntx == 0: no plan
   int nctas = 0, ns = 0;  // CTAs, tiles per CTA at most
+  int cta_nodes = 0;      // nodes of a CTA's tiles at most (a strip does not fill them)
   __host__ __device__ int tiles() const { return ntx * nty; }
-  // nodes of a CTA's tiles at most (a strip does not fill them)
-  __host__ __device__ size_t cta_nodes() const {
-    const int ts = 1 << lt;
-    return (size_t)ns * (nx < ts ? nx : ts) * (ny < ts ? ny : ts);
-  }
-  size_t queue_entries() const { return nctas * cta_nodes(); }
+  size_t queue_entries() const { return (size_t)nctas * cta_nodes; }
 };
 
 // heavy-path chains (fsb_chains.cu): nodes of a long one; ticket buckets (32

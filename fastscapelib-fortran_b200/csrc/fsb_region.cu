@@ -718,7 +718,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   unsigned char* rim = smem + tm.ns * kNodes;                                        // tm.ns * R::kCells
   unsigned* seen = reinterpret_cast<unsigned*>(rim + tm.ns * R::kCells);            // tm.ns * R::kWords
   TileInfo* tab = reinterpret_cast<TileInfo*>(seen + tm.ns * R::kWords);  // tm.ns
-  long long* q = queue + blockIdx.x * tm.cta_nodes();
+  long long* q = queue + (size_t)blockIdx.x * tm.cta_nodes;
+  asm volatile("" : "+l"(q));  // kept, not worked out anew for every look (1 to 2 % of a sweep)
   const unsigned long long t0 = global_ns();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int kWarps = kThreads / 32;
@@ -1163,6 +1164,7 @@ TileMap plan_tiles(int nx, int ny, int lt, int sms) {
   tm.nctas = std::min(std::max(1, sms), tm.tiles());
   tm.ns = (tm.tiles() + tm.nctas - 1) / tm.nctas;
   if (region_smem(tm) > kMaxSmem) tm.ntx = 0;
+  else tm.cta_nodes = tm.ns * std::min(1 << lt, nx) * std::min(1 << lt, ny);
   return tm;
 }
 
