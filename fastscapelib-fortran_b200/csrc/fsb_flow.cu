@@ -1400,12 +1400,9 @@ __global__ void k_diff_finish(Bounds bd, double dt, const double* __restrict__ U
 
 void mfd_receivers(Ctx& c) {
   const int nn = c.nn;
-  if (c.mixed)
-    k_mfd_receivers<true><<<(nn + kMrecvThreads - 1) / kMrecvThreads, kMrecvThreads, 0, c.stream>>>(c.bd, c.p, c.hwater, c.ltab, c.mrec, c.mnrec, c.mwrec,
-                                                               c.mlrec, c.mdmask);
-  else
-    k_mfd_receivers<false><<<(nn + kMrecvThreads - 1) / kMrecvThreads, kMrecvThreads, 0, c.stream>>>(c.bd, c.p, c.hwater, c.ltab, c.mrec, c.mnrec,
-                                                                c.mwrec, c.mlrec, c.mdmask);
+  const auto receivers = c.mixed ? k_mfd_receivers<true> : k_mfd_receivers<false>;
+  receivers<<<(nn + kMrecvThreads - 1) / kMrecvThreads, kMrecvThreads, 0, c.stream>>>(
+      c.bd, c.p, c.hwater, c.ltab, c.mrec, c.mnrec, c.mwrec, c.mlrec, c.mdmask);
   c.count_launch();
   if (c.capture) {  // a topological order of mrec (the reference's mstack is a LIFO Kahn order)
     k_order_keys<<<grid1d(nn), kBlock, 0, c.stream>>>(nn, c.stack, c.hwater, c.o_keys, c.o_vals);

@@ -137,7 +137,9 @@ struct Ctx {
   bool chains_valid = false;  // the chain schedule matches the current forest
   // last-arriver sweeps (multiple flow)
   int *la_queue = nullptr, *la_cnt = nullptr, *cnt_acc = nullptr, *cnt_spl = nullptr;
-  void* mfd_line = nullptr;  // one 128-byte record per node (area, then stream power)
+  // one record per node (area, then stream power): 128 bytes of the queue engine, 96 or
+  // 64 of the region sweeps
+  void* mfd_line = nullptr;
   double* hw = nullptr;      // (elevation, water surface) pairs of the stream-power sweep
   double* slots = nullptr;   // kSlotStride input slots per node of the multiple-flow sweeps
   // region-owned sweeps (fsb_region.cu)

@@ -43,7 +43,7 @@ constexpr int kNrCounters = 15;  // counters the NR sort reads back
 // The sort's segments by length: above kNrSplit they are partitioned level by
 // level over the whole grid, up to kNrSplit by one block in global memory (the
 // parts of one segment by as many blocks), up to kNrBlock in a block's shared
-// memory (both k_nr_block).  kNrMedium is the longest part nr_sort_local takes.
+// memory (both k_nr_block).  kNrMedium is the longest segment nr_sort_local takes.
 // A grid-wide level costs 80-110 us whatever its segments are, most of it
 // barriers; a block partitions 91,445 elements in 50 us and 4,000 in 8, and
 // the parts go on at once.  With kNrSplit 2^17 or 2^19 the stage of 2049^2
@@ -437,9 +437,9 @@ __device__ inline int nr_apply_one(int q, const int* segof, const int* seg,
 }
 
 // children segments [l, j-1] and [i, ir]: partitioned at the next level when
-// they hold more than `limit` elements (counted in cnt[out_slot]), finished
-// in shared memory when they hold 8..limit (cnt[C_NMED]), insertion-sorted
-// when fewer (M = 7)
+// they hold more than `limit` elements (counted in cnt[out_slot]), queued for
+// k_nr_block when they hold 8..limit (cnt[C_NMED]), insertion-sorted when fewer
+// (M = 7)
 // The children's ids go to child[4s..4s+3] (i, left id, right id, j); child
 // may be meta itself (i and j are read before anything is written).
 __device__ inline void nr_newsegs_one(int s, int out_slot, const int* seg, const int* meta, int* child,
@@ -715,6 +715,8 @@ __global__ void k_nr_insertion(int nsmall, const int* __restrict__ small, const 
 // segment (the median index (l+ir)/2 keeps its value relative to l).
 // Segments are independent, so the order they are finished in does not
 // matter, and the insertion stops at the segment's start as k_nr_insertion's does.
+// k_nr_block calls it for its last parts of up to kNrTail elements where one holds a
+// NaN; whole, it is the sequential form that the tests hold the parallel ones to.
 __device__ bool nr_sort_local(double* key, int* id, int n) {
   int stk[32];
   int js = 0, l = 0, ir = n - 1;
@@ -1743,9 +1745,9 @@ bool local_minima(Ctx& c) {
                                                  c.ht_first, c.ht_best, cap, c.d_cnt);
   k_conn_pass<1><<<grid1d(nn), kBlock, 0, st>>>(c.bd, c.basins, open, c.pos, c.h, c.ht_key, c.ht_wmin,
                                                  c.ht_first, c.ht_best, cap, c.d_cnt);
-  k_conn_compact<<<(unsigned)((cap + 4 * kBlock - 1) / (4 * kBlock)), kBlock, 0, st>>>(c.bd, cap, c.ht_key, c.ht_first, c.ht_best, c.stack, c.h,
-                                                  c.conn_cap, c.e_key, c.r_b1, c.r_b2, c.r_n1, c.r_n2,
-                                                  c.r_w, c.d_cnt);
+  const unsigned compact_blocks = (unsigned)((cap + 4 * kBlock - 1) / (4 * kBlock));
+  k_conn_compact<<<compact_blocks, kBlock, 0, st>>>(c.bd, cap, c.ht_key, c.ht_first, c.ht_best, c.stack, c.h, c.conn_cap,
+                                                    c.e_key, c.r_b1, c.r_b2, c.r_n1, c.r_n2, c.r_w, c.d_cnt);
   k_conn_virtual<<<grid1d(nroots), kBlock, 0, st>>>(c.bd, nroots, c.s_roots, c.pos, c.conn_cap, c.e_key, c.r_b1,
                                                      c.r_b2, c.r_n1, c.r_n2, c.r_w, c.d_cnt);
   c.count_launch(4);

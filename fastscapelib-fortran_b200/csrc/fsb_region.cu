@@ -13,7 +13,7 @@
 // over one CTA per SM (cooperative launch, all co-resident), so that the
 // front, wherever it runs, is spread over all SMs.  A CTA keeps its nodes'
 // dependency counters in shared memory and hands ready nodes to its warps
-// through a queue that its L1 serves; one lane computes one node.  What a
+// through a queue that its L1 serves; eight lanes compute one node.  What a
 // node needs beyond its inputs' values is one 96-byte record, built in
 // parallel before the sweep and brought into L1 by the nodes it waits for.
 // A value that crosses a tile edge is written into a mailbox cell of the
@@ -53,7 +53,10 @@ constexpr unsigned long long kRegionTimeLimitNs = 4000000000ull;  // a sweep giv
 // nodes).  2049^2, B200: 384 threads 5.9 + 7.9 ms (area + stream power), 512
 // threads 5.8 + 7.3, 768 threads 5.8 + 7.5.
 constexpr int kThreads = 512;
-// grids whose records (96 bytes a node) L2 does not keep
+// Grids whose records (96 bytes a node) L2 does not keep: the area sweep then brings
+// the records two hops on into L2.  With / without that code, random surfaces:
+// 1025^2 2.91 / 2.81 ms, 2049^2 5.46 / 5.84, 4097^2 30.2 / 32.9; reliefs 2.50 / 2.36,
+// 5.29 / 5.23, 14.0 / 14.2.
 constexpr int kL2Records = 1 << 20;
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -1171,8 +1174,10 @@ TileMap plan_tiles(int nx, int ny, int lt, int sms) {
 // Tile sides.  Smaller tiles spread the front over more SMs and halve the
 // nodes that share an SM; larger ones have fewer crossings, and the area's
 // nodes, all sources at once, are spread anyway.  B200, side 32 / 64: area
-// 257^2 0.48 / 0.53 ms, 1025x769 3.05 / 2.88, 2049^2 6.4 / 5.8; stream power
-// (n = 1.5) 0.69 / 0.84, 3.98 / 4.27, 6.9 / 7.3, 4097^2 18.0 / 18.0.
+// 257^2 0.48 / 0.53 ms, 1025x769 3.05 / 2.88, 2049^2 6.4 / 5.8, and around the
+// border (random surfaces) 385^2 0.81 / 0.83, 513^2 0.83 / 0.83, 577^2 1.46 / 1.42,
+// 641^2 1.34 / 1.26; stream power (n = 1.5) 0.69 / 0.84, 3.98 / 4.27, 6.9 / 7.3,
+// 4097^2 18.0 / 18.0.
 // A strip that one larger tile spans and a smaller one does not takes the larger:
 // its flow runs along it, and every row of nodes would wait for a crossing
 // (4000x33, a cone: area 11.3 / 5.5 ms, stream power 15.7 / 10.8; 256x50, a ramp:
