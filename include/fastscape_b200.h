@@ -104,7 +104,8 @@ int fsb_set_v(fsb_ctx* c, const double* vx, const double* vy, int where);
    the ADI residuals stay FP64, integer routing stays exact; the multiple-flow
    slopes and weights, the drainage area, the stream-power erosion factors and
    Newton iterations (solved for the increment of h) and the tridiagonal
-   solves (for the increment of the surface) run in FP32. */
+   solves (for the increment of the surface) run in FP32; beyond 296 blocks of
+   256 x 128 nodes the area and the Newton iterations stay FP64. */
 enum { FSB_PREC_FP64 = 0, FSB_PREC_MIXED = 1 };
 int fsb_set_precision(fsb_ctx* c, int precision);
 int fsb_get_precision(fsb_ctx* c, int* precision);
